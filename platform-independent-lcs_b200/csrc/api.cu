@@ -424,6 +424,7 @@ struct slcs_batch_plan {
         L.progress = d_work + WORK_HEAD;
         L.status = device_status_word();
         L.wait_ns = wait_ns;
+        L.wide = wide_ids(max_ids, 0);
         return L;
     }
 
@@ -553,6 +554,7 @@ slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_
     L.single.m = m;
     L.single.n = n;
     L.tw = pick_tw(tm, ntasks, n, b);
+    L.wide = wide_ids(m, n);
     // h and v may live in separate allocations: address v relative to h.
     L.single.out_off = 0;
     slcs_status s;
@@ -881,6 +883,10 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         P->need_b = std::max<int64_t>(P->need_b, pairs[p].b_offset + pairs[p].n);
         P->need_out = std::max<int64_t>(P->need_out, pairs[p].out_offset + pairs[p].m + pairs[p].n);
         P->max_ids = std::max<int64_t>(P->max_ids, int64_t(pairs[p].m) + pairs[p].n);
+    }
+    if (wide_ids(P->max_ids, 0)) { // the batch kernel has only the fast cell rule
+        P->stm = 0;
+        P->classes.clear();
     }
     int32_t stream_rows = 0;
     for (const auto &c : P->classes) stream_rows = std::max(stream_rows, c.tm * c.seg);

@@ -33,9 +33,9 @@
 //     stripes fit at once, each SM runs one block of ceil(stripes / SMs)
 //     warps, so that the stripes spread evenly over the SMs.
 //   * Rows past m and columns past n are masked by data, not by branches:
-//     a masked row has symbol -1 and h = INT_MIN (never swaps), a masked column
-//     has symbol -2 and v = INT_MAX (never swaps), so edge tiles need no host
-//     fixup.
+//     a masked row has a symbol nothing matches and h = -1 (never swaps), a
+//     masked column likewise and v = INT_MAX (never swaps), so edge tiles need
+//     no host fixup.
 #include <climits>
 #include <mutex>
 #include <type_traits>
@@ -89,19 +89,49 @@ struct StripeWait {
     }
 };
 
-__device__ __forceinline__ void cell(int a_sym, int b_sym, int &h, int &v)
+// Symbols as floats.  A symbol s of a or b becomes the float with bits
+// 0x43000000 | s << 16 (128 + s up to 127, 2 s above: distinct symbols are at
+// least 1 apart, and one byte permute makes it); masked rows and columns hold
+// floats far from every symbol and from each other.
+__device__ __forceinline__ uint32_t symbol_code(uint32_t word, int j)
 {
-    const bool swap = (a_sym == b_sym) | (h > v);
-    const int nh = swap ? v : h;
-    v = swap ? h : v;
-    h = nh;
+    return __byte_perm(word, 0x43000000u, 0x7044u | (uint32_t(j) << 8));
+}
+constexpr uint32_t MASKED_ROW = 0xF149F2CAu;    // -1e30f
+constexpr uint32_t MASKED_COLUMN = 0x7149F2CAu; // 1e30f
+
+// The cell rule.  With far = fma.sat(d, -d, 1), d = a - b: far holds the bits
+// of 1.0f (0x3F800000) when the symbols match and 0 otherwise, so that
+//   h' = min(h + far, v)   (v on a match, min(h, v) otherwise; one VIADDMNMX)
+//   v' = h + v - h'        (the other of the two)
+// for 0 <= h, v < FAST_IDS, 4 instructions of which two run on the FMA pipe.
+// A comb is bound by instruction issue and the integer pipe: compare, compare
+// and two selects (all on the integer pipe) measured 6.76 cycles per warp and
+// cell of a sub-partition holding 4 warps of 16 rows per lane, this 4.59.
+// Masked rows hold h = -1 and masked columns v = INT_MAX; neither ever
+// matches, so neither swaps.  WIDE keeps the compare and selects for pairs
+// whose ids reach FAST_IDS.
+template <bool WIDE>
+__device__ __forceinline__ void cell(uint32_t a, uint32_t b, int &h, int &v)
+{
+    if constexpr (WIDE) {
+        const bool swap = (a == b) | (h > v);
+        const int nh = swap ? v : h;
+        v = swap ? h : v;
+        h = nh;
+    } else {
+        const float d = __uint_as_float(a) - __uint_as_float(b);
+        const int nh = __viaddmin_s32(h, __float_as_int(__saturatef(__fmaf_rn(d, -d, 1.0f))), v);
+        v = int(uint32_t(h) + uint32_t(v) - uint32_t(nh));
+        h = nh;
+    }
 }
 
 // One row stripe of one pair, combed by one warp.  TW columns form a block,
 // the unit of a step, of a scratch-row transfer and of the shuffle hand-off;
 // the ring holds RING blocks of TW strands per warp.  TW = 4 everywhere but
 // in launches that pick_tw() gives 8 (short stripe chains of tall tiles).
-template <int TM, int TW>
+template <int TM, int TW, bool WIDE>
 struct Stripe {
     static constexpr int Q = TW / 4;                 // int4 per block
     static constexpr int PREF = pref_of(TM);
@@ -115,7 +145,8 @@ struct Stripe {
     StripeWait W;
     int m, n, nb, lane;
     bool first, has_next;
-    int av[TM], hv[TM], vc[TW];
+    uint32_t av[TM];
+    int hv[TM], vc[TW];
 
     // Column symbols of a whole block as one word (b aligned to its size).
     using Word = typename std::conditional<TW == 8, uint2, uint32_t>::type;
@@ -123,23 +154,23 @@ struct Stripe {
 
     __device__ __forceinline__ Word word(int blk) const { return __ldg(reinterpret_cast<const Word *>(b + blk * TW)); }
 
-    __device__ __forceinline__ static void unpack(uint32_t w, int *bs)
+    __device__ __forceinline__ static void unpack(uint32_t w, uint32_t *bs)
     {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) bs[j] = int((w >> (8 * j)) & 0xffu);
+        for (int j = 0; j < 4; ++j) bs[j] = symbol_code(w, j);
     }
-    __device__ __forceinline__ static void unpack(uint2 w, int *bs)
+    __device__ __forceinline__ static void unpack(uint2 w, uint32_t *bs)
     {
         unpack(w.x, bs);
         unpack(w.y, bs + 4);
     }
 
-    // Column symbols of block blk: -2 past n or when the lane is idle.
-    __device__ __forceinline__ void symbols(int blk, bool act, int (&bs)[TW]) const
+    // Column symbols of block blk: masked past n or when the lane is idle.
+    __device__ __forceinline__ void symbols(int blk, bool act, uint32_t (&bs)[TW]) const
     {
         const int c = blk * TW;
 #pragma unroll
-        for (int j = 0; j < TW; ++j) bs[j] = (act && c + j < n) ? int(__ldg(b + c + j)) : -2;
+        for (int j = 0; j < TW; ++j) bs[j] = (act && c + j < n) ? symbol_code(__ldg(b + c + j), 0) : MASKED_COLUMN;
     }
 
     // Lane 0: the v strands entering block t at the top of the stripe.
@@ -191,7 +222,7 @@ struct Stripe {
 #pragma unroll
         for (int j = 0; j < TW; ++j) vi[j] = __shfl_up_sync(FULL_MASK, vc[j], 1);
         if (lane == 0) top<FULL>(t, vi);
-        int bs[TW];
+        uint32_t bs[TW];
         if (FULL) {
             // The word was loaded one step ago; fetch the next one now, so
             // that the load's latency hides behind this step's cells.
@@ -204,7 +235,7 @@ struct Stripe {
         for (int j = 0; j < TW; ++j) {
             int v = vi[j];
 #pragma unroll
-            for (int k = 0; k < TM; ++k) cell(av[k], bs[j], hv[k], v);
+            for (int k = 0; k < TM; ++k) cell<WIDE>(av[k], bs[j], hv[k], v);
             vc[j] = v;
         }
         if (lane == 31 && act) {
@@ -225,11 +256,12 @@ struct Stripe {
     }
 };
 
-template <int TM, int TW = 4>
+template <int TM, int TW = 4, bool WIDE = false>
 __device__ __forceinline__ void comb_stripe(const CombLaunch &L, const PairDev &P, int64_t scr_off,
                                             int stripe, int task, int4 *ring, int lane)
 {
-    Stripe<TM, TW> S;
+    using StripeT = Stripe<TM, TW, WIDE>;
+    StripeT S;
     const int m = P.m, n = P.n;
     const uint8_t *__restrict__ a = L.a_blob + P.a_off;
     int32_t *hout = L.out + P.out_off;
@@ -249,8 +281,8 @@ __device__ __forceinline__ void comb_stripe(const CombLaunch &L, const PairDev &
     for (int k = 0; k < TM; ++k) {
         const int r = r0 + lane * TM + k;
         const bool in = r < m;
-        S.av[k] = in ? int(a[r]) : -1;
-        S.hv[k] = in ? (m - 1 - r) : INT_MIN;
+        S.av[k] = in ? symbol_code(a[r], 0) : MASKED_ROW;
+        S.hv[k] = in ? (m - 1 - r) : -1;
     }
     S.first = stripe == 0;
     S.has_next = r0 + 32 * TM < m;
@@ -258,13 +290,13 @@ __device__ __forceinline__ void comb_stripe(const CombLaunch &L, const PairDev &
 
     if (!S.first && lane == 0) {
 #pragma unroll
-        for (int d = 0; d < Stripe<TM, TW>::PREF; ++d) {
+        for (int d = 0; d < StripeT::PREF; ++d) {
             if (d < nb) {
                 S.W.until(d);
                 if (!S.W.dead) {
 #pragma unroll
-                    for (int q = 0; q < Stripe<TM, TW>::Q; ++q)
-                        cp_async_cg16(&ring[d * Stripe<TM, TW>::Q + q], S.scr + d * TW + 4 * q);
+                    for (int q = 0; q < StripeT::Q; ++q)
+                        cp_async_cg16(&ring[d * StripeT::Q + q], S.scr + d * TW + 4 * q);
                 }
             }
             cp_async_commit();
@@ -318,7 +350,7 @@ __device__ __forceinline__ void task_of(const CombLaunch &L, int k, PairDev &P, 
 // w * gridDim.x + b in a cooperative launch, spreads consecutive stripes over
 // the SMs; it combed the 2^20 pair in 763 ms instead of 407 ms, because the
 // four stripes sharing a sub-partition then start and finish far apart.)
-template <int TM, int WARPS, int TW>
+template <int TM, int WARPS, int TW, bool WIDE = false>
 __global__ void __launch_bounds__(WARPS * 32) comb_wavefront_kernel(const CombLaunch L)
 {
     __shared__ __align__(16) int4 ring[WARPS][RING * TW / 4];
@@ -333,7 +365,7 @@ __global__ void __launch_bounds__(WARPS * 32) comb_wavefront_kernel(const CombLa
         k = __shfl_sync(FULL_MASK, k, 0);
         if (k >= L.ntasks) break;
         task_of(L, k, P, stripe, so);
-        comb_stripe<TM, TW>(L, P, so, stripe, k, ring[w], lane);
+        comb_stripe<TM, TW, WIDE>(L, P, so, stripe, k, ring[w], lane);
     }
 }
 
@@ -398,15 +430,15 @@ __device__ __forceinline__ void fetch_next(const CombLaunch &L, int pair, int r0
 // Make the fetched pair current: rows r0.. get its symbols and start ids.
 template <int TM>
 __device__ __forceinline__ void take_next(const CombLaunch &L, const NextPair<TM> &N, int r0, StreamTask<TM> &T,
-                                          int (&av)[TM], int (&hv)[TM])
+                                          uint32_t (&av)[TM], int (&hv)[TM])
 {
     T.pair = N.pair;
     if (N.pair < 0) {
         T.m = T.n = T.nb = 0;
 #pragma unroll
         for (int k = 0; k < TM; ++k) {
-            av[k] = -1;
-            hv[k] = INT_MIN;
+            av[k] = MASKED_ROW;
+            hv[k] = -1;
         }
         return;
     }
@@ -421,8 +453,8 @@ __device__ __forceinline__ void take_next(const CombLaunch &L, const NextPair<TM
 #pragma unroll
     for (int k = 0; k < TM; ++k) {
         const bool in = r0 + k < T.m;
-        av[k] = in ? int((N.sym[k / 4] >> (8 * (k % 4))) & 0xffu) : -1;
-        hv[k] = in ? (T.m - 1 - r0 - k) : INT_MIN;
+        av[k] = in ? symbol_code(N.sym[k / 4], k % 4) : MASKED_ROW;
+        hv[k] = in ? (T.m - 1 - r0 - k) : -1;
     }
 }
 
@@ -489,7 +521,8 @@ __device__ __forceinline__ void stream_segment(const BatchLaunch &B, int cls, in
     p1 = __shfl_sync(FULL_MASK, p1, seg_lane0);
     StreamTask<TM> T;
     NextPair<TM> N;
-    int av[TM], hv[TM];
+    uint32_t av[TM];
+    int hv[TM];
     fetch_next<TM>(L, p0, r0, N);
     take_next<TM>(L, N, r0, T, av, hv);
     T.nb = (T.n + TNS - 1) / TNS;
@@ -516,31 +549,32 @@ __device__ __forceinline__ void stream_segment(const BatchLaunch &B, int cls, in
             for (int j = 0; j < TNS; ++j) vi[j] = (act && c + j < T.n) ? T.m + c + j : INT_MAX;
         }
 
-        int bs[TNS];
+        uint32_t bs[TNS];
         // Whole-word loads only where b is aligned to TNS bytes (c is a multiple of TNS).
         if (act && c + TNS <= T.n && (reinterpret_cast<uintptr_t>(T.b) & (TNS - 1)) == 0) {
             if constexpr (TNS == 8) {
                 const uint2 w = __ldg(reinterpret_cast<const uint2 *>(T.b + c));
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    bs[j] = int((w.x >> (8 * j)) & 0xffu);
-                    bs[4 + j] = int((w.y >> (8 * j)) & 0xffu);
+                    bs[j] = symbol_code(w.x, j);
+                    bs[4 + j] = symbol_code(w.y, j);
                 }
             } else {
                 const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(T.b + c));
 #pragma unroll
-                for (int j = 0; j < TNS; ++j) bs[j] = int((w >> (8 * j)) & 0xffu);
+                for (int j = 0; j < TNS; ++j) bs[j] = symbol_code(w, j);
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < TNS; ++j) bs[j] = (act && c + j < T.n) ? int(__ldg(T.b + c + j)) : -2;
+            for (int j = 0; j < TNS; ++j)
+                bs[j] = (act && c + j < T.n) ? symbol_code(__ldg(T.b + c + j), 0) : MASKED_COLUMN;
         }
 
 #pragma unroll
         for (int j = 0; j < TNS; ++j) {
             int v = vi[j];
 #pragma unroll
-            for (int k = 0; k < TM; ++k) cell(av[k], bs[j], hv[k], v);
+            for (int k = 0; k < TM; ++k) cell<false>(av[k], bs[j], hv[k], v);
             vc[j] = v;
         }
 
@@ -577,25 +611,30 @@ __device__ __forceinline__ void stream_segment(const BatchLaunch &B, int cls, in
 // h and v register holds pair A in its low 16 bits and pair B in its high 16
 // bits, so one instruction works on two cells.  Strand ids are stored plus
 // one (1..32767); a masked row holds h = 0 and symbol 0x1FF, a masked column
-// v = 0x7FFF and symbol 0x100, so neither ever swaps.  The cell rule per half
-// is evaluated in bit 15 without carries between the halves:
-//   y = (a ^ b) + 0x7FFF      bit 15 set iff the symbols differ (a^b <= 0x1FF)
-//   d = (v + 0x8000) - h      bit 15 set iff v >= h (no crossing)
-//   keep = d & y & 0x8000 -> expanded to 0xFFFF by a sign-replicating byte
-//   permute (PTX prmt with selector nibbles 0x9/0xB: bit 3 of a nibble
-//   replicates the sign of the chosen byte; __byte_perm only copies bytes);
-//   h' = keep ? h : v, v' = keep ? v : h.
+// v = 0x7FFF and symbol 0x100, so neither ever swaps.  The cell rule per half:
+//   x = a ^ b                    0 on a match (both below 0x200)
+//   far = fma.relu(x, -inf, 0)   on two 16-bit floats: 0 * -inf is NaN, which
+//                                relu turns into 0x7FFF; a positive x gives
+//                                -inf, which relu turns into 0
+//   h' = min(h + far, v)         unsigned halves, one VIADDMNMX
+//   v' = h + v - h'              as one 32-bit sum: the carries between the
+//                                halves cancel
+// On a match h + far is at least any v, so h' = v.  Seven integer instructions
+// (a carry-safe difference, a byte permute expanding its sign to a mask, two
+// bitwise selects) measured 5.50 cycles per warp and cell, these four 2.39
+// (one sub-partition, 4 warps of 16 rows per lane).
 // Both pairs of a couple switch together after max(nb_A, nb_B) blocks; the
 // shorter pair's extra columns are masked.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cell16(uint32_t a, uint32_t b, uint32_t &h, uint32_t &v)
 {
-    const uint32_t y = (a ^ b) + 0x7FFF7FFFu;
-    const uint32_t d = (v + 0x80008000u) - h;
-    uint32_t keep;
-    asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(keep) : "r"(d & y & 0x80008000u));
-    const uint32_t nh = (h & keep) | (v & ~keep);
-    v = (v & keep) | (h & ~keep);
+    uint32_t far;
+    asm("{\n\t.reg .b32 ninf, zero;\n\tmov.b32 ninf, 0xFF80FF80;\n\tmov.b32 zero, 0;\n\t"
+        "fma.rn.relu.bf16x2 %0, %1, ninf, zero;\n\t}"
+        : "=r"(far)
+        : "r"(a ^ b));
+    const uint32_t nh = __viaddmin_u16x2(h, far, v);
+    v = h + v - nh;
     h = nh;
 }
 
@@ -999,15 +1038,12 @@ slcs_status occupancy_of(int threads, int *occ_out)
 // `sms` is the SM count of the current device (passed in by the caller, so
 // that entry points that must not allocate never touch the lazily created
 // per-device state behind sm_count()).
-template <int TM, int WARPS, int TW>
-slcs_status launch_variant_tw(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out)
+template <int TM, int WARPS, int TW, bool WIDE>
+slcs_status launch_persistent(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out)
 {
     if (sms < 1) sms = 1;
-    bool done = false;
-    const slcs_status bs = launch_balanced<TM, TW>(L, sms, stream, grid_out, &done);
-    if (bs != SLCS_OK || done) return bs;
     int occ = 1;
-    const slcs_status os = occupancy_of<comb_wavefront_kernel<TM, WARPS, TW>>(WARPS * 32, &occ);
+    const slcs_status os = occupancy_of<comb_wavefront_kernel<TM, WARPS, TW, WIDE>>(WARPS * 32, &occ);
     if (os != SLCS_OK) return os;
     if (stream == PREPARE_ONLY) return SLCS_OK;
     // More stripes than fit at once: persistent blocks take stripes from the
@@ -1019,10 +1055,19 @@ slcs_status launch_variant_tw(const CombLaunch &L, long sms, cudaStream_t stream
     long grid = sms * occ;
     if (want < grid) grid = want;
     if (grid < 1) grid = 1;
-    comb_wavefront_kernel<TM, WARPS, TW><<<int(grid), WARPS * 32, 0, stream>>>(L);
+    comb_wavefront_kernel<TM, WARPS, TW, WIDE><<<int(grid), WARPS * 32, 0, stream>>>(L);
     if (grid_out) *grid_out = int(grid);
     SLCS_CUDA(cudaGetLastError());
     return SLCS_OK;
+}
+
+template <int TM, int WARPS, int TW>
+slcs_status launch_variant_tw(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out)
+{
+    bool done = false;
+    const slcs_status bs = launch_balanced<TM, TW>(L, sms, stream, grid_out, &done);
+    if (bs != SLCS_OK || done) return bs;
+    return launch_persistent<TM, WARPS, TW, false>(L, sms, stream, grid_out);
 }
 
 template <int TM, int WARPS>
@@ -1061,6 +1106,7 @@ static slcs_status launch_comb_sms(const CombLaunch &L, int tile_m, int warps, l
     if (L.ntasks <= 0) return SLCS_OK;
 #define SLCS_TM_CASE(TM)                                                                   \
     case TM:                                                                               \
+        if (L.wide) return launch_persistent<TM, 4, 4, true>(L, sms, stream, grid_out);    \
         if (warps == 2) return launch_variant<TM, 2>(L, sms, stream, grid_out);            \
         if (warps == 8) return launch_variant<TM, 8>(L, sms, stream, grid_out);            \
         return launch_variant<TM, 4>(L, sms, stream, grid_out);

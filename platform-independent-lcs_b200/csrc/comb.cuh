@@ -24,7 +24,14 @@ struct CombLaunch {
     uint64_t wait_ns;           // limit of one bounded wait
     PairDev single;
     int32_t tw;                 // wavefront columns per step: 8 (tile_m 14/16 only) or 4 (0 = 4)
+    bool wide;                  // some pair of the launch has ids of FAST_IDS and more (launch_comb only)
 };
+
+// Strand ids (below m + n of a pair) the cell rule's fast form takes: below
+// the bits of 1.0f, so that adding those to an id passes every other id and
+// stays below 2^31.
+constexpr int64_t FAST_IDS = 0x3F800000;
+inline bool wide_ids(int64_t m, int64_t n) { return m + n > FAST_IDS; }
 
 // Columns per step for a wavefront launch whose longest stripe chain has
 // `chain` stripes and whose narrowest tile has `width` columns of b: 8 halves
