@@ -390,6 +390,7 @@ struct slcs_batch_plan {
     cudaStream_t cap_stream = nullptr;
     // Extents the descriptors reach (elements), checked by the host-pointer run.
     int64_t need_a = 0, need_b = 0, need_out = 0;
+    bool wide = false;   // ids past the fast cell rule (wavefront launch only)
     int64_t max_ids = 0; // largest m + n of a pair (strand ids are below it)
     // Device int16 copy of the strands for slcs_batch_plan_run_host16, grown on demand.
     int16_t *d_out16 = nullptr;
@@ -424,7 +425,7 @@ struct slcs_batch_plan {
         L.progress = d_work + WORK_HEAD;
         L.status = device_status_word();
         L.wait_ns = wait_ns;
-        L.wide = wide_ids(max_ids, 0);
+        L.wide = wide;
         return L;
     }
 
@@ -554,7 +555,7 @@ slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_
     L.single.m = m;
     L.single.n = n;
     L.tw = pick_tw(tm, ntasks, n, b);
-    L.wide = wide_ids(m, n);
+    L.wide = wide_ids(m, n, cfg);
     // h and v may live in separate allocations: address v relative to h.
     L.single.out_off = 0;
     slcs_status s;
@@ -884,7 +885,8 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         P->need_out = std::max<int64_t>(P->need_out, pairs[p].out_offset + pairs[p].m + pairs[p].n);
         P->max_ids = std::max<int64_t>(P->max_ids, int64_t(pairs[p].m) + pairs[p].n);
     }
-    if (wide_ids(P->max_ids, 0)) { // the batch kernel has only the fast cell rule
+    P->wide = wide_ids(P->max_ids, 0, wavefront_only ? cfg : nullptr);
+    if (P->wide && !wavefront_only) { // the batch kernel has only the fast cell rule
         P->stm = 0;
         P->classes.clear();
     }

@@ -102,12 +102,14 @@ constexpr uint32_t MASKED_COLUMN = 0x7149F2CAu; // 1e30f
 
 // The cell rule.  With far = fma.sat(d, -d, 1), d = a - b: far holds the bits
 // of 1.0f (0x3F800000) when the symbols match and 0 otherwise, so that
-//   h' = min(h + far, v)   (v on a match, min(h, v) otherwise; one VIADDMNMX)
-//   v' = h + v - h'        (the other of the two)
-// for 0 <= h, v < FAST_IDS, 4 instructions of which two run on the FMA pipe.
-// A comb is bound by instruction issue and the integer pipe: compare, compare
-// and two selects (all on the integer pipe) measured 6.76 cycles per warp and
-// cell of a sub-partition holding 4 warps of 16 rows per lane, this 4.59.
+//   h' = min(h + far, v)   (v on a match, min(h, v) otherwise)
+//   v' = max(v - far, h)   (h on a match, max(h, v) otherwise)
+// for 0 <= h, v < FAST_IDS: 4 instructions, two of them on the FMA pipe.  A
+// comb is bound by instruction issue and the integer pipe, a lone warp by the
+// chain through h and v.  In cycles per warp and cell (4 columns per step, 16
+// rows per lane): compare, compare and two selects 6.76 with 4 warps on a
+// sub-partition and 10.0 with one, this 4.61 and 5.45; v' = h + v - h' instead
+// of the max (h' is then in v's chain) 4.58 and 7.92.
 // Masked rows hold h = -1 and masked columns v = INT_MAX; neither ever
 // matches, so neither swaps.  WIDE keeps the compare and selects for pairs
 // whose ids reach FAST_IDS.
@@ -121,8 +123,9 @@ __device__ __forceinline__ void cell(uint32_t a, uint32_t b, int &h, int &v)
         h = nh;
     } else {
         const float d = __uint_as_float(a) - __uint_as_float(b);
-        const int nh = __viaddmin_s32(h, __float_as_int(__saturatef(__fmaf_rn(d, -d, 1.0f))), v);
-        v = int(uint32_t(h) + uint32_t(v) - uint32_t(nh));
+        const int far = __float_as_int(__saturatef(__fmaf_rn(d, -d, 1.0f)));
+        const int nh = __viaddmin_s32(h, far, v);
+        v = __viaddmax_s32(v, -far, h);
         h = nh;
     }
 }

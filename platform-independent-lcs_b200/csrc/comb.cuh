@@ -31,7 +31,10 @@ struct CombLaunch {
 // the bits of 1.0f, so that adding those to an id passes every other id and
 // stays below 2^31.
 constexpr int64_t FAST_IDS = 0x3F800000;
-inline bool wide_ids(int64_t m, int64_t n) { return m + n > FAST_IDS; }
+inline bool wide_ids(int64_t m, int64_t n, const slcs_config *cfg)
+{
+    return m + n > FAST_IDS || (cfg && cfg->strand_bits == 32);
+}
 
 // Columns per step for a wavefront launch whose longest stripe chain has
 // `chain` stripes and whose narrowest tile has `width` columns of b: 8 halves

@@ -161,6 +161,6 @@ extern "C" SLCS_API slcs_status slcs_comb_pair_noalloc(const uint8_t *a, int32_t
     L.single.m = m;
     L.single.n = n;
     L.tw = pick_tw(tm, ntasks, n, b);
-    L.wide = wide_ids(m, n);
+    L.wide = wide_ids(m, n, cfg);
     return launch_comb_on(L, tm, pick_warps(cfg, tm), state.sms, st);
 }

@@ -304,7 +304,7 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
             width = std::min<int64_t>(width, d.n);
         }
         L.tw = pick_tw(tm, chain, width, b);
-        L.wide = std::any_of(pd.begin(), pd.end(), [](const slcs_pair_desc &d) { return wide_ids(d.m, d.n); });
+        L.wide = std::any_of(pd.begin(), pd.end(), [&](const slcs_pair_desc &d) { return wide_ids(d.m, d.n, cfg); });
         s = launch_comb(L, tm, warps, st, nullptr);
     }
     // Strands of every tile -> its permutation (row -> col) in Y.
