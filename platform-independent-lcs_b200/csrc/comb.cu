@@ -40,6 +40,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "cell.cuh"
 #include "comb.cuh"
 
 namespace slcs {
@@ -88,47 +89,6 @@ struct StripeWait {
         }
     }
 };
-
-// Symbols as floats.  A symbol s of a or b becomes the float with bits
-// 0x43000000 | s << 16 (128 + s up to 127, 2 s above: distinct symbols are at
-// least 1 apart, and one byte permute makes it); masked rows and columns hold
-// floats far from every symbol and from each other.
-__device__ __forceinline__ uint32_t symbol_code(uint32_t word, int j)
-{
-    return __byte_perm(word, 0x43000000u, 0x7044u | (uint32_t(j) << 8));
-}
-constexpr uint32_t MASKED_ROW = 0xF149F2CAu;    // -1e30f
-constexpr uint32_t MASKED_COLUMN = 0x7149F2CAu; // 1e30f
-
-// The cell rule.  With far = fma.sat(d, -d, 1), d = a - b: far holds the bits
-// of 1.0f (0x3F800000) when the symbols match and 0 otherwise, so that
-//   h' = min(h + far, v)   (v on a match, min(h, v) otherwise)
-//   v' = max(v - far, h)   (h on a match, max(h, v) otherwise)
-// for 0 <= h, v < FAST_IDS: 4 instructions, two of them on the FMA pipe.  A
-// comb is bound by instruction issue and the integer pipe, a lone warp by the
-// chain through h and v.  In cycles per warp and cell (4 columns per step, 16
-// rows per lane): compare, compare and two selects 6.76 with 4 warps on a
-// sub-partition and 10.0 with one, this 4.61 and 5.45; v' = h + v - h' instead
-// of the max (h' is then in v's chain) 4.58 and 7.92.
-// Masked rows hold h = -1 and masked columns v = INT_MAX; neither ever
-// matches, so neither swaps.  WIDE keeps the compare and selects for pairs
-// whose ids reach FAST_IDS.
-template <bool WIDE>
-__device__ __forceinline__ void cell(uint32_t a, uint32_t b, int &h, int &v)
-{
-    if constexpr (WIDE) {
-        const bool swap = (a == b) | (h > v);
-        const int nh = swap ? v : h;
-        v = swap ? h : v;
-        h = nh;
-    } else {
-        const float d = __uint_as_float(a) - __uint_as_float(b);
-        const int far = __float_as_int(__saturatef(__fmaf_rn(d, -d, 1.0f)));
-        const int nh = __viaddmin_s32(h, far, v);
-        v = __viaddmax_s32(v, -far, h);
-        h = nh;
-    }
-}
 
 // One row stripe of one pair, combed by one warp.  TW columns form a block,
 // the unit of a step, of a scratch-row transfer and of the shuffle hand-off;
@@ -358,7 +318,7 @@ __global__ void __launch_bounds__(WARPS * 32) comb_wavefront_kernel(const CombLa
 {
     __shared__ __align__(16) int4 ring[WARPS][RING * TW / 4];
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
+    const int w = __shfl_sync(FULL_MASK, int(threadIdx.x) >> 5, 0); // warp-uniform for the compiler
     PairDev P;
     int stripe;
     int64_t so;
@@ -885,7 +845,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) comb_batch_kernel(cons
 {
     __shared__ __align__(16) int4 wf_ring[WARPS][RING];
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
+    const int w = __shfl_sync(FULL_MASK, int(threadIdx.x) >> 5, 0); // warp-uniform for the compiler
     const int gw = blockIdx.x * WARPS + w;
     const CombLaunch &L = B.wf;
     // Phase 1: this warp's stream segments (class and lists fixed by the plan).
