@@ -129,7 +129,16 @@ typedef struct {
     int32_t braid_cutoff; /* steady-ant cutoff of the merge products (0: no merge)   */
     int32_t stripes;      /* row stripes of all tiles (warp tasks of the comb)       */
     int32_t cols_per_step;/* wavefront columns per step (4 or 8) for b aligned to 8  */
-    int32_t reserved[8];
+    /* relay_tile_m > 0: the pair is combed by the relay kernel (a wavefront
+     * whose stripes hand down in shared memory) and the fields above say only
+     * what the wavefront kernel would do.  Its rows per lane, columns per
+     * step, combing warps per block, column strips and row bands: */
+    int32_t relay_tile_m;
+    int32_t relay_cols;
+    int32_t relay_warps;
+    int32_t relay_strips;
+    int32_t relay_bands;
+    int32_t reserved[3];
 } slcs_pair_info;
 SLCS_API slcs_status slcs_pair_plan_info(int32_t m, int32_t n, const slcs_config *cfg, slcs_pair_info *info);
 /* The same plan for a device of `sms` SMs; touches no device (planning ahead
@@ -323,9 +332,9 @@ SLCS_API slcs_status slcs_probe_int_rates(int32_t iters, double *int32_ops_per_s
                                           void *stream);
 
 /* Check of the failure path the reference reports through exceptions
- * (src/main.cpp:83-94): enqueues one wavefront launch of a small two-stripe
- * pair whose first stripe is never claimed, so the second stripe's bounded
- * wait for it runs out after wait_ms (1..5000).  After synchronising the
+ * (src/main.cpp:83-94): enqueues one wavefront and one relay launch of a small
+ * pair whose first stripe (group) is never claimed, so that the second one's
+ * bounded wait for it runs out after wait_ms (1..5000).  After synchronising the
  * stream, slcs_device_status() reports SLCS_ERR_TIMEOUT; the context stays
  * usable and later calls run normally. */
 SLCS_API slcs_status slcs_probe_wait_expiry(int32_t wait_ms, void *stream);

@@ -15,6 +15,7 @@
 #include "braid.cuh"
 #include "comb.cuh"
 #include "queries.cuh"
+#include "relay.cuh"
 #include "strips.cuh"
 
 namespace slcs {
@@ -174,10 +175,70 @@ int pick_warps(const slcs_config *cfg, int tm) { return (cfg && cfg->warps) ? cf
 
 namespace {
 
+// Shapes of the relay kernel: rows per lane, columns per step, combing warps,
+// and the cycles one step takes while a block has its SM to itself (B200,
+// inside whole combs; a step is bound by the chain shuffle -> cells -> shuffle
+// until 8 rows per lane, then by instruction issue).
+struct RelayCost {
+    RelayShape shape;
+    double step;
+};
+const RelayCost RELAY_COSTS[] = {{{1, 4, 3}, 66.0},  {{2, 4, 3}, 79.0},  {{4, 2, 3}, 76.0},
+                                 {{8, 2, 3}, 108.0}, {{8, 4, 4}, 212.0}, {{16, 4, 4}, 425.0}};
+constexpr double RELAY_GHZ = 1.965;     // the clock those cycles were measured at
+constexpr double RELAY_WARP_LAG = 40.0; // steps a warp starts after the warp above it
+constexpr double RELAY_HOP_LAG = 45.0;  // more steps for the hand-down to the next block
+
+// Microseconds of one braid product of overlap k inside a merge level (B200).
+double braid_us(double k)
+{
+    static const double log2k[] = {6, 8, 10, 12, 14, 16, 17, 20};
+    static const double us[] = {52, 97, 185, 266, 376, 542, 675, 1550};
+    const double x = std::log2(std::max(k, 64.0));
+    for (int i = 0; i < 6; ++i)
+        if (x < log2k[i + 1]) return us[i] + (us[i + 1] - us[i]) * (x - log2k[i]) / (log2k[i + 1] - log2k[i]);
+    return us[6] + (us[7] - us[6]) * (x - 17.0) / 3.0;
+}
+
+// The relay kernel's plan for one pair: shape, column strips and row bands
+// with the least predicted time among those whose groups fit one to an SM
+// (two blocks on one SM slow the whole chain: 342 groups of (4, 2, 3) on 148
+// SMs combed 131072 x 131072 in 13.2 ms, 128 of (8, 4, 4) in 6.4 ms).
+// relay.tm == 0: no shape fits.  Predicted: a chain's steps (columns, then
+// the lags of its warps and blocks) at the shape's step time, and the merge
+// levels, each at least a product of its overlap and, when it holds several,
+// about 55 us of launches a product.
+struct RelayPlan {
+    RelayShape relay{};
+    int strips = 1, bands = 1;
+    double us = 0;
+};
+RelayPlan plan_relay(int32_t m, int32_t n, int sms)
+{
+    RelayPlan best;
+    for (const RelayCost &c : RELAY_COSTS)
+        for (int R = 1; R <= 16 && (R == 1 || m / R >= 4096); R *= 2)
+            for (int S = 1; S <= 64 && (S == 1 || n / S >= 4096); S *= 2) {
+                const double stripes = std::ceil(std::ceil(double(m) / (32 * c.shape.tm)) / R);
+                const double groups = std::ceil(stripes / c.shape.warps);
+                if (groups * R * S > sms) continue;
+                const double steps = double(n) / S / c.shape.tw + RELAY_WARP_LAG * stripes + RELAY_HOP_LAG * groups;
+                double us = 6.0 + steps * c.step / (RELAY_GHZ * 1e3);
+                if (R * S > 1) us += 20.0;
+                for (int p = S; p > 1; p /= 2) us += std::max(braid_us(double(m) / R) + 35.0, 55.0 * R * (p / 2));
+                for (int p = R; p > 1; p /= 2) us += std::max(braid_us(double(n)) + 35.0, 55.0 * (p / 2));
+                if (best.relay.tm == 0 || us < best.us) best = RelayPlan{c.shape, S, R, us};
+            }
+    return best;
+}
+
 // How slcs_comb_pair combs one pair: the effective configuration (algo
-// WAVEFRONT or STRIPS with tile_m, warps, strips, bands, braid_cutoff set).
+// WAVEFRONT or STRIPS with tile_m, warps, strips, bands, braid_cutoff set),
+// and the relay plan that takes its place when nothing is configured and the
+// pair fits one.
 struct PairPlan {
     slcs_config c;
+    RelayPlan relay;
 };
 
 slcs_status plan_pair(int32_t m, int32_t n, const slcs_config *cfg, int sms, PairPlan *P)
@@ -200,6 +261,7 @@ slcs_status plan_pair(int32_t m, int32_t n, const slcs_config *cfg, int sms, Pai
     c.strips = 1;
     c.bands = 1;
     if (!auto_all) return SLCS_OK;
+    if (!wide_ids(m, n, cfg)) P->relay = plan_relay(m, n, sms);
     int R = auto_bands(m, n, tm);
     const int S = R > 1 ? 1 : auto_strips(m, n);
     if (S > 1) R = strip_bands(m);
@@ -231,6 +293,7 @@ __global__ void identity_strands_kernel(int32_t *h, int32_t m, int32_t *v, int32
 // contributes its row stripes as consecutive wavefront tasks, with a scratch
 // row when it has more than one stripe.
 struct Schedule {
+    std::vector<int32_t> order; // every pair, most cells first
     std::vector<int2> tasks;
     std::vector<int32_t> stream_pairs;
     std::vector<int64_t> scratch_off;
@@ -240,7 +303,8 @@ struct Schedule {
 Schedule build_schedule(const slcs_pair_desc *pairs, int32_t npairs, int tm, int32_t stream_rows)
 {
     Schedule S;
-    std::vector<int32_t> order(npairs);
+    std::vector<int32_t> &order = S.order;
+    order.resize(npairs);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) {
         return int64_t(pairs[x].m) * pairs[x].n > int64_t(pairs[y].m) * pairs[y].n;
@@ -384,6 +448,13 @@ struct slcs_batch_plan {
     int32_t *d_scratch = nullptr;
     int32_t *d_work = nullptr; // [counters(4) | progress(ntasks)]
     size_t work_bytes = 0;
+    // Pairs combed by the relay kernel instead (relay.tm > 0): all of the plan.
+    RelayShape relay{};
+    int32_t nrelay = 0;         // groups of all pairs
+    int2 *d_relay = nullptr;    // (pair, group)
+    int64_t *d_row_off = nullptr;
+    char *d_relay_ws = nullptr; // counters and hand-down rows, cleared by every run
+    size_t relay_ws_bytes = 0;
     std::vector<slcs_pair_desc> empty_pairs; // pairs with m == 0 or n == 0
     cudaGraphExec_t gexec = nullptr;
     const void *g_a = nullptr, *g_b = nullptr, *g_out = nullptr;
@@ -431,9 +502,24 @@ struct slcs_batch_plan {
 
     slcs_status enqueue(const uint8_t *a, const uint8_t *b, int32_t *out, cudaStream_t st) const
     {
-        SLCS_CUDA(cudaMemsetAsync(d_work, 0, work_bytes, st));
+        SLCS_CUDA(nrelay > 0 ? cudaMemsetAsync(d_relay_ws, 0, relay_ws_bytes, st)
+                             : cudaMemsetAsync(d_work, 0, work_bytes, st));
         slcs_status s;
-        if (stm > 0) {
+        if (nrelay > 0) {
+            RelayLaunch L{};
+            L.pairs = d_pairs;
+            L.items = d_relay;
+            L.nitems = nrelay;
+            L.a_blob = a;
+            L.b_blob = b;
+            L.out = out;
+            L.counters = reinterpret_cast<int32_t *>(d_relay_ws);
+            L.rows = reinterpret_cast<int2 *>(d_relay_ws + 16);
+            L.row_off = d_row_off;
+            L.status = device_status_word();
+            L.wait_ns = wait_ns;
+            s = launch_relay(L, relay, sm_count(), st);
+        } else if (stm > 0) {
             BatchLaunch B{launch(a, b, out), d_seg_off, d_seg_list, d_seg_list2, nwarps, grid, nclass, {}, {}};
             for (int c = 0; c < nclass; ++c) {
                 B.class_warp_end[c] = class_warp_end[c];
@@ -515,6 +601,36 @@ slcs_status slcs_device_status(int32_t device, int32_t clear)
     return SLCS_OK;
 }
 
+static slcs_status comb_pair_relay(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n, int32_t *h_out,
+                                   int32_t *v_out, const RelayShape &shape, const slcs_config *cfg, cudaStream_t st)
+{
+    RelayLaunch L{};
+    L.nitems = relay_groups(m, shape);
+    L.a_blob = a;
+    L.b_blob = b;
+    L.out = h_out;
+    L.v_single = v_out;
+    L.status = device_status_word();
+    L.wait_ns = wait_limit_ns(cfg);
+    L.single.m = m;
+    L.single.n = n;
+    char *ws = nullptr;
+    if (L.nitems > 1) { // one group hands nothing down
+        const size_t bytes = 16 + sizeof(int2) * size_t(relay_row_elems(m, n, shape));
+        SLCS_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&ws), bytes, st));
+        const cudaError_t e = cudaMemsetAsync(ws, 0, bytes, st);
+        if (e != cudaSuccess) {
+            cudaFreeAsync(ws, st);
+            return cuda_fail(e, "hand-down row");
+        }
+        L.counters = reinterpret_cast<int32_t *>(ws);
+        L.rows = reinterpret_cast<int2 *>(ws + 16);
+    }
+    const slcs_status s = launch_relay(L, shape, sm_count(), st);
+    if (ws) SLCS_CUDA(cudaFreeAsync(ws, st));
+    return s;
+}
+
 slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n, int32_t *h_out,
                            int32_t *v_out, const slcs_config *cfg, void *stream)
 {
@@ -528,8 +644,18 @@ slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_
     PairPlan pp;
     const slcs_status ps = plan_pair(m, n, cfg, sm_count(), &pp);
     if (ps != SLCS_OK) return ps;
+    if (pp.relay.relay.tm > 0) {
+        if (pp.relay.strips * pp.relay.bands == 1)
+            return comb_pair_relay(a, m, b, n, h_out, v_out, pp.relay.relay, cfg, st);
+        slcs_config rc{};
+        rc.strips = pp.relay.strips;
+        rc.bands = pp.relay.bands;
+        rc.braid_cutoff = cfg && cfg->braid_cutoff > 0 ? cfg->braid_cutoff : 256;
+        rc.wait_ms = cfg ? cfg->wait_ms : 0;
+        return comb_strips(a, m, b, n, h_out, v_out, &rc, 0, 0, &pp.relay.relay, st);
+    }
     const int tm = pp.c.tile_m;
-    if (pp.c.algo == SLCS_ALGO_STRIPS) return comb_strips(a, m, b, n, h_out, v_out, &pp.c, tm, pp.c.warps, st);
+    if (pp.c.algo == SLCS_ALGO_STRIPS) return comb_strips(a, m, b, n, h_out, v_out, &pp.c, tm, pp.c.warps, nullptr, st);
     const int32_t ntasks = stripes_of(m, tm);
     const size_t work_bytes = align_up(sizeof(int32_t) * (4 + size_t(ntasks)), 256);
     const size_t scr_bytes = sizeof(int32_t) * size_t(scratch_elems(m, n, tm));
@@ -1180,6 +1306,27 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
             }
         }
     }
+    // Relay items: the groups of every pair, largest pair first.
+    std::vector<int2> relay_items;
+    std::vector<int64_t> row_off;
+    if (P->relay.tm > 0) {
+        const slcs_status rs = launch_relay(RelayLaunch{}, P->relay, sm_count(), PREPARE_ONLY);
+        if (rs != SLCS_OK) {
+            delete P;
+            return rs;
+        }
+        int64_t row_elems = 0;
+        row_off.assign(npairs, 0);
+        for (int32_t p : S.order) {
+            if (pairs[p].m == 0 || pairs[p].n == 0) continue;
+            const int32_t groups = relay_groups(pairs[p].m, P->relay);
+            for (int32_t g = 0; g < groups; ++g) relay_items.push_back(make_int2(p, g));
+            row_off[p] = row_elems;
+            row_elems += relay_row_elems(pairs[p].m, pairs[p].n, P->relay);
+        }
+        P->nrelay = int32_t(relay_items.size());
+        P->relay_ws_bytes = 16 + sizeof(int2) * size_t(row_elems);
+    }
     P->work_bytes = align_up(sizeof(int32_t) * (WORK_HEAD + S.tasks.size()), 256);
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **ptr, size_t bytes) {
@@ -1208,6 +1355,15 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     alloc(reinterpret_cast<void **>(&P->d_scr_off), sizeof(int64_t) * size_t(npairs));
     alloc(reinterpret_cast<void **>(&P->d_scratch), sizeof(int32_t) * size_t(S.scratch_elems) + 16);
     alloc(reinterpret_cast<void **>(&P->d_work), P->work_bytes);
+    if (P->nrelay > 0) {
+        alloc(reinterpret_cast<void **>(&P->d_relay), sizeof(int2) * relay_items.size());
+        alloc(reinterpret_cast<void **>(&P->d_row_off), sizeof(int64_t) * row_off.size());
+        alloc(reinterpret_cast<void **>(&P->d_relay_ws), P->relay_ws_bytes);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(P->d_relay, relay_items.data(), sizeof(int2) * relay_items.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(P->d_row_off, row_off.data(), sizeof(int64_t) * row_off.size(), cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess && npairs)
         e = cudaMemcpy(P->d_pairs, pairs, sizeof(PairDev) * size_t(npairs), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !S.tasks.empty())
@@ -1251,6 +1407,13 @@ slcs_status slcs_pair_plan_info_sms(int32_t m, int32_t n, const slcs_config *cfg
         for (int32_t w : strip_widths(n, c.strips)) width = std::min<int64_t>(width, w);
     }
     info->cols_per_step = pick_tw(c.tile_m, chain, width, nullptr);
+    if (pp.relay.relay.tm > 0) {
+        info->relay_tile_m = pp.relay.relay.tm;
+        info->relay_cols = pp.relay.relay.tw;
+        info->relay_warps = pp.relay.relay.warps;
+        info->relay_strips = pp.relay.strips;
+        info->relay_bands = pp.relay.bands;
+    }
     return SLCS_OK;
 }
 
@@ -1480,6 +1643,9 @@ slcs_status slcs_batch_plan_destroy(slcs_batch_plan *P)
     cudaFree(P->d_seg_list2);
     cudaFree(P->d_pool_list);
     cudaFree(P->d_pool_list2);
+    cudaFree(P->d_relay);
+    cudaFree(P->d_row_off);
+    cudaFree(P->d_relay_ws);
     cudaFree(P->d_lane_map);
     cudaFree(P->d_tasks);
     cudaFree(P->d_scr_off);

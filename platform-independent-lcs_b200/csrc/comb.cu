@@ -42,6 +42,7 @@
 
 #include "cell.cuh"
 #include "comb.cuh"
+#include "occupancy.cuh"
 
 namespace slcs {
 
@@ -910,7 +911,6 @@ __global__ void strands_to_perm_kernel(const int32_t *__restrict__ h, int32_t m,
 // average 13.8 set the pace of the whole wavefront.)  Dynamic shared memory of
 // more than half an SM keeps a second block off every SM.
 constexpr int WF_SM_WARPS = 16;
-constexpr int MAX_DEVICES = 64;
 
 struct Balanced {
     bool ok = false;
@@ -968,33 +968,6 @@ slcs_status launch_balanced(const CombLaunch &L, long sms, cudaStream_t stream, 
     comb_wavefront_kernel<TM, WF_SM_WARPS, TW><<<int(grid), int(per_sm) * 32, size_t(B.smem), stream>>>(L);
     if (grid_out) *grid_out = int(grid);
     SLCS_CUDA(cudaGetLastError());
-    return SLCS_OK;
-}
-
-// Resident blocks per SM of one kernel on the current device (queried once
-// per kernel and device: occupancy belongs to a device, like function
-// attributes).  The kernel is a template argument, so that every kernel
-// keeps its own table.
-template <auto Kernel>
-slcs_status occupancy_of(int threads, int *occ_out)
-{
-    static int per_dev[MAX_DEVICES] = {}; // 0: not queried yet
-    static std::mutex mu;
-    int dev = 0;
-    SLCS_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
-    int *slot = (dev >= 0 && dev < MAX_DEVICES) ? &per_dev[dev] : nullptr;
-    if (!slot || *slot == 0) {
-        int occ = 0;
-        SLCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, Kernel, threads, 0));
-        if (occ < 1) occ = 1;
-        if (!slot) {
-            *occ_out = occ;
-            return SLCS_OK;
-        }
-        *slot = occ;
-    }
-    *occ_out = *slot;
     return SLCS_OK;
 }
 

@@ -11,7 +11,7 @@
 // slcs_probe_wait_expiry checks the failure path of the bounded waits on the
 // device: a stripe waits for a producer that never runs, the wait runs out,
 // and the launch ends with an error status instead of a hang.
-#include "comb.cuh"
+#include "relay.cuh"
 
 namespace slcs {
 namespace {
@@ -124,7 +124,8 @@ extern "C" SLCS_API slcs_status slcs_probe_wait_expiry(int32_t wait_ms, void *st
     // A pair of two row stripes (tile_m 2: 64 rows each) and 64 columns.
     constexpr int TM = 2, M = 128, N = 64;
     const size_t o_b = 256, o_out = 512, o_work = o_out + 256 * sizeof(int32_t), o_scr = o_work + 256;
-    const size_t bytes = o_scr + sizeof(int32_t) * size_t(scratch_elems(M, N, TM)) + 256;
+    const size_t o_row = o_scr + 256 + sizeof(int32_t) * size_t(scratch_elems(M, N, TM));
+    const size_t bytes = o_row + sizeof(int2) * N;
     char *ws = nullptr;
     (void)sm_count(); // per-device set-up (memory pool, status word) before the allocation
     SLCS_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&ws), bytes, st));
@@ -144,7 +145,29 @@ extern "C" SLCS_API slcs_status slcs_probe_wait_expiry(int32_t wait_ms, void *st
     L.wait_ns = uint64_t(wait_ms) * 1000000ull;
     L.single.m = M;
     L.single.n = N;
-    const slcs_status s = launch_comb(L, TM, 4, st, nullptr);
+    slcs_status s = launch_comb(L, TM, 4, st, nullptr);
+    // The same for the relay kernel: two groups, the first never claimed, so
+    // that no entry of the hand-down row carries the number that the second
+    // waits for.
+    constexpr RelayShape shape{1, 4, 3}; // 96 rows per group
+    if (s == SLCS_OK) {
+        cudaError_t e = cudaMemsetAsync(ws + o_out, 0, bytes - o_out, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ws + o_work, 1, 1, st);
+        if (e != cudaSuccess) s = cuda_fail(e, "cudaMemsetAsync");
+        RelayLaunch R{};
+        R.nitems = relay_groups(M, shape);
+        R.a_blob = L.a_blob;
+        R.b_blob = L.b_blob;
+        R.out = L.out;
+        R.v_single = L.out + M;
+        R.counters = L.counters;
+        R.rows = reinterpret_cast<int2 *>(ws + o_row);
+        R.status = L.status;
+        R.wait_ns = L.wait_ns;
+        R.single.m = M;
+        R.single.n = N;
+        if (s == SLCS_OK) s = launch_relay(R, shape, sm_count(), st);
+    }
     SLCS_CUDA(cudaFreeAsync(ws, st));
     return s;
 }

@@ -215,8 +215,9 @@ slcs_status perm_to_strands(const int32_t *r2c, int32_t m, int32_t n, int32_t *h
 }
 
 slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n, int32_t *h_out, int32_t *v_out,
-                        const slcs_config *cfg, int tm, int warps, cudaStream_t st)
+                        const slcs_config *cfg, int tm, int warps, const RelayShape *relay, cudaStream_t st)
 {
+    if (relay) tm = relay->tm;
     const int R = band_count(cfg, m, tm);
     const int S = strip_count(cfg, n);
     const std::vector<int32_t> hgt = band_heights(m, R, tm);
@@ -238,16 +239,17 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         }
     }
     const int64_t total = o0; // S*m + R*n strands
-    // Schedule of the wavefront launch: the stripes of every tile, tile after
-    // tile, so that a stripe's producer is the task before it.
+    // Schedule of the comb: the stripes (relay: groups of stripes) of every
+    // tile, tile after tile, so that a stripe's producer is the task before it.
     std::vector<int2> tasks;
     std::vector<int64_t> scr_off(size_t(T), 0);
-    int64_t scr_elems = 0;
+    int64_t scr_elems = 0; // int32 of the wavefront's scratch, int2 of the relay's rows
     for (int t = 0; t < T; ++t) {
-        const int32_t st_count = stripes_of(pd[size_t(t)].m, tm);
-        for (int32_t k = 0; k < st_count; ++k) tasks.push_back(make_int2(t, k));
+        const slcs_pair_desc &d = pd[size_t(t)];
+        const int32_t count = relay ? relay_groups(d.m, *relay) : stripes_of(d.m, tm);
+        for (int32_t k = 0; k < count; ++k) tasks.push_back(make_int2(t, k));
         scr_off[size_t(t)] = scr_elems;
-        scr_elems += scratch_elems(pd[size_t(t)].m, pd[size_t(t)].n, tm);
+        scr_elems += relay ? relay_row_elems(d.m, d.n, *relay) : scratch_elems(d.m, d.n, tm);
     }
     const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 1024;
     // Products glue strips with overlap = band height and bands with overlap
@@ -260,9 +262,12 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     const size_t o_tasks = align256(o_pairs + sizeof(PairDev) * size_t(T));
     const size_t o_soff = align256(o_tasks + sizeof(int2) * tasks.size());
     const size_t o_work = align256(o_soff + sizeof(int64_t) * size_t(T));
-    const size_t work_bytes = align256(sizeof(int32_t) * (4 + tasks.size()));
+    // The counters and, after them, what must be zero with them: the
+    // wavefront's progress or the relay's rows.
+    const size_t scr_bytes = size_t(scr_elems) * (relay ? sizeof(int2) : sizeof(int32_t));
+    const size_t work_bytes = align256(relay ? 16 + scr_bytes : sizeof(int32_t) * (4 + tasks.size()));
     const size_t o_scr = o_work + work_bytes;
-    const size_t o_x = align256(o_scr + sizeof(int32_t) * size_t(scr_elems) + 16);
+    const size_t o_x = align256(o_scr + (relay ? 0 : scr_bytes + 16));
     const size_t o_y = align256(o_x + sizeof(int32_t) * size_t(total));
     const size_t o_braid = align256(o_y + sizeof(int32_t) * size_t(total));
     const int most = std::max(R * (S / 2), R / 2); // products of the widest merge level
@@ -284,7 +289,21 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     cu(cudaMemsetAsync(ws + o_work, 0, work_bytes, st), "counters");
     int32_t *X = reinterpret_cast<int32_t *>(ws + o_x);
     int32_t *Y = reinterpret_cast<int32_t *>(ws + o_y);
-    if (s == SLCS_OK) {
+    if (s == SLCS_OK && relay) {
+        RelayLaunch L{};
+        L.pairs = reinterpret_cast<const PairDev *>(ws + o_pairs);
+        L.items = reinterpret_cast<const int2 *>(ws + o_tasks);
+        L.nitems = int32_t(tasks.size());
+        L.a_blob = a;
+        L.b_blob = b;
+        L.out = X;
+        L.counters = reinterpret_cast<int32_t *>(ws + o_work);
+        L.rows = reinterpret_cast<int2 *>(ws + o_work + 16);
+        L.row_off = reinterpret_cast<const int64_t *>(ws + o_soff);
+        L.status = device_status_word();
+        L.wait_ns = wait_limit_ns(cfg);
+        s = launch_relay(L, *relay, sm_count(), st);
+    } else if (s == SLCS_OK) {
         CombLaunch L{};
         L.pairs = reinterpret_cast<const PairDev *>(ws + o_pairs);
         L.tasks = reinterpret_cast<const int2 *>(ws + o_tasks);

@@ -4,7 +4,7 @@
 
 #include <vector>
 
-#include "slcs_internal.cuh"
+#include "relay.cuh"
 
 namespace slcs {
 
@@ -19,8 +19,9 @@ std::vector<int32_t> band_heights(int32_t m, int bands, int tm);
 // Strands of P(a, b) from its row -> col array.
 slcs_status perm_to_strands(const int32_t *r2c, int32_t m, int32_t n, int32_t *h, int32_t *v, cudaStream_t st);
 // Comb (a, b) as band x strip tiles and merge them; the result equals the
-// direct comb.
+// direct comb.  With `relay` the tiles are combed by the relay kernel of that
+// shape (cfg's strips and bands say how many), else by the wavefront kernel.
 slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n, int32_t *h_out, int32_t *v_out,
-                        const slcs_config *cfg, int tm, int warps, cudaStream_t st);
+                        const slcs_config *cfg, int tm, int warps, const RelayShape *relay, cudaStream_t st);
 
 } // namespace slcs

@@ -61,7 +61,9 @@ class PlanInfo(ctypes.Structure):
 class PairInfo(ctypes.Structure):
     _fields_ = [("algo", ctypes.c_int32), ("tile_m", ctypes.c_int32), ("warps", ctypes.c_int32),
                 ("strips", ctypes.c_int32), ("bands", ctypes.c_int32), ("braid_cutoff", ctypes.c_int32),
-                ("stripes", ctypes.c_int32), ("cols_per_step", ctypes.c_int32), ("reserved", ctypes.c_int32 * 8)]
+                ("stripes", ctypes.c_int32), ("cols_per_step", ctypes.c_int32), ("relay_tile_m", ctypes.c_int32),
+                ("relay_cols", ctypes.c_int32), ("relay_warps", ctypes.c_int32), ("relay_strips", ctypes.c_int32),
+                ("relay_bands", ctypes.c_int32), ("reserved", ctypes.c_int32 * 3)]
 
     def as_dict(self):
         return {k: int(getattr(self, k)) for k, _ in self._fields_ if k != "reserved"}
