@@ -236,12 +236,17 @@ typedef struct {
     int32_t wavefront_tile_m;/* rows per lane of wavefront stripes                  */
     int32_t warps;           /* warps per block                                     */
     int32_t stream_pairs;    /* pairs combed in stream mode                         */
-    int32_t wavefront_tasks; /* row stripes combed as wavefront tasks               */
+    int32_t wavefront_tasks; /* row stripes of wavefront plans; in others the stripes of
+                                wavefront_tile_m rows per lane that the taller pairs have */
     int32_t stream_classes;  /* stream classes in use                               */
     int32_t tile_n;          /* stream columns per step                             */
     int32_t grid;            /* blocks of the launch                                */
     int32_t packed_pairs;    /* stream pairs combed two per register (16-bit ids)   */
-    int32_t reserved[2];
+    /* Groups of stripes combed by the relay kernel: those of the pairs that do
+     * not stream, or (relay_all) of every pair, in which case the fields above
+     * say what a configuration naming a variant would get.                     */
+    int32_t relay_groups;
+    int32_t relay_all;
 } slcs_plan_info;
 SLCS_API slcs_status slcs_batch_plan_info(const slcs_batch_plan *plan, slcs_plan_info *info);
 

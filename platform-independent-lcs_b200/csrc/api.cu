@@ -10,10 +10,12 @@
 #include <numeric>
 #include <queue>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "braid.cuh"
 #include "comb.cuh"
+#include "couples.cuh"
 #include "queries.cuh"
 #include "relay.cuh"
 #include "strips.cuh"
@@ -232,6 +234,39 @@ RelayPlan plan_relay(int32_t m, int32_t n, int sms)
     return best;
 }
 
+// Instructions a combing warp of a relay shape issues per step (about; B200,
+// counted for (4, 4) and scaled by cells), the I/O warp about 12.
+double relay_issue(const RelayShape &s) { return 4.3 * s.tm * s.tw + 10.0 + 3.0 * s.tw; }
+
+// Microseconds the relay kernel takes for the pairs that `take` selects, with
+// the best shape: its longest chain plus its blocks' issue slots, spread over
+// the SMs (on B200 within a factor of 0.85 to 1.7 of sweeps from 64 reads to
+// 1,000 pairs of 9000 x 100 rows and columns).
+template <class Take>
+double batch_relay_us(const slcs_pair_desc *pairs, int32_t npairs, int sms, Take take, RelayShape *shape)
+{
+    double best = -1.0;
+    for (const RelayCost &c : RELAY_COSTS) {
+        const RelayShape &s = c.shape;
+        const double issue = relay_issue(s);
+        double chain = 0, slots = 0;
+        for (int32_t p = 0; p < npairs; ++p) {
+            if (!take(p) || pairs[p].m == 0 || pairs[p].n == 0) continue;
+            const int32_t stripes = (pairs[p].m + 32 * s.tm - 1) / (32 * s.tm);
+            const int32_t groups = (stripes + s.warps - 1) / s.warps;
+            const double own = double(pairs[p].n) / s.tw + 31.0; // steps of one warp
+            chain = std::max(chain, own + RELAY_WARP_LAG * stripes + RELAY_HOP_LAG * groups);
+            slots += stripes * own * issue + groups * (own + RELAY_WARP_LAG * (s.warps - 1)) * 12.0;
+        }
+        const double us = 8.0 + 1.2 * (chain * c.step + slots / (4.0 * sms)) / (RELAY_GHZ * 1e3);
+        if (best < 0 || us < best) {
+            best = us;
+            *shape = s;
+        }
+    }
+    return best;
+}
+
 // How slcs_comb_pair combs one pair: the effective configuration (algo
 // WAVEFRONT or STRIPS with tile_m, warps, strips, bands, braid_cutoff set),
 // and the relay plan that takes its place when nothing is configured and the
@@ -379,8 +414,6 @@ using namespace slcs;
 
 struct StreamClass {
     int tm, seg;  // rows per lane, lanes per segment
-    bool packed;
-    bool var = false; // a lane count of the variable packed class (segments share warps)
 };
 
 // Relative time of one step of a warp of a stream class (all its segments
@@ -388,29 +421,20 @@ struct StreamClass {
 // warp's pace is not its own instruction count: the warps of an SM
 // sub-partition share its issue slots and integer pipe, so the classes differ
 // less than their rows per lane do.  Fitted to B200 per-warp clocks of the
-// 20,000 read/window pairs (4 columns per step, 8 warps per SM): packed
-// classes of 4, 8, 12 and 16 rows per lane 1554, 1327, 1392 and 1909 ns per
-// step, 32-bit 32-lane classes of 12 and 16 rows 1348 and 1500 ns.  Plans
-// with 8 columns per step weigh every class alike (no measurements).
+// 20,000 read/window pairs (4 columns per step): 32-lane classes of 12 and 16
+// rows 1348 and 1500 ns.  Plans with 8 columns per step weigh every class
+// alike (no measurements).
 static double class_step_time(const StreamClass &k, int tns)
 {
     if (tns != 4) return 1.0;
-    if (k.packed) {
-        switch (k.tm) {
-        case 4: return 1554.0;
-        case 8: return 1327.0;
-        case 12: return 1392.0;
-        default: return 1909.0;
-        }
-    }
     if (k.seg == 32) return k.tm <= 12 ? 1348.0 : 1500.0;
-    return 1000.0 + 30.0 * k.tm; // 16-lane 32-bit classes: between the two above
+    return 1000.0 + 30.0 * k.tm; // 16-lane classes: between the two above
 }
 
 // Head of a batch plan's work buffer: counters [0] wavefront ticket and [1]
-// abort, [2..3] unused, then MAX_POOLS pool tickets;
-// the wavefront progress counters follow.
-static constexpr int WORK_HEAD = 4 + MAX_POOLS;
+// abort, [2] ticket of the staged bundles, [3] unused, then MAX_CLASSES pool
+// tickets; the wavefront progress counters follow.
+static constexpr int WORK_HEAD = 4 + MAX_CLASSES;
 
 struct slcs_batch_plan {
     int device = 0;
@@ -428,29 +452,40 @@ struct slcs_batch_plan {
     int32_t nclass = 0; // classes with warps
     int32_t class_warp_end[MAX_CLASSES] = {};
     int32_t class_code[MAX_CLASSES] = {};
-    int32_t class_pool[MAX_CLASSES] = {};
-    std::vector<int32_t> lane_map; // the variable class's warps: 32 entries each (BatchLaunch::lane_map)
-    int32_t *d_lane_map = nullptr;
     int32_t nwarps = 0; // warps with a stream class
     int grid = 0;       // blocks of the batch launch
     uint64_t wait_ns = DEFAULT_WAIT_NS;
     bool use_graph = false;
+    char *d_block = nullptr; // every device array of the plan lies in it
     PairDev *d_pairs = nullptr;
     int32_t *d_seg_off = nullptr;
     int32_t *d_seg_list = nullptr;
-    int32_t *d_seg_list2 = nullptr;
     int32_t *d_pool_list = nullptr;
-    int32_t *d_pool_list2 = nullptr;
-    int32_t pool_off[MAX_POOLS + 1] = {};
+    int32_t pool_off[MAX_CLASSES + 1] = {};
+    int couple_tm = 0; // rows per lane of the packed pairs (0: none)
+    int depth = 0;     // their warps per SM sub-partition (0: the default)
+    CoupleDev *d_couples = nullptr;
+    int32_t *d_others = nullptr; // pairs not in couples
+    int32_t nothers = 0;
+    int32_t nstaged = 0, ncouples = 0, nstaged_bundles = 0, nlists = 0;
+    int32_t *d_list_off = nullptr; // of the bundles that are not staged
+    uint4 *d_couple_stage = nullptr;
+    BundleLane *d_bundles = nullptr;
     int pool_pct = 15;
     int2 *d_tasks = nullptr;
     int64_t *d_scr_off = nullptr;
     int32_t *d_scratch = nullptr;
     int32_t *d_work = nullptr; // [counters(4) | progress(ntasks)]
     size_t work_bytes = 0;
-    // Pairs combed by the relay kernel instead (relay.tm > 0): all of the plan.
+    // Pairs combed by the relay kernel: those too tall to stream (few of them
+    // beside the couples, on a stream of their own and SMs left to them, else
+    // after the others), or all of the plan.
     RelayShape relay{};
-    int32_t nrelay = 0;         // groups of all pairs
+    bool relay_all = false;
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int32_t nrelay = 0;         // groups of those pairs
+    int32_t relay_sms = 0;      // SMs the couples leave to them
     int2 *d_relay = nullptr;    // (pair, group)
     int64_t *d_row_off = nullptr;
     char *d_relay_ws = nullptr; // counters and hand-down rows, cleared by every run
@@ -500,40 +535,22 @@ struct slcs_batch_plan {
         return L;
     }
 
-    slcs_status enqueue(const uint8_t *a, const uint8_t *b, int32_t *out, cudaStream_t st) const
+    // With out16 the couples' strands go there, as int16, and the others' to out.
+    slcs_status enqueue(const uint8_t *a, const uint8_t *b, int32_t *out, int16_t *out16, cudaStream_t st) const
     {
-        SLCS_CUDA(nrelay > 0 ? cudaMemsetAsync(d_relay_ws, 0, relay_ws_bytes, st)
-                             : cudaMemsetAsync(d_work, 0, work_bytes, st));
-        slcs_status s;
-        if (nrelay > 0) {
-            RelayLaunch L{};
-            L.pairs = d_pairs;
-            L.items = d_relay;
-            L.nitems = nrelay;
-            L.a_blob = a;
-            L.b_blob = b;
-            L.out = out;
-            L.counters = reinterpret_cast<int32_t *>(d_relay_ws);
-            L.rows = reinterpret_cast<int2 *>(d_relay_ws + 16);
-            L.row_off = d_row_off;
-            L.status = device_status_word();
-            L.wait_ns = wait_ns;
-            s = launch_relay(L, relay, sm_count(), st);
-        } else if (stm > 0) {
-            BatchLaunch B{launch(a, b, out), d_seg_off, d_seg_list, d_seg_list2, nwarps, grid, nclass, {}, {}};
-            for (int c = 0; c < nclass; ++c) {
-                B.class_warp_end[c] = class_warp_end[c];
-                B.class_code[c] = class_code[c];
-                B.class_pool[c] = class_pool[c];
-            }
-            B.lane_map = d_lane_map;
-            B.pool_list = d_pool_list;
-            B.pool_list2 = d_pool_list2;
-            B.pool_ticket = d_work + 4;
-            for (int c = 0; c <= MAX_POOLS; ++c) B.pool_off[c] = pool_off[c];
-            s = launch_batch(B, tns, st, nullptr);
+        slcs_status s = SLCS_OK;
+        if (relay_all) {
+            s = enqueue_relay(a, b, out, st);
+        } else if (!side) {
+            s = enqueue_rest(a, b, out, out16, st);
+            if (s == SLCS_OK) s = enqueue_relay(a, b, out, st);
         } else {
-            s = launch_comb(launch(a, b, out), tm, warps, st, nullptr);
+            SLCS_CUDA(cudaEventRecord(fork, st));
+            SLCS_CUDA(cudaStreamWaitEvent(side, fork, 0));
+            s = enqueue_relay(a, b, out, side);
+            SLCS_CUDA(cudaEventRecord(join, side));
+            if (s == SLCS_OK) s = enqueue_rest(a, b, out, out16, st);
+            SLCS_CUDA(cudaStreamWaitEvent(st, join, 0));
         }
         if (s != SLCS_OK) return s;
         for (const auto &d : empty_pairs) {
@@ -541,6 +558,51 @@ struct slcs_batch_plan {
             if (s != SLCS_OK) return s;
         }
         return SLCS_OK;
+    }
+
+    slcs_status enqueue_relay(const uint8_t *a, const uint8_t *b, int32_t *out, cudaStream_t st) const
+    {
+        if (nrelay <= 0) return SLCS_OK;
+        SLCS_CUDA(cudaMemsetAsync(d_relay_ws, 0, relay_ws_bytes, st));
+        RelayLaunch L{};
+        L.pairs = d_pairs;
+        L.items = d_relay;
+        L.nitems = nrelay;
+        L.a_blob = a;
+        L.b_blob = b;
+        L.out = out;
+        L.counters = reinterpret_cast<int32_t *>(d_relay_ws);
+        L.rows = reinterpret_cast<int2 *>(d_relay_ws + 16);
+        L.row_off = d_row_off;
+        L.status = device_status_word();
+        L.wait_ns = wait_ns;
+        return launch_relay(L, relay, sm_count(), st);
+    }
+
+    // The streamed pairs, or all pairs of a wavefront plan.
+    slcs_status enqueue_rest(const uint8_t *a, const uint8_t *b, int32_t *out, int16_t *out16, cudaStream_t st) const
+    {
+        if (stm > 0 ? nstream <= 0 : ntasks <= 0) return SLCS_OK;
+        if (stm <= 0 || nstaged > 0 || nwarps > 0) SLCS_CUDA(cudaMemsetAsync(d_work, 0, work_bytes, st));
+        if (stm > 0) {
+            CouplesLaunch C{a,      b,       out,            out16,           d_couples, nstaged, d_couple_stage,
+                            d_bundles, nstaged_bundles, nlists, d_list_off, d_work + 2};
+            if (ncouples > 0) {
+                const slcs_status s = launch_couples(C, couple_tm, depth, relay_sms > 0, sm_count(), st);
+                if (s != SLCS_OK) return s;
+            }
+            if (nwarps <= 0) return SLCS_OK;
+            BatchLaunch B{launch(a, b, out), d_seg_off, d_seg_list, nwarps, grid, nclass, {}, {}};
+            for (int c = 0; c < nclass; ++c) {
+                B.class_warp_end[c] = class_warp_end[c];
+                B.class_code[c] = class_code[c];
+            }
+            B.pool_list = d_pool_list;
+            B.pool_ticket = d_work + 4;
+            for (int c = 0; c <= MAX_CLASSES; ++c) B.pool_off[c] = pool_off[c];
+            return launch_batch(B, tns, st, nullptr);
+        }
+        return launch_comb(launch(a, b, out), tm, warps, st, nullptr);
     }
 };
 
@@ -810,7 +872,7 @@ slcs_status slcs_comb_pair_words_host(const int32_t *a, int32_t m, const int32_t
 }
 
 static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_desc *pairs, int32_t npairs,
-                                    const slcs_config *cfg, bool var_class = true);
+                                    const slcs_config *cfg, bool chunk = false);
 static void plan_add_chunks(slcs_batch_plan *P, const slcs_pair_desc *pairs, int32_t npairs, const slcs_config *cfg);
 
 slcs_status slcs_batch_plan_create(slcs_batch_plan **plan_out, const slcs_pair_desc *pairs, int32_t npairs,
@@ -824,10 +886,10 @@ slcs_status slcs_batch_plan_create(slcs_batch_plan **plan_out, const slcs_pair_d
 // Chunks for host runs (an optimisation only: without them run_host copies
 // everything in, combs, and copies everything out).  Made for batches of at
 // least CHUNK_MIN_PAIRS pairs whose chunks' byte ranges do not overlap.
-// 12 chunks: the 20,000 reads' int16 host run took 0.578 ms against 0.61 ms
-// with 4, 6, 8 or 16 chunks on one B200 (int32 strands: 0.755 against
-// 0.77-0.84 ms).
-static constexpr int HOST_CHUNKS = 12;
+// 4 chunks: the 20,000 reads' int16 host run took 0.42 ms, with 2, 3 and 6
+// chunks 0.44, 0.43 and 0.44 ms (one B200; the copies alone take 0.38 ms one
+// after the other, and every chunk costs the host a dozen calls).
+static constexpr int HOST_CHUNKS = 4;
 static constexpr int32_t CHUNK_MIN_PAIRS = 8192;
 
 static void plan_add_chunks(slcs_batch_plan *P, const slcs_pair_desc *pairs, int32_t npairs, const slcs_config *cfg)
@@ -860,7 +922,7 @@ static void plan_add_chunks(slcs_batch_plan *P, const slcs_pair_desc *pairs, int
             k.o_hi = std::max(k.o_hi, d.out_offset + d.m + d.n);
         }
         // Sub-plan over the chunk's pairs (offsets stay global).
-        if (plan_create_impl(&k.plan, pairs + p0, p1 - p0, cfg, false) != SLCS_OK) {
+        if (plan_create_impl(&k.plan, pairs + p0, p1 - p0, cfg, true) != SLCS_OK) {
             for (auto &x : ch) slcs_batch_plan_destroy(x.plan);
             if (k.plan) slcs_batch_plan_destroy(k.plan);
             return;
@@ -901,8 +963,83 @@ static void plan_add_chunks(slcs_batch_plan *P, const slcs_pair_desc *pairs, int
     P->chunks = std::move(ch);
 }
 
+// Bundles of couples [k0, k1) side by side in a warp: longest couple first,
+// each into the first bundle with lanes left whose length it comes near (within
+// BUNDLE_SLACK), else into a new one; at most `blocks` blocks together.
+static void make_bundles(const std::vector<CoupleDev> &couples, size_t k0, size_t k1, int tm, int64_t blocks,
+                         std::vector<BundleLane> &out)
+{
+    constexpr double BUNDLE_SLACK = 0.6; // 0.85 left 5 % more steps on the 20,000 reads
+    struct Open {
+        int32_t index, room, steps, used;
+    };
+    auto lanes_of = [&](const CoupleDev &k) { return k.rows / tm; };
+    auto steps_of = [&](const CoupleDev &k) { return k.nb + lanes_of(k) - 1; };
+    std::vector<int32_t> order(k1 - k0);
+    std::iota(order.begin(), order.end(), int32_t(k0));
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int32_t x, int32_t y) { return steps_of(couples[x]) > steps_of(couples[y]); });
+    std::vector<Open> open;
+    for (int32_t i : order) {
+        const CoupleDev &k = couples[size_t(i)];
+        const int lanes = lanes_of(k), steps = steps_of(k);
+        size_t w = 0, keep = 0;
+        for (size_t x = 0; x < open.size(); ++x) // bundles too long for this couple are closed
+            if (double(open[x].steps) * BUNDLE_SLACK <= double(steps)) open[keep++] = open[x];
+        open.resize(keep);
+        while (w < open.size() && (open[w].room < lanes || open[w].used + k.nb > blocks)) ++w;
+        if (w == open.size()) {
+            open.push_back({int32_t(out.size() / 32), 32, steps, 0});
+            out.insert(out.end(), 32, BundleLane{-1, 0, 1, 0, steps});
+        }
+        Open &o = open[w];
+        BundleLane *b = &out[size_t(o.index) * 32 + size_t(32 - o.room)];
+        for (int l = 0; l < lanes; ++l) b[l] = BundleLane{i, int16_t(l), int16_t(lanes), o.used, o.steps};
+        o.room -= lanes;
+        o.used += k.nb;
+        if (o.room == 0) open.erase(open.begin() + long(w));
+    }
+}
+
+// Deal the bundles from the first on out to at most `most` lists, longest
+// first to the least loaded one, and put them in the order of the lists;
+// off: where each list starts among them, and their number.
+static void deal_bundles(std::vector<BundleLane> &lanes, size_t first, int most, std::vector<int32_t> &off)
+{
+    const size_t count = lanes.size() / 32 - first;
+    const size_t nlists = std::min(count, size_t(most));
+    off.assign(1, 0);
+    if (count == 0) return;
+    constexpr int64_t BUNDLE_COST = 12; // filling and emptying a bundle, in steps
+    std::vector<int32_t> order(count);
+    std::iota(order.begin(), order.end(), 0);
+    auto steps = [&](int32_t k) { return lanes[(first + size_t(k)) * 32].steps; };
+    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return steps(x) > steps(y); });
+    using Load = std::pair<int64_t, int32_t>;
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+    for (size_t l = 0; l < nlists; ++l) heap.push({0, int32_t(l)});
+    std::vector<std::vector<int32_t>> list(nlists);
+    for (int32_t k : order) {
+        Load top = heap.top();
+        heap.pop();
+        list[size_t(top.second)].push_back(k);
+        top.first += steps(k) + BUNDLE_COST;
+        heap.push(top);
+    }
+    std::vector<BundleLane> dealt;
+    dealt.reserve(count * 32);
+    for (const auto &l : list) {
+        for (int32_t k : l) {
+            const auto b = lanes.begin() + long((first + size_t(k)) * 32);
+            dealt.insert(dealt.end(), b, b + 32);
+        }
+        off.push_back(int32_t(dealt.size() / 32));
+    }
+    std::copy(dealt.begin(), dealt.end(), lanes.begin() + long(first * 32));
+}
+
 static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_desc *pairs, int32_t npairs,
-                                    const slcs_config *cfg, bool var_class)
+                                    const slcs_config *cfg, bool chunk)
 {
     if (!plan_out) return fail(SLCS_ERR_INVALID, "plan is null");
     *plan_out = nullptr;
@@ -938,7 +1075,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     } else {
         // Stream mode: pairs of at most 512 rows stream through segments,
         // each pair in the smallest class whose segment holds all its rows;
-        // taller pairs run as wavefront tasks of BATCH_WF_TM rows per lane.
+        // taller pairs are the relay kernel's (P->tm only counts their stripes).
         // A configuration naming tile_m (and seg) asks for that one class.
         P->tm = BATCH_WF_TM;
         const int bits = cfg ? cfg->strand_bits : 0;
@@ -956,52 +1093,37 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
             delete P;
             return fail(SLCS_ERR_UNSUPPORTED, "stream mode needs tile_n 4 or 8");
         }
-        const bool pack = bits != 32 && P->tns == 4;
+        // Long packed pairs are staged in 8 bytes per row and column of a couple;
+        // batches beyond 16 GiB of that comb 32-bit strands.
+        int64_t ids = 0;
+        for (int32_t p = 0; p < npairs; ++p) ids += int64_t(pairs[p].m) + pairs[p].n + 64;
+        const bool pack = bits != 32 && P->tns == 4 && 8 * ids < (int64_t(16) << 30);
+        // Packed pairs are combed in couples of as many lanes as their rows
+        // need, 16 rows per lane; a configuration naming tile_m (and 16 lanes)
+        // asks for couples of 16 lanes of that height.
         if (cfg && cfg->tile_m) {
             P->stm = cfg->tile_m;
             P->seg = cfg->seg ? cfg->seg : 16;
-            if (pack && packed16_supported(P->stm, P->seg)) P->classes.push_back({P->stm, P->seg, true});
-            P->classes.push_back({P->stm, P->seg, false});
+            if (pack && packed16_supported(P->stm, P->seg)) P->couple_tm = P->stm;
+            P->classes.push_back({P->stm, P->seg});
         } else {
             P->stm = 16;
             P->seg = 16;
-            // Packed pairs: the variable class, one item class per lane count
-            // (16 rows per lane, segments of VAR_MIN_LANES..32 lanes side by
-            // side in a warp), so that a pair's rows are padded to a multiple
-            // of 16 rather than to one of a few class heights.
-            // (The sub-plans of a chunked host run keep the fixed packed
-            // classes at 8 warps per SM: their chunks of ~1,700 pairs measured
-            // 0.584 ms per host run that way, 0.656 ms with the variable class.)
-            if (pack && var_class)
-                for (int l = VAR_MIN_LANES; l <= 32; ++l) P->classes.push_back({VAR_TM, l, true, true});
-            else if (pack)
-                for (int t : {4, 8, 12, 16}) P->classes.push_back({t, 16, true});
-            for (int t : {4, 8, 12, 16}) P->classes.push_back({t, 16, false});
-            P->classes.push_back({12, 32, false});
-            P->classes.push_back({16, 32, false});
+            if (pack) P->couple_tm = COUPLE_TM;
+            for (int t : {4, 8, 12, 16}) P->classes.push_back({t, 16});
+            P->classes.push_back({12, 32});
+            P->classes.push_back({16, 32});
         }
         for (const auto &c : P->classes)
-            if (!c.var && (c.packed ? !packed16_supported(c.tm, c.seg) : !stream_variant_supported(c.tm, c.seg))) {
+            if (!stream_variant_supported(c.tm, c.seg)) {
                 delete P;
                 return fail(SLCS_ERR_UNSUPPORTED, "stream mode needs tile_m in {4,8,12,16} and seg in {8,16,32}");
             }
-        // Packed plans: half of each class's work in its pool.  Fixed packed
-        // classes (16-lane segments) run 8 warps per SM: a packed item is a
-        // couple of pairs, and with 16 warps per SM a segment combed only one
-        // or two of them, so the launch ended with whichever segments drew
-        // two; at 8 warps per SM each warp runs twice as fast and combs twice
-        // as many items (20,000 reads on B200: 0.381 -> 0.328 ms).  The
-        // variable class keeps the full occupancy: its segments are as short
-        // as their pairs allow, so many more of them run side by side
-        // (0.340 ms at 8 warps per SM, 0.318 ms at 16).  32-bit plans keep
-        // the full occupancy too (2 blocks per SM: 0.361 -> 0.420 ms) and a
-        // 15 % pool.
-        const bool packed_plan = pack && std::any_of(P->classes.begin(), P->classes.end(),
-                                                     [](const StreamClass &k) { return k.packed; });
-        const bool var_plan = std::any_of(P->classes.begin(), P->classes.end(),
-                                          [](const StreamClass &k) { return k.var; });
-        P->blocks_per_sm = (cfg && cfg->blocks_per_sm > 0) ? cfg->blocks_per_sm : (packed_plan && !var_plan ? 2 : 0);
-        P->pool_pct = packed_plan ? 50 : 15;
+        // 32-bit classes run at full occupancy (2 blocks per SM: 361 -> 420 us
+        // on the 20,000 reads) with 15 % of a class's work in its pool.
+        P->blocks_per_sm = (cfg && cfg->blocks_per_sm > 0) ? cfg->blocks_per_sm : 0;
+        P->depth = P->blocks_per_sm;
+        P->pool_pct = 15;
         if (cfg && cfg->pool_pct != 0) P->pool_pct = cfg->pool_pct < 0 ? 0 : std::min(cfg->pool_pct, 90);
     }
     for (int32_t p = 0; p < npairs; ++p) {
@@ -1014,6 +1136,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     P->wide = wide_ids(P->max_ids, 0, wavefront_only ? cfg : nullptr);
     if (P->wide && !wavefront_only) { // the batch kernel has only the fast cell rule
         P->stm = 0;
+        P->couple_tm = 0;
         P->classes.clear();
     }
     int32_t stream_rows = 0;
@@ -1029,287 +1152,222 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         dummy.ntasks = 1;
         slcs_status ps = P->stm > 0 ? launch_batch(BatchLaunch{dummy}, P->tns, PREPARE_ONLY, &full_grid)
                                     : launch_comb(dummy, P->tm, P->warps, PREPARE_ONLY, nullptr);
+        if (ps == SLCS_OK && P->couple_tm > 0) ps = launch_couples(CouplesLaunch{}, P->couple_tm, 0, false, 1, PREPARE_ONLY);
         if (ps != SLCS_OK) {
             delete P;
             return ps;
         }
     }
     P->nstream = int32_t(S.stream_pairs.size());
-    // Stream classes, warps and pair lists.  A pair costs its column blocks
-    // plus a switch; each class gets warps in proportion to its cost per
-    // warp (a warp runs 32/seg segments side by side), and within a class
-    // the pairs go longest first to the least loaded segment.  The grid is
-    // the persistent one (or blocks_per_sm per SM), fewer for small batches.
-    std::vector<int32_t> seg_off, seg_list, seg_list2, pool_list, pool_list2;
-    if (P->stm > 0) {
+    // The pairs too tall to stream: the relay shape, and whether a quarter of
+    // the SMs holds all their groups.
+    const int sms = sm_count();
+    auto tall = [&](int32_t p) { return pairs[p].m > stream_rows; };
+    double tall_us = 0.0;
+    if (P->stm > 0 && P->ntasks > 0) {
+        tall_us = batch_relay_us(pairs, npairs, sms, tall, &P->relay);
+        int64_t groups = 0;
+        for (int32_t p = 0; p < npairs; ++p)
+            if (tall(p) && pairs[p].n > 0) groups += relay_groups(pairs[p].m, P->relay);
+        if (groups <= sms / 4) P->relay_sms = int32_t(groups);
+    }
+    // Couples of the packed pairs and their bundles.
+    std::vector<CoupleDev> couples;
+    std::vector<BundleLane> bundle_lanes;
+    std::vector<int32_t> list_off;
+    int64_t stage_elems = COUPLE_HEAD;
+    std::vector<int32_t> single_pairs; // streamed with 32-bit strands, largest first
+    std::vector<char> in_couple(size_t(npairs), 0);
+    {
+        const int tm = P->couple_tm;
+        const int fixed = cfg && cfg->tile_m ? 16 : 0; // lanes of a couple when the configuration says
+        std::vector<std::pair<int, int32_t>> packed;   // (lanes, pair)
+        for (int32_t p : S.stream_pairs) {
+            const int lanes = tm > 0 ? (fixed ? fixed : (pairs[p].m + tm - 1) / tm) : 0;
+            if (tm > 0 && pairs[p].m <= lanes * tm && lanes <= 32 && pairs[p].m + pairs[p].n <= PACKED16_MAX_IDS)
+                packed.push_back({lanes, p}), in_couple[size_t(p)] = 1;
+            else
+                single_pairs.push_back(p);
+        }
+        P->npacked = int32_t(packed.size());
+        // Pairs of as many lanes and about as many columns go together.
+        std::sort(packed.begin(), packed.end(), [&](const std::pair<int, int32_t> &x, const std::pair<int, int32_t> &y) {
+            if (x.first != y.first) return x.first > y.first;
+            if (pairs[x.second].n != pairs[y.second].n) return pairs[x.second].n > pairs[y.second].n;
+            return x.second < y.second;
+        });
+        for (size_t i = 0; i < packed.size(); ++i) {
+            CoupleDev k{};
+            std::memcpy(&k.a, &pairs[packed[i].second], sizeof(k.a));
+            k.rows = tm * packed[i].first;
+            k.nb = (k.a.n + 3) / 4; // the longer of the two
+            if (i + 1 < packed.size() && packed[i + 1].first == packed[i].first)
+                std::memcpy(&k.b, &pairs[packed[++i].second], sizeof(k.b));
+            couples.push_back(k);
+        }
+        // The staged ones first: those that do not fit, and those so long for
+        // their lanes that bundles of them would leave lanes idle (2,000
+        // pairs of 300 x 3000: 262 us staged, 440 with a couple to a bundle).
+        const auto mid = std::stable_partition(couples.begin(), couples.end(), [&](const CoupleDev &k) {
+            return k.nb > BUNDLE_BLOCKS || int64_t(k.nb) * 24 > int64_t(BUNDLE_BLOCKS) * (k.rows / tm);
+        });
+        P->nstaged = int32_t(mid - couples.begin());
+        P->ncouples = int32_t(couples.size());
+        for (int32_t i = 0; i < P->nstaged; ++i) {
+            CoupleDev &k = couples[size_t(i)];
+            k.off = int32_t(stage_elems);
+            stage_elems += int64_t(k.rows) / 2 + 2 * int64_t(k.nb);
+        }
+        make_bundles(couples, 0, size_t(P->nstaged), tm, INT32_MAX, bundle_lanes);
+        P->nstaged_bundles = int32_t(bundle_lanes.size() / 32);
+        make_bundles(couples, size_t(P->nstaged), couples.size(), tm, BUNDLE_BLOCKS, bundle_lanes);
+        deal_bundles(bundle_lanes, P->nstaged_bundles, 4 * (sm_count() - P->relay_sms), list_off);
+        P->nlists = int32_t(list_off.size()) - 1;
+    }
+    // Stream classes, warps and pair lists of the other pairs.  A pair costs
+    // its column blocks plus a switch; each class gets warps in proportion to
+    // its cost per warp (a warp runs 32/seg segments side by side), and within
+    // a class the pairs go longest first to the least loaded segment.  The grid
+    // is the persistent one (or blocks_per_sm per SM), fewer for small batches.
+    std::vector<int32_t> seg_off, seg_list, pool_list;
+    if (!single_pairs.empty()) {
         const int occ_blocks = std::max(1, full_grid / std::max(1, sm_count()));
         int grid = sm_count() * (P->blocks_per_sm > 0 ? std::min(P->blocks_per_sm, occ_blocks) : occ_blocks);
         const int nclass = int(P->classes.size());
-        // Items of a class: single pairs, or couples (pair A, pair B) for a
-        // packed class -- its pairs sorted by length and taken two by two.
-        std::vector<std::vector<int32_t>> cls_pairs(nclass);
-        for (int32_t p : S.stream_pairs) { // largest first
+        std::vector<std::vector<int32_t>> items(nclass);
+        for (int32_t p : single_pairs) {
             int c = 0;
-            for (; c < nclass; ++c) {
-                const StreamClass &k = P->classes[c];
-                if (pairs[p].m <= k.tm * k.seg && (!k.packed || int64_t(pairs[p].m) + pairs[p].n <= PACKED16_MAX_IDS))
-                    break;
-            }
-            if (c == nclass) { // cannot happen: the tallest class is a 32-bit one
+            while (c < nclass && pairs[p].m > P->classes[c].tm * P->classes[c].seg) ++c;
+            if (c == nclass) { // cannot happen: stream_rows is the tallest class
                 delete P;
                 return fail(SLCS_ERR_INVALID, "internal: no stream class for a pair");
             }
-            cls_pairs[c].push_back(p);
+            items[c].push_back(p);
         }
-        std::vector<std::vector<std::pair<int32_t, int32_t>>> items(nclass);
-        for (int c = 0; c < nclass; ++c) {
-            auto &cp = cls_pairs[c];
-            if (P->classes[c].packed) {
-                std::stable_sort(cp.begin(), cp.end(), [&](int32_t x, int32_t y) { return pairs[x].n > pairs[y].n; });
-                for (size_t i = 0; i < cp.size(); i += 2)
-                    items[c].push_back({cp[i], i + 1 < cp.size() ? cp[i + 1] : -1});
-            } else {
-                for (int32_t p : cp) items[c].push_back({p, -1});
-            }
-        }
-        // Cost of an item: its column blocks plus a pair switch, in steps.
-        auto cost = [&](int c, const std::pair<int32_t, int32_t> &it) {
-            const int cols = P->classes[c].packed ? 4 : P->tns;
-            const int32_t n = std::max(pairs[it.first].n, it.second >= 0 ? pairs[it.second].n : 0);
-            return int64_t((n + cols - 1) / cols) + 2;
-        };
-        // Per class: its steps in total, its longest item, and how many units
-        // can have work at all.  A unit is a warp of a fixed class (32 / seg
-        // segments) or one segment of the variable class (its lane count).
+        // Cost of a pair: its column blocks plus a pair switch, in steps.
+        auto cost = [&](int32_t p) { return int64_t((pairs[p].n + P->tns - 1) / P->tns) + 2; };
+        // Per class: its steps in total, its longest pair, and how many warps
+        // (of 32 / seg segments) can have work at all.
         std::vector<double> csteps(nclass, 0.0), clong(nclass, 0.0);
         std::vector<long> umax(nclass, 0);
-        auto unit_lanes = [&](int c) { return P->classes[c].var ? P->classes[c].seg : 32; };
-        auto unit_segs = [&](int c) { return P->classes[c].var ? 1 : 32 / P->classes[c].seg; };
+        auto unit_segs = [&](int c) { return 32 / P->classes[c].seg; };
+        long want = 0;
         for (int c = 0; c < nclass; ++c) {
-            int64_t w = 0, longest = 0;
-            for (const auto &it : items[c]) {
-                w += cost(c, it);
-                longest = std::max(longest, cost(c, it));
+            for (int32_t p : items[c]) {
+                csteps[c] += double(cost(p));
+                clong[c] = std::max(clong[c], double(cost(p)));
             }
-            csteps[c] = double(w);
-            clong[c] = double(longest);
             umax[c] = (long(items[c].size()) + unit_segs(c) - 1) / unit_segs(c);
+            want += umax[c];
         }
-        const long want_wf = (long(P->ntasks) + BATCH_WARPS - 1) / BATCH_WARPS;
-        long want = std::max<long>(1, want_wf);
-        long lanes_max = 0;
-        for (int c = 0; c < nclass; ++c) lanes_max += umax[c] * unit_lanes(c);
-        want = std::max(want, (lanes_max / 32 + 1 + BATCH_WARPS - 1) / BATCH_WARPS);
-        grid = int(std::max<long>(1, std::min<long>(grid, want)));
-        // One warp per wavefront task gets no stream list: those warps take
-        // the tasks from the start, so the stripe chains of the tall pairs
-        // run under the stream work instead of after it (a 3-stripe chain of
-        // 800 columns alone on a drained GPU took ~50 us, about an eighth of
-        // the 20,000-read launch).
-        const long reserve = std::min<long>(P->ntasks, long(grid) * BATCH_WARPS / 8);
-        const long warps_total = long(grid) * BATCH_WARPS - reserve;
-        // Units per class so that the classes end together.  A class of u
-        // units ends about when each of its segments has combed its share of
-        // the class's steps and the last one its longest item, half of which
+        grid = int(std::max<long>(1, std::min<long>(grid, (want + BATCH_WARPS - 1) / BATCH_WARPS)));
+        const long warps_total = long(grid) * BATCH_WARPS;
+        // Warps per class so that the classes end together.  A class of u
+        // warps ends about when each of its segments has combed its share of
+        // the class's steps and the last one its longest pair, half of which
         // is still to go on average: end(u) = t * (S / (u * segments per
-        // unit) + L / 2), t the class's time per step.  Each unit goes to the
-        // class that would end last, while the lanes last.  (Shares in
-        // proportion to S * t alone gave the 385-512-row class of the 20,000
-        // reads 30 warps for 64 items of ~150 steps: it ended ~40 us after
-        // every other class.)
+        // warp) + L / 2), t the class's time per step.  Each warp goes to the
+        // class that would end last, while the warps last.
         std::vector<long> uc(nclass, 0);
         auto class_end = [&](int c, long u) {
             return class_step_time(P->classes[c], P->tns) * (csteps[c] / double(u * unit_segs(c)) + clong[c] / 2.0);
         };
-        // Warps the variable class's segments need, packed first fit
-        // (largest first); layout[w] lists (class, lanes) of warp w.
-        std::vector<std::vector<std::pair<int, int>>> layout;
-        auto pack_var = [&]() {
-            std::vector<std::pair<int, int>> segs; // (lanes, class)
-            for (int c = 0; c < nclass; ++c)
-                if (P->classes[c].var)
-                    for (long u = 0; u < uc[c]; ++u) segs.push_back({P->classes[c].seg, c});
-            std::stable_sort(segs.begin(), segs.end(), [](const std::pair<int, int> &x, const std::pair<int, int> &y) {
-                return x.first > y.first;
-            });
-            layout.clear();
-            std::vector<int> room;
-            for (const auto &sg : segs) {
-                size_t w = 0;
-                while (w < room.size() && room[w] < sg.first) ++w;
-                if (w == room.size()) {
-                    room.push_back(32);
-                    layout.emplace_back();
-                }
-                room[w] -= sg.first;
-                layout[w].push_back({sg.second, sg.first});
-            }
-            return long(layout.size());
-        };
-        auto warps_needed = [&]() {
-            long w = pack_var();
-            for (int c = 0; c < nclass; ++c)
-                if (!P->classes[c].var) w += uc[c];
-            return w;
-        };
-        long lanes_used = 0;
-        for (int c = 0; c < nclass; ++c) {
-            if (items[c].empty()) continue;
-            uc[c] = 1;
-            lanes_used += unit_lanes(c);
-        }
-        for (;;) {
+        long used = 0;
+        for (int c = 0; c < nclass; ++c)
+            if (!items[c].empty()) ++used, uc[c] = 1;
+        while (used < warps_total) {
             int worst = -1;
             double worst_end = -1.0;
             for (int c = 0; c < nclass; ++c) {
-                if (uc[c] == 0 || uc[c] >= umax[c] || lanes_used + unit_lanes(c) > warps_total * 32) continue;
+                if (uc[c] == 0 || uc[c] >= umax[c]) continue;
                 const double e = class_end(c, uc[c]);
                 if (e > worst_end) {
                     worst_end = e;
                     worst = c;
                 }
             }
-            if (worst < 0) break; // out of lanes, or every class has a unit per item
+            if (worst < 0) break; // every class has a warp per 32 / seg pairs
             ++uc[worst];
-            lanes_used += unit_lanes(worst);
-        }
-        // Packing loses a few lanes: take units back from the classes that
-        // end first until the warps fit.
-        for (long need = warps_needed(); need > warps_total; need = warps_needed()) {
-            int best = -1;
-            double best_end = 0.0;
-            for (int c = 0; c < nclass; ++c) {
-                if (uc[c] <= 1) continue;
-                const double e = class_end(c, uc[c] - 1);
-                if (best < 0 || e < best_end) {
-                    best_end = e;
-                    best = c;
-                }
-            }
-            if (best < 0) break;
-            --uc[best];
-        }
-        const long var_warps = pack_var();
-        long used = var_warps;
-        int nfixed = 0;
-        for (int c = 0; c < nclass; ++c)
-            if (!P->classes[c].var && uc[c] > 0) {
-                used += uc[c];
-                ++nfixed;
-            }
-        int npools = 0;
-        for (int c = 0; c < nclass; ++c) npools += uc[c] > 0;
-        if (nfixed + (var_warps > 0) > MAX_CLASSES || npools > MAX_POOLS) {
-            delete P;
-            return fail(SLCS_ERR_UNSUPPORTED, "too many stream classes in use");
+            ++used;
         }
         P->grid = int(std::max<long>(grid, (used + BATCH_WARPS - 1) / BATCH_WARPS));
-        P->nclass = 0;
-        std::vector<std::vector<std::pair<int32_t, int32_t>>> slot_lists(size_t(std::max(used, 1L)) * SEG_SLOTS);
-        std::vector<std::pair<int32_t, int32_t>> pool_items;
-        // Segments of every class, as global slot ids (SEG_SLOTS * warp + slot).
-        std::vector<std::vector<long>> class_slots(nclass);
-        std::vector<int> class_pool_of(nclass, -1);
-        if (var_warps > 0) {
-            P->lane_map.assign(size_t(var_warps) * 32, -1);
-            int next_pool = 0;
-            for (int c = 0; c < nclass; ++c)
-                if (P->classes[c].var && uc[c] > 0) class_pool_of[c] = next_pool++;
-            for (long w = 0; w < var_warps; ++w) {
-                int lane0 = 0;
-                for (size_t j = 0; j < layout[w].size(); ++j) {
-                    const int c = layout[w][j].first, nl = layout[w][j].second;
-                    class_slots[c].push_back(long(w) * SEG_SLOTS + long(j));
-                    for (int l = 0; l < nl; ++l)
-                        P->lane_map[size_t(w) * 32 + size_t(lane0 + l)] =
-                            (class_pool_of[c] << 24) | (int(j) << 16) | (l << 8) | nl;
-                    lane0 += nl;
-                }
-            }
-            P->class_warp_end[P->nclass] = int32_t(var_warps);
-            P->class_code[P->nclass] = PACKED16_VAR_CODE + VAR_TM * 100;
-            P->class_pool[P->nclass] = -1;
-            ++P->nclass;
-        }
-        {
-            int next_pool = 0;
-            for (int c = 0; c < nclass; ++c)
-                if (class_pool_of[c] >= 0) next_pool = std::max(next_pool, class_pool_of[c] + 1);
-            long wbase = var_warps;
-            for (int c = 0; c < nclass; ++c) {
-                if (P->classes[c].var || uc[c] == 0) continue;
-                const int spw = 32 / P->classes[c].seg;
-                for (long u = 0; u < uc[c]; ++u)
-                    for (int j = 0; j < spw; ++j) class_slots[c].push_back((wbase + u) * SEG_SLOTS + j);
-                wbase += uc[c];
-                class_pool_of[c] = next_pool++;
-                P->class_warp_end[P->nclass] = int32_t(wbase);
-                P->class_code[P->nclass] = P->classes[c].tm * 100 + P->classes[c].seg +
-                                           (P->classes[c].packed ? PACKED16_CODE : 0);
-                P->class_pool[P->nclass] = class_pool_of[c];
-                ++P->nclass;
-            }
-        }
-        // Lists and pools, pool by pool.
-        std::vector<int> by_pool(npools, -1);
-        for (int c = 0; c < nclass; ++c)
-            if (class_pool_of[c] >= 0) by_pool[class_pool_of[c]] = c;
-        for (int pi = 0; pi < npools; ++pi) {
-            const int c = by_pool[pi];
-            const auto &slots = class_slots[c];
-            const long nseg = long(slots.size());
+        std::vector<std::vector<int32_t>> slot_lists(size_t(used) * SEG_SLOTS);
+        long wbase = 0;
+        for (int c = 0; c < nclass; ++c) {
+            if (uc[c] == 0) continue;
+            const int spw = unit_segs(c), k = P->nclass++;
+            const long nseg = uc[c] * spw;
             using Load = std::pair<int64_t, int64_t>;
             std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
             for (long sgi = 0; sgi < nseg; ++sgi) heap.push({0, sgi});
             std::stable_sort(items[c].begin(), items[c].end(),
-                             [&](const std::pair<int32_t, int32_t> &x, const std::pair<int32_t, int32_t> &y) {
-                                 return cost(c, x) > cost(c, y);
-                             });
+                             [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
             // Longest first to the least loaded segment until every segment
             // holds (100 - pool_pct) % of the class's average load; the rest,
-            // the shortest items, form the class's pool, which segments claim
-            // one item at a time when their lists run out, so that the class
+            // the shortest pairs, form the class's pool, which segments claim
+            // one pair at a time when their lists run out, so that the class
             // ends evenly whatever the real speed of its segments.
-            int64_t class_cost = 0;
-            for (const auto &it : items[c]) class_cost += cost(c, it);
-            const double cap = (100 - P->pool_pct) / 100.0 * double(class_cost) / double(nseg);
-            P->pool_off[pi] = int32_t(pool_items.size());
-            for (const auto &it : items[c]) {
+            const double cap = (100 - P->pool_pct) / 100.0 * csteps[c] / double(nseg);
+            P->pool_off[k] = int32_t(pool_list.size());
+            for (int32_t p : items[c]) {
                 Load top = heap.top();
                 if (P->pool_pct > 0 && double(top.first) >= cap) {
-                    pool_items.push_back(it);
+                    pool_list.push_back(p);
                     continue;
                 }
                 heap.pop();
-                slot_lists[size_t(slots[size_t(top.second)])].push_back(it);
-                top.first += cost(c, it);
+                slot_lists[size_t((wbase + top.second / spw) * SEG_SLOTS + top.second % spw)].push_back(p);
+                top.first += cost(p);
                 heap.push(top);
             }
-            P->pool_off[pi + 1] = int32_t(pool_items.size());
-            if (P->classes[c].packed) P->npacked += int32_t(cls_pairs[c].size());
+            wbase += uc[c];
+            P->class_warp_end[k] = int32_t(wbase);
+            P->class_code[k] = P->classes[c].tm * 100 + P->classes[c].seg;
         }
+        for (int k = P->nclass; k <= MAX_CLASSES; ++k) P->pool_off[k] = int32_t(pool_list.size());
         P->nwarps = int32_t(used);
-        for (int pi = npools + 1; pi <= MAX_POOLS; ++pi) P->pool_off[pi] = P->pool_off[npools];
-        for (const auto &it : pool_items) {
-            pool_list.push_back(it.first);
-            pool_list2.push_back(it.second);
-        }
-        if (P->nwarps > 0) {
-            seg_off.reserve(size_t(P->nwarps) * SEG_SLOTS + 1);
-            seg_off.push_back(0);
-            for (long sl = 0; sl < long(P->nwarps) * SEG_SLOTS; ++sl) {
-                for (const auto &it : slot_lists[size_t(sl)]) {
-                    seg_list.push_back(it.first);
-                    seg_list2.push_back(it.second);
-                }
-                seg_off.push_back(int32_t(seg_list.size()));
-            }
+        seg_off.push_back(0);
+        for (const auto &l : slot_lists) {
+            seg_list.insert(seg_list.end(), l.begin(), l.end());
+            seg_off.push_back(int32_t(seg_list.size()));
         }
     }
-    // Relay items: the groups of every pair, largest pair first.
+    // Relay items: the groups of every pair that does not stream (all pairs
+    // when the relay kernel takes the whole plan), largest pair first.
     std::vector<int2> relay_items;
     std::vector<int64_t> row_off;
-    if (P->relay.tm > 0) {
+    // Without a configuration the relay kernel takes a whole batch where it is
+    // predicted to end first: few pairs, or tall or wide ones, leave a warp of
+    // couples a chain of its own.  Of couples, a step of a chain takes about 0.22
+    // us and a step in all 0.22 us of a sub-partition; of streamed 32-bit pairs,
+    // about three times that.  (20,000 reads: 115 us in couples, 361 by relay;
+    // 4,000: 54 and 81; 1,000: 51 and 43; 64: 47 and 25; 64 pairs of 400 x 5000:
+    // 390 in staged couples, 76 by relay.)
+    if (P->stm > 0) {
+        double chain = 0, steps = 0;
+        for (size_t i = 0; i < bundle_lanes.size(); i += 32) {
+            const bool staged = i / 32 < size_t(P->nstaged_bundles);
+            chain = std::max(chain, (staged ? 0.3 : 0.22) * bundle_lanes[i].steps);
+            steps += 0.22 * (bundle_lanes[i].steps + 12.0);
+        }
+        for (int32_t p : single_pairs) {
+            chain = std::max(chain, 0.66 * (pairs[p].n / double(P->tns) + 32.0));
+            steps += 0.33 * (pairs[p].n / double(P->tns) + 2.0);
+        }
+        double us = P->nstream > 0 ? (P->nstaged > 0 ? 25.0 : 10.0) + std::max(chain, steps / (4.0 * sms)) : 0.0;
+        us = P->relay_sms > 0 ? std::max(us, tall_us) : us + tall_us;
+        // (A chunk of a host run shares the GPU with the others: couples take less
+        // of it.)
+        const bool plain = chunk ? false : !cfg || (cfg->algo == SLCS_ALGO_AUTO && cfg->tile_m == 0 && cfg->tile_n == 0 &&
+                                    cfg->warps == 0 && cfg->seg == 0 && cfg->blocks_per_sm == 0 &&
+                                    cfg->strand_bits == 0 && cfg->pool_pct == 0);
+        RelayShape all{};
+        if (P->nstream == 0 || (plain && batch_relay_us(pairs, npairs, sms, [](int32_t) { return true; }, &all) < us)) {
+            P->relay_all = P->nstream + P->ntasks > 0;
+            if (P->nstream > 0) P->relay = all;
+        }
+    }
+    if (P->relay_all || (P->stm > 0 && P->ntasks > 0)) {
         const slcs_status rs = launch_relay(RelayLaunch{}, P->relay, sm_count(), PREPARE_ONLY);
         if (rs != SLCS_OK) {
             delete P;
@@ -1318,7 +1376,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         int64_t row_elems = 0;
         row_off.assign(npairs, 0);
         for (int32_t p : S.order) {
-            if (pairs[p].m == 0 || pairs[p].n == 0) continue;
+            if (pairs[p].m == 0 || pairs[p].n == 0 || (!P->relay_all && pairs[p].m <= stream_rows)) continue;
             const int32_t groups = relay_groups(pairs[p].m, P->relay);
             for (int32_t g = 0; g < groups; ++g) relay_items.push_back(make_int2(p, g));
             row_off[p] = row_elems;
@@ -1327,49 +1385,80 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         P->nrelay = int32_t(relay_items.size());
         P->relay_ws_bytes = 16 + sizeof(int2) * size_t(row_elems);
     }
-    P->work_bytes = align_up(sizeof(int32_t) * (WORK_HEAD + S.tasks.size()), 256);
-    cudaError_t e = cudaSuccess;
-    auto alloc = [&](void **ptr, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(ptr, bytes < 16 ? 16 : bytes);
+    P->work_bytes = align_up(sizeof(int32_t) * (WORK_HEAD + (P->stm > 0 ? 0 : S.tasks.size())), 256);
+    // One device block for the plan: what is uploaded first, then the work
+    // areas (an allocation and a copy for each array took a third of the time
+    // to make a plan).
+    std::vector<char> up;
+    size_t bytes = 0;
+    auto place = [&](auto **ptr, size_t count) {
+        const size_t at = align_up(bytes, 256);
+        bytes = at + sizeof(**ptr) * count;
+        *ptr = reinterpret_cast<std::remove_pointer_t<decltype(ptr)>>(at); // an offset until the block exists
+        return at;
     };
-    alloc(reinterpret_cast<void **>(&P->d_pairs), sizeof(PairDev) * size_t(npairs));
-    alloc(reinterpret_cast<void **>(&P->d_seg_off), sizeof(int32_t) * seg_off.size());
-    alloc(reinterpret_cast<void **>(&P->d_seg_list), sizeof(int32_t) * seg_list.size());
-    alloc(reinterpret_cast<void **>(&P->d_seg_list2), sizeof(int32_t) * seg_list2.size());
-    alloc(reinterpret_cast<void **>(&P->d_pool_list), sizeof(int32_t) * pool_list.size());
-    alloc(reinterpret_cast<void **>(&P->d_pool_list2), sizeof(int32_t) * pool_list2.size());
-    alloc(reinterpret_cast<void **>(&P->d_lane_map), sizeof(int32_t) * P->lane_map.size());
-    if (e == cudaSuccess && !P->lane_map.empty())
-        e = cudaMemcpy(P->d_lane_map, P->lane_map.data(), sizeof(int32_t) * P->lane_map.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !pool_list.empty())
-        e = cudaMemcpy(P->d_pool_list, pool_list.data(), sizeof(int32_t) * pool_list.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !pool_list2.empty())
-        e = cudaMemcpy(P->d_pool_list2, pool_list2.data(), sizeof(int32_t) * pool_list2.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !seg_list2.empty())
-        e = cudaMemcpy(P->d_seg_list2, seg_list2.data(), sizeof(int32_t) * seg_list2.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !seg_off.empty())
-        e = cudaMemcpy(P->d_seg_off, seg_off.data(), sizeof(int32_t) * seg_off.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !seg_list.empty())
-        e = cudaMemcpy(P->d_seg_list, seg_list.data(), sizeof(int32_t) * seg_list.size(), cudaMemcpyHostToDevice);
-    alloc(reinterpret_cast<void **>(&P->d_tasks), sizeof(int2) * S.tasks.size());
-    alloc(reinterpret_cast<void **>(&P->d_scr_off), sizeof(int64_t) * size_t(npairs));
-    alloc(reinterpret_cast<void **>(&P->d_scratch), sizeof(int32_t) * size_t(S.scratch_elems) + 16);
-    alloc(reinterpret_cast<void **>(&P->d_work), P->work_bytes);
-    if (P->nrelay > 0) {
-        alloc(reinterpret_cast<void **>(&P->d_relay), sizeof(int2) * relay_items.size());
-        alloc(reinterpret_cast<void **>(&P->d_row_off), sizeof(int64_t) * row_off.size());
-        alloc(reinterpret_cast<void **>(&P->d_relay_ws), P->relay_ws_bytes);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(P->d_relay, relay_items.data(), sizeof(int2) * relay_items.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(P->d_row_off, row_off.data(), sizeof(int64_t) * row_off.size(), cudaMemcpyHostToDevice);
+    auto upload = [&](auto **ptr, const void *src, size_t count) {
+        const size_t at = place(ptr, count);
+        up.resize(bytes);
+        if (count) std::memcpy(up.data() + at, src, sizeof(**ptr) * count);
+    };
+    static const uint32_t masked_block[4 * COUPLE_HEAD] = {0x01000100u, 0x01000100u, 0x01000100u, 0x01000100u,
+                                                           0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu};
+    const bool stream = !P->relay_all && P->stm > 0;
+    if (P->relay_all) P->nstaged = P->ncouples = P->nstaged_bundles = P->nlists = P->nwarps = 0;
+    upload(&P->d_pairs, pairs, size_t(npairs));
+    upload(&P->d_relay, relay_items.data(), relay_items.size());
+    upload(&P->d_row_off, row_off.data(), row_off.size());
+    upload(&P->d_seg_off, seg_off.data(), stream ? seg_off.size() : 0);
+    upload(&P->d_seg_list, seg_list.data(), stream ? seg_list.size() : 0);
+    upload(&P->d_pool_list, pool_list.data(), stream ? pool_list.size() : 0);
+    std::vector<int32_t> others;
+    if (P->ncouples > 0)
+        for (int32_t p = 0; p < npairs; ++p)
+            if (!in_couple[size_t(p)]) others.push_back(p);
+    P->nothers = int32_t(others.size());
+    upload(&P->d_others, others.data(), others.size());
+    upload(&P->d_couples, couples.data(), size_t(P->ncouples));
+    upload(&P->d_bundles, bundle_lanes.data(), P->ncouples > 0 ? bundle_lanes.size() : 0);
+    upload(&P->d_list_off, list_off.data(), P->nlists > 0 ? list_off.size() : 0);
+    upload(&P->d_tasks, S.tasks.data(), P->stm > 0 ? 0 : S.tasks.size());
+    upload(&P->d_scr_off, S.scratch_off.data(), P->stm > 0 ? 0 : S.scratch_off.size());
+    upload(&P->d_couple_stage, masked_block, P->nstaged > 0 ? COUPLE_HEAD : 0);
+    if (P->nstaged > 0) bytes += sizeof(uint4) * size_t(stage_elems - COUPLE_HEAD); // the couples, after the block
+    place(&P->d_scratch, P->stm > 0 ? 0 : size_t(S.scratch_elems));
+    place(&P->d_work, P->work_bytes / sizeof(int32_t));
+    place(&P->d_relay_ws, P->relay_ws_bytes);
+    // From the memory pool that the workspaces of other calls come from (a
+    // cudaMalloc beyond a megabyte maps memory, about 300 us a plan); the copy
+    // below orders it before any stream's work.
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&P->d_block), std::max<size_t>(bytes, 256), nullptr);
+    auto rebase = [&](auto *&ptr) {
+        ptr = e == cudaSuccess ? reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(
+                                     P->d_block + reinterpret_cast<uintptr_t>(ptr))
+                               : nullptr;
+    };
+    rebase(P->d_pairs);
+    rebase(P->d_relay);
+    rebase(P->d_row_off);
+    rebase(P->d_seg_off);
+    rebase(P->d_seg_list);
+    rebase(P->d_pool_list);
+    rebase(P->d_others);
+    rebase(P->d_couples);
+    rebase(P->d_bundles);
+    rebase(P->d_list_off);
+    rebase(P->d_tasks);
+    rebase(P->d_scr_off);
+    rebase(P->d_couple_stage);
+    rebase(P->d_scratch);
+    rebase(P->d_work);
+    rebase(P->d_relay_ws);
+    if (e == cudaSuccess && !up.empty()) e = cudaMemcpy(P->d_block, up.data(), up.size(), cudaMemcpyHostToDevice);
+    if (P->nrelay > 0 && !P->relay_all && P->relay_sms > 0 && P->nstream > 0) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->join, cudaEventDisableTiming);
     }
-    if (e == cudaSuccess && npairs)
-        e = cudaMemcpy(P->d_pairs, pairs, sizeof(PairDev) * size_t(npairs), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !S.tasks.empty())
-        e = cudaMemcpy(P->d_tasks, S.tasks.data(), sizeof(int2) * S.tasks.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && npairs)
-        e = cudaMemcpy(P->d_scr_off, S.scratch_off.data(), sizeof(int64_t) * size_t(npairs), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         slcs_batch_plan_destroy(P);
         return cuda_fail(e, "batch plan upload");
@@ -1434,7 +1523,7 @@ slcs_status slcs_batch_plan_info(const slcs_batch_plan *P, slcs_plan_info *info)
     std::memset(info, 0, sizeof(*info));
     info->stream_tile_m = P->stm;
     info->seg = P->stm > 0 ? P->seg : 0;
-    info->stream_classes = P->nclass;
+    info->stream_classes = P->nclass + (P->npacked > 0 ? 1 : 0);
     info->tile_n = P->stm > 0 ? P->tns : 4;
     info->grid = P->grid;
     info->wavefront_tile_m = P->tm;
@@ -1442,13 +1531,18 @@ slcs_status slcs_batch_plan_info(const slcs_batch_plan *P, slcs_plan_info *info)
     info->stream_pairs = P->nstream;
     info->wavefront_tasks = P->ntasks;
     info->packed_pairs = P->npacked;
+    info->relay_groups = P->nrelay;
+    info->relay_all = P->relay_all;
     return SLCS_OK;
 }
 
 int32_t slcs_batch_plan_launches(const slcs_batch_plan *P)
 {
     if (!P) return 0;
-    return ((P->ntasks > 0 || P->nstream > 0) ? 1 : 0) + int32_t(P->empty_pairs.size());
+    const bool rest = !P->relay_all && (P->stm > 0 ? P->nstream > 0 : P->ntasks > 0);
+    const int32_t stream = P->stm > 0 ? (P->nwarps > 0 ? 1 : 0) + (P->nstaged > 0 ? 3 : 0) + (P->nlists > 0 ? 1 : 0) : 1;
+    return (rest ? stream : 0) + (P->nrelay > 0 ? 1 : 0) +
+           int32_t(P->empty_pairs.size());
 }
 
 slcs_status slcs_batch_plan_run(slcs_batch_plan *P, const uint8_t *a, const uint8_t *b, int32_t *out, void *stream)
@@ -1457,7 +1551,7 @@ slcs_status slcs_batch_plan_run(slcs_batch_plan *P, const uint8_t *a, const uint
     if (P->npairs > 0 && (!out || (P->ntasks > 0 && (!a || !b))))
         return fail(SLCS_ERR_INVALID, "null blob or output pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!P->use_graph) return P->enqueue(a, b, out, st);
+    if (!P->use_graph) return P->enqueue(a, b, out, nullptr, st);
     if (!P->gexec || P->g_a != a || P->g_b != b || P->g_out != out) {
         if (P->gexec) {
             cudaGraphExecDestroy(P->gexec);
@@ -1465,7 +1559,7 @@ slcs_status slcs_batch_plan_run(slcs_batch_plan *P, const uint8_t *a, const uint
         }
         if (!P->cap_stream) SLCS_CUDA(cudaStreamCreateWithFlags(&P->cap_stream, cudaStreamNonBlocking));
         SLCS_CUDA(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal));
-        slcs_status s = P->enqueue(a, b, out, P->cap_stream);
+        slcs_status s = P->enqueue(a, b, out, nullptr, P->cap_stream);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(P->cap_stream, &g);
         if (s != SLCS_OK) {
@@ -1556,6 +1650,30 @@ static slcs_status narrow16(const int32_t *in, int16_t *out, int64_t lo, int64_t
     return SLCS_OK;
 }
 
+// The same for the strands of the listed pairs, one block each.
+__global__ void narrow16_pairs_kernel(const PairDev *pairs, const int32_t *list, const int32_t *__restrict__ in,
+                                      int16_t *__restrict__ out)
+{
+    const PairDev P = pairs[list[blockIdx.x]];
+    for (int32_t i = threadIdx.x; i < P.m + P.n; i += blockDim.x) out[P.out_off + i] = int16_t(in[P.out_off + i]);
+}
+
+// A run of the plan whose strands end up as int16 in out16 (entries lo to hi):
+// the couples write them so, the other pairs' are narrowed from out.
+static slcs_status run16(slcs_batch_plan *P, const uint8_t *a, const uint8_t *b, int32_t *out, int16_t *out16,
+                         int64_t lo, int64_t hi, cudaStream_t st)
+{
+    if (P->ncouples == 0) {
+        const slcs_status s = slcs_batch_plan_run(P, a, b, out, st);
+        return s == SLCS_OK ? narrow16(out, out16, lo, hi, st) : s;
+    }
+    const slcs_status s = P->enqueue(a, b, out, out16, st);
+    if (s != SLCS_OK || P->nothers == 0) return s;
+    narrow16_pairs_kernel<<<P->nothers, 256, 0, st>>>(P->d_pairs, P->d_others, out, out16);
+    SLCS_CUDA(cudaGetLastError());
+    return SLCS_OK;
+}
+
 slcs_status slcs_batch_plan_run_host16(slcs_batch_plan *P, const uint8_t *a, int64_t a_len, const uint8_t *b,
                                        int64_t b_len, int16_t *out, int64_t out_len, void *stream)
 {
@@ -1591,8 +1709,7 @@ slcs_status slcs_batch_plan_run_host16(slcs_batch_plan *P, const uint8_t *a, int
     int16_t *d16 = P->d_out16;
     if (!P->chunks.empty()) {
         // As slcs_batch_plan_run_host, chunk by chunk on their own streams,
-        // with each chunk's strands narrowed on the device before they cross
-        // the bus (half the bytes of the copy back).
+        // with half the bytes to copy back.
         SLCS_CUDA(cudaEventRecord(P->chunk_start, st));
         for (auto &k : P->chunks) {
             SLCS_CUDA(cudaStreamWaitEvent(k.stream, P->chunk_start, 0));
@@ -1602,8 +1719,7 @@ slcs_status slcs_batch_plan_run_host16(slcs_batch_plan *P, const uint8_t *a, int
             if (k.b_hi > k.b_lo)
                 SLCS_CUDA(cudaMemcpyAsync(db + k.b_lo, b + k.b_lo, size_t(k.b_hi - k.b_lo), cudaMemcpyHostToDevice,
                                           k.stream));
-            slcs_status s = slcs_batch_plan_run(k.plan, da, db, dout, k.stream);
-            if (s == SLCS_OK) s = narrow16(dout, d16, k.o_lo, k.o_hi, k.stream);
+            const slcs_status s = run16(k.plan, da, db, dout, d16, k.o_lo, k.o_hi, k.stream);
             if (s != SLCS_OK) return s;
             if (k.o_hi > k.o_lo)
                 SLCS_CUDA(cudaMemcpyAsync(out + k.o_lo, d16 + k.o_lo, sizeof(int16_t) * size_t(k.o_hi - k.o_lo),
@@ -1616,8 +1732,7 @@ slcs_status slcs_batch_plan_run_host16(slcs_batch_plan *P, const uint8_t *a, int
     }
     if (P->need_a) SLCS_CUDA(cudaMemcpyAsync(da, a, size_t(P->need_a), cudaMemcpyHostToDevice, st));
     if (P->need_b) SLCS_CUDA(cudaMemcpyAsync(db, b, size_t(P->need_b), cudaMemcpyHostToDevice, st));
-    slcs_status s = slcs_batch_plan_run(P, da, db, dout, stream);
-    if (s == SLCS_OK) s = narrow16(dout, d16, 0, P->need_out, st);
+    const slcs_status s = run16(P, da, db, dout, d16, 0, P->need_out, st);
     if (s != SLCS_OK) return s;
     if (P->need_out)
         SLCS_CUDA(cudaMemcpyAsync(out, d16, sizeof(int16_t) * size_t(P->need_out), cudaMemcpyDeviceToHost, st));
@@ -1637,20 +1752,17 @@ slcs_status slcs_batch_plan_destroy(slcs_batch_plan *P)
     if (P->chunk_start) cudaEventDestroy(P->chunk_start);
     if (P->gexec) cudaGraphExecDestroy(P->gexec);
     if (P->cap_stream) cudaStreamDestroy(P->cap_stream);
-    cudaFree(P->d_pairs);
-    cudaFree(P->d_seg_off);
-    cudaFree(P->d_seg_list);
-    cudaFree(P->d_seg_list2);
-    cudaFree(P->d_pool_list);
-    cudaFree(P->d_pool_list2);
-    cudaFree(P->d_relay);
-    cudaFree(P->d_row_off);
-    cudaFree(P->d_relay_ws);
-    cudaFree(P->d_lane_map);
-    cudaFree(P->d_tasks);
-    cudaFree(P->d_scr_off);
-    cudaFree(P->d_scratch);
-    cudaFree(P->d_work);
+    if (P->side) cudaStreamDestroy(P->side);
+    if (P->fork) cudaEventDestroy(P->fork);
+    if (P->join) cudaEventDestroy(P->join);
+    if (P->d_block) {
+        int cur = 0;
+        cudaGetDevice(&cur);
+        if (cur != P->device) cudaSetDevice(P->device);
+        cudaDeviceSynchronize(); // as cudaFree waits: the plan may still be running
+        cudaFreeAsync(P->d_block, nullptr);
+        if (cur != P->device) cudaSetDevice(cur);
+    }
     cudaFree(P->h_stage);
     delete P;
     return SLCS_OK;

@@ -422,46 +422,39 @@ __device__ __forceinline__ void take_next(const CombLaunch &L, const NextPair<TM
     }
 }
 
-// The items of one segment, in order: its list from the plan, then items of
+// The pairs of one segment, in order: its list from the plan, then pairs of
 // its class's pool, claimed one at a time.  Only lane 0 of a segment picks;
-// lane l learns each item from lane l - 1, which switched to it one step
+// lane l learns each pair from lane l - 1, which switched to it one step
 // earlier (every lane of a segment sees the same column blocks, l steps
 // behind lane 0).  Lane 0 claims its pool tickets one pick ahead, so that the
 // atomic's round trip overlaps a whole pair instead of stalling the warp.
 struct ItemSource {
-    const int32_t *la, *lb; // the segment's list (lb: high-half pairs, packed classes only)
-    int count;              // items in the list
-    int q;                  // lane 0: position of the next item to pick
+    const int32_t *list; // the segment's list
+    int count;           // pairs in it
+    int q;               // lane 0: position of the next pair to pick
     int cls;
-    int ahead;              // lane 0: pool ticket claimed for the next pick (-1: none yet)
+    int ahead;           // lane 0: pool ticket claimed for the next pick (-1: none yet)
 
     __device__ __forceinline__ int claim(const BatchLaunch &B, int size) const
     {
         return size > 0 ? atomicAdd(B.pool_ticket + cls, 1) : 0;
     }
 
-    __device__ __forceinline__ void pick(const BatchLaunch &B, int &pa, int &pb)
+    __device__ __forceinline__ int pick(const BatchLaunch &B) // -1: no more
     {
-        if (cls < 0) { // an idle lane of a variable warp
-            pa = pb = -1;
-            return;
-        }
         const int off = B.pool_off[cls], size = B.pool_off[cls + 1] - off;
         if (q < count) {
-            pa = la[q];
-            pb = lb ? lb[q] : -1;
+            const int p = list[q];
             if (++q == count && ahead < 0) ahead = claim(B, size);
-            return;
+            return p;
         }
         const int k = ahead >= 0 ? ahead : claim(B, size);
-        if (k < size) {
-            ahead = claim(B, size);
-            pa = B.pool_list[off + k];
-            pb = lb ? B.pool_list2[off + k] : -1;
-        } else {
+        if (k >= size) {
             ahead = size;
-            pa = pb = -1;
+            return -1;
         }
+        ahead = claim(B, size);
+        return B.pool_list[off + k];
     }
 };
 
@@ -473,13 +466,13 @@ __device__ __forceinline__ void stream_segment(const BatchLaunch &B, int cls, in
     const int r0 = sl * TM;
     const int seg_lane0 = lane & ~(SEG - 1);
     const int beg = B.seg_off[seg_id];
-    ItemSource src{B.seg_list + beg, nullptr, B.seg_off[seg_id + 1] - beg, 0, cls, -1};
+    ItemSource src{B.seg_list + beg, B.seg_off[seg_id + 1] - beg, 0, cls, -1};
 
     // The first two items, picked by lane 0 and shared with the segment.
-    int p0 = -1, p1 = -1, unused = -1;
+    int p0 = -1, p1 = -1;
     if (sl == 0) {
-        src.pick(B, p0, unused);
-        if (p0 >= 0) src.pick(B, p1, unused);
+        p0 = src.pick(B);
+        if (p0 >= 0) p1 = src.pick(B);
     }
     p0 = __shfl_sync(FULL_MASK, p0, seg_lane0);
     p1 = __shfl_sync(FULL_MASK, p1, seg_lane0);
@@ -556,277 +549,10 @@ __device__ __forceinline__ void stream_segment(const BatchLaunch &B, int cls, in
                 if (r0 + k < T.m) T.h_out[T.m - 1 - r0 - k] = hv[k];
             take_next<TM>(L, N, r0, T, av, hv);
             T.nb = (T.n + TNS - 1) / TNS;
-            int p = -1, unused2 = -1;
-            if (T.pair >= 0) {
-                if (sl == 0) src.pick(B, p, unused2);
-                else p = up;
-            }
+            int p = -1;
+            if (T.pair >= 0) p = sl == 0 ? src.pick(B) : up;
             nxt = p;
             fetch_next<TM>(L, p, r0, N);
-            blk = 0;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Packed stream mode: two pairs per register.
-//
-// A couple of pairs (A, B) of one row class is combed together: every symbol,
-// h and v register holds pair A in its low 16 bits and pair B in its high 16
-// bits, so one instruction works on two cells.  Strand ids are stored plus
-// one (1..32767); a masked row holds h = 0 and symbol 0x1FF, a masked column
-// v = 0x7FFF and symbol 0x100, so neither ever swaps.  The cell rule per half:
-//   x = a ^ b                    0 on a match (both below 0x200)
-//   far = fma.relu(x, -inf, 0)   on two 16-bit floats: 0 * -inf is NaN, which
-//                                relu turns into 0x7FFF; a positive x gives
-//                                -inf, which relu turns into 0
-//   h' = min(h + far, v)         unsigned halves, one VIADDMNMX
-//   v' = h + v - h'              as one 32-bit sum: the carries between the
-//                                halves cancel
-// On a match h + far is at least any v, so h' = v.  Seven integer instructions
-// (a carry-safe difference, a byte permute expanding its sign to a mask, two
-// bitwise selects) measured 5.50 cycles per warp and cell, these four 2.39
-// (one sub-partition, 4 warps of 16 rows per lane).
-// Both pairs of a couple switch together after max(nb_A, nb_B) blocks; the
-// shorter pair's extra columns are masked.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void cell16(uint32_t a, uint32_t b, uint32_t &h, uint32_t &v)
-{
-    uint32_t far;
-    asm("{\n\t.reg .b32 ninf, zero;\n\tmov.b32 ninf, 0xFF80FF80;\n\tmov.b32 zero, 0;\n\t"
-        "fma.rn.relu.bf16x2 %0, %1, ninf, zero;\n\t}"
-        : "=r"(far)
-        : "r"(a ^ b));
-    const uint32_t nh = __viaddmin_u16x2(h, far, v);
-    v = h + v - nh;
-    h = nh;
-}
-
-template <int TM>
-struct CoupleTask {
-    int pa, pb;      // pair indices (-1: none)
-    int ma, na, mb, nb_cols, nb;
-    int full_blocks; // leading blocks where both pairs have 4 columns and b is word-aligned
-    uint32_t vbase;  // (ma + 1) | (mb + 1) << 16: packed start id of column 0
-    const uint8_t *ba, *bb;
-    int32_t *ha, *va, *hb, *vb;
-};
-
-template <int TM>
-struct NextCouple {
-    NextPair<TM> A, B;
-};
-
-// Make a fetched couple current: packed row symbols and start ids.  This runs
-// on one lane at a time (each lane switches one step after its left
-// neighbour), so it is written to be short: per row one byte permute picks
-// both pairs' symbols, and the masks and start ids follow from the rows left
-// in each pair, m - r (the id + 1 of row r's h strand while r < m).
-template <int TM>
-__device__ __forceinline__ void take_couple(const CombLaunch &L, const NextCouple<TM> &N, int r0, CoupleTask<TM> &T,
-                                            uint32_t (&ap)[TM], uint32_t (&hp)[TM])
-{
-    const bool va = N.A.pair >= 0, vb = N.B.pair >= 0;
-    T.pa = N.A.pair;
-    T.pb = N.B.pair;
-    T.ma = va ? N.A.d1.z : 0;
-    T.na = va ? N.A.d1.w : 0;
-    T.mb = vb ? N.B.d1.z : 0;
-    T.nb_cols = vb ? N.B.d1.w : 0;
-    const int64_t ba = va ? int64_t((uint64_t(uint32_t(N.A.d0.w)) << 32) | uint32_t(N.A.d0.z)) : 0;
-    const int64_t oa = va ? int64_t((uint64_t(uint32_t(N.A.d1.y)) << 32) | uint32_t(N.A.d1.x)) : 0;
-    const int64_t bb = vb ? int64_t((uint64_t(uint32_t(N.B.d0.w)) << 32) | uint32_t(N.B.d0.z)) : 0;
-    const int64_t ob = vb ? int64_t((uint64_t(uint32_t(N.B.d1.y)) << 32) | uint32_t(N.B.d1.x)) : 0;
-    T.ba = L.b_blob + ba;
-    T.bb = L.b_blob + bb;
-    T.ha = L.out + oa;
-    T.va = T.ha + T.ma;
-    T.hb = L.out + ob;
-    T.vb = T.hb + T.mb;
-    T.nb = (max(T.na, T.nb_cols) + 3) / 4;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(T.ba) | reinterpret_cast<uintptr_t>(T.bb)) & 3) == 0;
-    T.full_blocks = (vb && aligned) ? min(T.na, T.nb_cols) / 4 : 0;
-    T.vbase = uint32_t(T.ma + 1) | (uint32_t(T.mb + 1) << 16);
-    const int ra = T.ma - r0, rb = T.mb - r0;
-    if (ra >= TM && rb >= TM) {
-        // Every row of this lane lies inside both pairs: the ids of the h
-        // strands, m - r, count down by one per row in both halves at once.
-        const uint32_t hbase = uint32_t(ra) | (uint32_t(rb) << 16);
-#pragma unroll
-        for (int k = 0; k < TM; ++k) {
-            const uint32_t j = uint32_t(k % 4);
-            ap[k] = __byte_perm(N.A.sym[k / 4], N.B.sym[k / 4], j | (j << 4) | ((4 + j) << 8) | ((4 + j) << 12)) &
-                    0x00FF00FFu;
-            hp[k] = hbase - uint32_t(k) * 0x00010001u;
-        }
-        return;
-    }
-    if (ra <= 0 && rb <= 0) { // no row of this lane in either pair
-#pragma unroll
-        for (int k = 0; k < TM; ++k) {
-            ap[k] = 0x01FF01FFu;
-            hp[k] = 0u;
-        }
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < TM; ++k) {
-        const uint32_t j = uint32_t(k % 4);
-        // byte j of A's word to byte 0, byte j of B's word to byte 2
-        const uint32_t sym = __byte_perm(N.A.sym[k / 4], N.B.sym[k / 4], j | (j << 4) | ((4 + j) << 8) | ((4 + j) << 12)) &
-                             0x00FF00FFu;
-        const int hA = ra - k, hB = rb - k;
-        ap[k] = sym | (hA <= 0 ? 0x1FFu : 0u) | (hB <= 0 ? 0x1FF0000u : 0u);
-        hp[k] = uint32_t(max(hA, 0)) | (uint32_t(max(hB, 0)) << 16);
-    }
-}
-
-// Four symbols of one pair at columns c..c+3 as bytes (masked: 0x100 later).
-__device__ __forceinline__ uint32_t sym4(const uint8_t *b, int c, int n, bool &full)
-{
-    full = c + 4 <= n;
-    if (full && (reinterpret_cast<uintptr_t>(b + c) & 3) == 0) return __ldg(reinterpret_cast<const uint32_t *>(b + c));
-    uint32_t w = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (c + j < n) w |= uint32_t(__ldg(b + c + j)) << (8 * j);
-    full = false;
-    return w;
-}
-
-// A segment of SEG lanes (lanes seg_lane0 .. seg_lane0 + SEG - 1 of the
-// warp; this lane is lane sl of it) streaming the items of pool `cls` (-1:
-// an idle lane, which only takes part in the warp's shuffles).  Segments of
-// any size may share a warp: a lane takes its neighbour's strands through a
-// full-warp shuffle, and the first lane of each segment replaces them with
-// the fresh ones of its column.
-template <int TM>
-__device__ __forceinline__ void stream_segment16(const BatchLaunch &B, int cls, int seg_id, int lane, int sl,
-                                                 int SEG)
-{
-    const CombLaunch &L = B.wf;
-    const int r0 = sl * TM;
-    const int seg_lane0 = lane - sl;
-    const int beg = cls < 0 ? 0 : B.seg_off[seg_id];
-    ItemSource src{B.seg_list + beg, B.seg_list2 + beg, cls < 0 ? 0 : B.seg_off[seg_id + 1] - beg, 0, cls, -1};
-
-    // The first two couples, picked by lane 0 and shared with the segment.
-    int a0 = -1, b0 = -1, a1 = -1, b1 = -1;
-    if (sl == 0) {
-        src.pick(B, a0, b0);
-        if (a0 >= 0) src.pick(B, a1, b1);
-    }
-    a0 = __shfl_sync(FULL_MASK, a0, seg_lane0);
-    b0 = __shfl_sync(FULL_MASK, b0, seg_lane0);
-    a1 = __shfl_sync(FULL_MASK, a1, seg_lane0);
-    b1 = __shfl_sync(FULL_MASK, b1, seg_lane0);
-    CoupleTask<TM> T;
-    NextCouple<TM> N;
-    uint32_t ap[TM], hp[TM];
-    fetch_next<TM>(L, a0, r0, N.A);
-    fetch_next<TM>(L, b0, r0, N.B);
-    take_couple<TM>(L, N, r0, T, ap, hp);
-    fetch_next<TM>(L, a1, r0, N.A);
-    fetch_next<TM>(L, b1, r0, N.B);
-    int nxa = a1, nxb = b1; // the couple after the current one (already fetched)
-    int blk = -sl;
-
-    uint32_t vc[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) vc[j] = 0x7FFF7FFFu;
-
-    for (int it = 0;; ++it) {
-        const bool live = T.pa >= 0;
-        if ((it & 3) == 0 && !__any_sync(FULL_MASK, live)) break;
-        const bool act = live && blk >= 0;
-        const int c = blk * 4;
-        const int upa = __shfl_up_sync(FULL_MASK, nxa, 1); // lane l - 1's next couple
-        const int upb = __shfl_up_sync(FULL_MASK, nxb, 1);
-
-        // Blocks where both pairs have all 4 columns (and b is word-aligned)
-        // take the short forms below; the pair edges take the checked ones.
-        const bool fast = act && blk < T.full_blocks;
-
-        uint32_t vi[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) vi[j] = __shfl_up_sync(FULL_MASK, vc[j], 1);
-        if (sl == 0) {
-            if (fast) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) vi[j] = T.vbase + uint32_t(c + j) * 0x00010001u;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t lo = (act && c + j < T.na) ? uint32_t(T.ma + c + j + 1) : 0x7FFFu;
-                    const uint32_t hi = (act && T.pb >= 0 && c + j < T.nb_cols) ? uint32_t(T.mb + c + j + 1) : 0x7FFFu;
-                    vi[j] = lo | (hi << 16);
-                }
-            }
-        }
-
-        uint32_t bp[4];
-        if (fast) {
-            const uint32_t wa = __ldg(reinterpret_cast<const uint32_t *>(T.ba + c));
-            const uint32_t wb = __ldg(reinterpret_cast<const uint32_t *>(T.bb + c));
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                bp[j] = __byte_perm(wa, wb, j | (j << 4) | ((4 + j) << 8) | ((4 + j) << 12)) & 0x00FF00FFu;
-        } else {
-            bool fa = false, fb = false;
-            const uint32_t wa = act ? sym4(T.ba, c, T.na, fa) : 0u;
-            const uint32_t wb = (act && T.pb >= 0) ? sym4(T.bb, c, T.nb_cols, fb) : 0u;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t sa = (act && c + j < T.na) ? ((wa >> (8 * j)) & 0xffu) : 0x100u;
-                const uint32_t sb = (act && T.pb >= 0 && c + j < T.nb_cols) ? ((wb >> (8 * j)) & 0xffu) : 0x100u;
-                bp[j] = sa | (sb << 16);
-            }
-        }
-
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            uint32_t v = vi[j];
-#pragma unroll
-            for (int k = 0; k < TM; ++k) cell16(ap[k], bp[j], hp[k], v);
-            vc[j] = v;
-        }
-
-        if (sl == SEG - 1 && act) {
-            if (fast) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    T.va[c + j] = int32_t(vc[j] & 0xFFFFu) - 1;
-                    T.vb[c + j] = int32_t(vc[j] >> 16) - 1;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (c + j < T.na) T.va[c + j] = int32_t(vc[j] & 0xFFFFu) - 1;
-                    if (T.pb >= 0 && c + j < T.nb_cols) T.vb[c + j] = int32_t(vc[j] >> 16) - 1;
-                }
-            }
-        }
-
-        if (live && ++blk == T.nb) {
-#pragma unroll
-            for (int k = 0; k < TM; ++k) {
-                if (r0 + k < T.ma) T.ha[T.ma - 1 - r0 - k] = int32_t(hp[k] & 0xFFFFu) - 1;
-                if (T.pb >= 0 && r0 + k < T.mb) T.hb[T.mb - 1 - r0 - k] = int32_t(hp[k] >> 16) - 1;
-            }
-            take_couple<TM>(L, N, r0, T, ap, hp);
-            int pa = -1, pb = -1;
-            if (T.pa >= 0) {
-                if (sl == 0) {
-                    src.pick(B, pa, pb);
-                } else {
-                    pa = upa;
-                    pb = upb;
-                }
-            }
-            nxa = pa;
-            nxb = pb;
-            fetch_next<TM>(L, pa, r0, N.A);
-            fetch_next<TM>(L, pb, r0, N.B);
             blk = 0;
         }
     }
@@ -835,59 +561,23 @@ __device__ __forceinline__ void stream_segment16(const BatchLaunch &B, int cls, 
 // Stream classes compiled into the batch kernel: (rows per lane, lanes per segment).
 #define SLCS_STREAM_CLASSES(X) X(4, 8) X(4, 16) X(4, 32) X(8, 8) X(8, 16) X(8, 32) \
     X(12, 8) X(12, 16) X(12, 32) X(16, 8) X(16, 16) X(16, 32)
-// Packed classes (4 columns per step).
-// (Packed classes of 6, 10 and 14 rows per lane halve the row padding, but
-// compiled into this kernel they slowed every class down by 10-15 %.)
-#define SLCS_PACKED_CLASSES(X) X(4, 16) X(8, 16) X(12, 16) X(16, 16)
-
 // Four blocks of 4 warps per SM need at most 128 registers per thread.
 template <int TNS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) comb_batch_kernel(const BatchLaunch B)
 {
-    __shared__ __align__(16) int4 wf_ring[WARPS][RING];
     const int lane = threadIdx.x & 31;
     const int w = __shfl_sync(FULL_MASK, int(threadIdx.x) >> 5, 0); // warp-uniform for the compiler
     const int gw = blockIdx.x * WARPS + w;
-    const CombLaunch &L = B.wf;
-    // Phase 1: this warp's stream segments (class and lists fixed by the plan).
-    if (gw < B.nwarps) {
-        int cls = 0;
-        while (cls < B.nclass - 1 && gw >= B.class_warp_end[cls]) ++cls;
-        const int code = B.class_code[cls];
+    if (gw >= B.nwarps) return;
+    // This warp's stream segments (class and lists fixed by the plan).
+    int cls = 0;
+    while (cls < B.nclass - 1 && gw >= B.class_warp_end[cls]) ++cls;
 #define SLCS_CASE(TM, SEG)                                                                 \
     case TM * 100 + SEG:                                                                   \
-        stream_segment<TM, SEG, TNS>(B, B.class_pool[cls], SEG_SLOTS * gw + lane / SEG, lane);  \
+        stream_segment<TM, SEG, TNS>(B, cls, SEG_SLOTS * gw + lane / SEG, lane);           \
         break;
-        switch (code) { SLCS_STREAM_CLASSES(SLCS_CASE) default: break; }
+    switch (B.class_code[cls]) { SLCS_STREAM_CLASSES(SLCS_CASE) default: break; }
 #undef SLCS_CASE
-        if (TNS == 4) {
-            if (code == PACKED16_VAR_CODE + VAR_TM * 100) {
-                // one call for every lane (idle lanes too), so that the warp
-                // runs a single copy of the body without diverging
-                const int e = B.lane_map[gw * 32 + lane];
-                const bool idle = e < 0;
-                stream_segment16<VAR_TM>(B, idle ? -1 : e >> 24, idle ? 0 : SEG_SLOTS * gw + ((e >> 16) & 0xff), lane,
-                                         idle ? 0 : (e >> 8) & 0xff, idle ? 1 : e & 0xff);
-            } else {
-#define SLCS_PCASE(TM, SEG)                                                                \
-    case PACKED16_CODE + TM * 100 + SEG:                                                   \
-        stream_segment16<TM>(B, B.class_pool[cls], SEG_SLOTS * gw + lane / SEG, lane, lane & (SEG - 1), SEG); \
-        break;
-                switch (code) { SLCS_PACKED_CLASSES(SLCS_PCASE) default: break; }
-#undef SLCS_PCASE
-            }
-        }
-    }
-    // Phase 2: stripes of pairs too tall to stream, whole warps, wavefront
-    // order, taken dynamically so that they also absorb the stream tail.
-    for (;;) {
-        int k = 0;
-        if (lane == 0) k = ld_relaxed_gpu(L.counters + 1) ? INT_MAX : atomicAdd(L.counters, 1);
-        k = __shfl_sync(FULL_MASK, k, 0);
-        if (k >= L.ntasks) break;
-        const int2 tk = L.tasks[k];
-        comb_stripe<BATCH_WF_TM>(L, L.pairs[tk.x], L.scratch_off[tk.x], tk.y, k, wf_ring[w], lane);
-    }
 }
 
 __global__ void strands_to_perm_kernel(const int32_t *__restrict__ h, int32_t m, const int32_t *__restrict__ v,
@@ -1064,8 +754,6 @@ slcs_status launch_comb_on(const CombLaunch &L, int tile_m, int warps, int sms, 
     return launch_comb_sms(L, tile_m, warps, sms, stream, nullptr);
 }
 
-bool packed16_supported(int tm, int seg) { return (tm == 4 || tm == 8 || tm == 12 || tm == 16) && seg == 16; }
-
 bool stream_variant_supported(int tm, int seg)
 {
     return (tm == 4 || tm == 8 || tm == 12 || tm == 16) && (seg == 8 || seg == 16 || seg == 32);
@@ -1073,7 +761,7 @@ bool stream_variant_supported(int tm, int seg)
 
 slcs_status launch_batch(const BatchLaunch &B, int tns, cudaStream_t stream, int *grid_out)
 {
-    if (stream != PREPARE_ONLY && B.wf.ntasks <= 0 && B.nwarps <= 0) return SLCS_OK;
+    if (stream != PREPARE_ONLY && B.nwarps <= 0) return SLCS_OK;
     if (tns == 8) return launch_batch_variant<8, BATCH_WARPS>(B, stream, grid_out);
     if (tns == 4) return launch_batch_variant<4, BATCH_WARPS>(B, stream, grid_out);
     return fail(SLCS_ERR_UNSUPPORTED, "stream columns per step must be 4 or 8");

@@ -48,46 +48,27 @@ inline int32_t pick_tw(int tm, int64_t chain, int64_t width, const void *b)
     return ((tm == 14 || tm == 16) && aligned && chain * 2000 <= width) ? 8 : 4;
 }
 
-// A batch launch: multi-stripe pairs go through the wavefront tasks above
-// (whole warps, tile_m rows per lane), then every single-stripe pair is
-// streamed: a segment of `seg` lanes combs pair after pair without draining
-// its pipeline between them.
+// A batch launch: pairs of at most 512 rows with 32-bit strands are streamed:
+// a segment of `seg` lanes combs pair after pair without draining its pipeline
+// between them.  (Pairs whose ids fit 15 bits are combed in couples, couples.cu;
+// taller pairs by the relay kernel.)
 constexpr int MAX_CLASSES = 12;
-constexpr int MAX_POOLS = 48; // item classes with a pool: fixed classes and the lane counts of the variable one
-constexpr int SEG_SLOTS = 8;  // segment slots per warp (32 / fewest lanes of a segment)
+constexpr int SEG_SLOTS = 4;  // segment slots per warp (32 / fewest lanes of a segment)
 struct BatchLaunch {
-    CombLaunch wf;           // wavefront part (tasks of pairs too tall to stream)
+    CombLaunch wf;           // pairs, blobs, output and status (no tasks)
     const int32_t *seg_off;  // device: SEG_SLOTS*nwarps+1 offsets into seg_list (CSR)
     const int32_t *seg_list; // device: pairs of each stream segment, in order
-    const int32_t *seg_list2; // device: packed classes: the partner pair combed in the high half (-1: none)
-    int32_t nwarps;          // warps 0..nwarps-1 (grid order) stream; the rest only take wavefront tasks
+    int32_t nwarps;          // warps that stream (grid order)
     int32_t grid;            // blocks of the persistent launch
     int32_t nclass;          // stream classes; warp w serves the first class c with w < class_warp_end[c]
     int32_t class_warp_end[MAX_CLASSES];
-    int32_t class_code[MAX_CLASSES]; // rows per lane * 100 + lanes per segment (+ PACKED16_CODE when packed;
-                                     // PACKED16_VAR_CODE + rows per lane for the variable class)
-    int32_t class_pool[MAX_CLASSES]; // the pool of a fixed class
-    // Variable class (its warps come first): per warp and lane, -1 (idle) or
-    // pool << 24 | segment slot << 16 | lane in the segment << 8 | lanes of the segment.
-    const int32_t *lane_map;
-    // Pool of each class: items no segment list holds, claimed one at a time
+    int32_t class_code[MAX_CLASSES]; // rows per lane * 100 + lanes per segment
+    // Pool of each class: pairs no segment list holds, claimed one at a time
     // (pool_ticket[c]) by segments of class c whose own lists are done.
-    const int32_t *pool_list;        // device: pairs (packed classes: the low-half pair)
-    const int32_t *pool_list2;       // device: packed classes: the high-half pair (-1: none)
-    int32_t *pool_ticket;            // device: MAX_POOLS counters, zero at launch
-    int32_t pool_off[MAX_POOLS + 1]; // CSR offsets of the pools
+    const int32_t *pool_list;          // device
+    int32_t *pool_ticket;              // device: MAX_CLASSES counters, zero at launch
+    int32_t pool_off[MAX_CLASSES + 1]; // CSR offsets of the pools
 };
-// Class-code offset of the packed variant: two pairs per register, strand ids
-// in 15 bits (pairs with m + n <= PACKED16_MAX_IDS), 4 columns per step.
-constexpr int PACKED16_CODE = 10000;
-// The variable packed class: segments of any lane count (4..32) side by side
-// in a warp, 16 rows per lane, so that a pair's rows are padded to a multiple
-// of 16 instead of to a class height.
-constexpr int PACKED16_VAR_CODE = 20000;
-constexpr int VAR_TM = 16;
-constexpr int VAR_MIN_LANES = 4;
-constexpr int PACKED16_MAX_IDS = 32767;
-bool packed16_supported(int tm, int seg);
 
 // Rows per lane that slcs_comb_pair uses for an m-row pair on a device of
 // `sms` SMs (the SM count matters only from 2^19 rows), and its warps per
@@ -118,10 +99,9 @@ slcs_status launch_comb_on(const CombLaunch &L, int tile_m, int warps, int sms, 
 
 // Stream-mode variants: rows per lane and lanes per segment.
 bool stream_variant_supported(int stream_tm, int seg);
-// Enqueue one persistent batch launch (counters [0] wavefront ticket and [1]
-// abort must be zero).  Wavefront tasks use tile_m 8; streamed pairs advance
-// `tns` (4 or 8) columns per step.  With PREPARE_ONLY as the stream,
-// *grid_out receives the full persistent grid (blocks).
+// Enqueue one persistent batch launch (pool tickets must be zero); streamed
+// pairs advance `tns` (4 or 8) columns per step.  With PREPARE_ONLY as the
+// stream, *grid_out receives the full persistent grid (blocks).
 slcs_status launch_batch(const BatchLaunch &L, int tns, cudaStream_t stream, int *grid_out);
 constexpr int BATCH_WARPS = 4;
 constexpr int BATCH_WF_TM = 8;

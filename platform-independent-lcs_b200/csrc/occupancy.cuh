@@ -14,7 +14,7 @@ constexpr int MAX_DEVICES = 64;
 // attributes).  The kernel is a template argument, so that every kernel
 // keeps its own table.
 template <auto Kernel>
-slcs_status occupancy_of(int threads, int *occ_out)
+slcs_status occupancy_of(int threads, int *occ_out, size_t smem = 0)
 {
     static int per_dev[MAX_DEVICES] = {}; // 0: not queried yet
     static std::mutex mu;
@@ -24,7 +24,10 @@ slcs_status occupancy_of(int threads, int *occ_out)
     int *slot = (dev >= 0 && dev < MAX_DEVICES) ? &per_dev[dev] : nullptr;
     if (!slot || *slot == 0) {
         int occ = 0;
-        SLCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, Kernel, threads, 0));
+        // Dynamic shared memory beyond 48 KB is opted into once per device.
+        if (smem > 0)
+            SLCS_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        SLCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, Kernel, threads, smem));
         if (occ < 1) occ = 1;
         if (!slot) {
             *occ_out = occ;
