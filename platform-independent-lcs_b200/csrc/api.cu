@@ -186,7 +186,8 @@ struct RelayCost {
     double step;
 };
 const RelayCost RELAY_COSTS[] = {{{1, 4, 3}, 66.0},  {{2, 4, 3}, 79.0},  {{4, 2, 3}, 76.0},
-                                 {{8, 2, 3}, 108.0}, {{8, 4, 4}, 212.0}, {{16, 4, 4}, 425.0}};
+                                 {{8, 2, 3}, 108.0}, {{8, 4, 4}, 212.0}, {{14, 4, 4}, 344.0},
+                                 {{14, 4, 8}, 665.0}, {{14, 4, 16}, 1277.0}};
 constexpr double RELAY_GHZ = 1.965;     // the clock those cycles were measured at
 constexpr double RELAY_WARP_LAG = 40.0; // steps a warp starts after the warp above it
 constexpr double RELAY_HOP_LAG = 45.0;  // more steps for the hand-down to the next block

@@ -314,7 +314,7 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                             store_block_if<TW>(lane == 31, &S.strands[w + 1][(base + s - 31) & (RING - 1)][0], vc);
                         }
                     } else {
-#pragma unroll 2 // all K steps would overflow the instruction cache
+#pragma unroll 4 // all 8 overflow the instruction cache (16 rows: 708 cycles a step, 4: 388, 2: 425)
                         for (int s = 0; s < K; ++s) {
                             int vi[TW], bs[TW];
 #pragma unroll
@@ -369,7 +369,8 @@ slcs_status launch_shape(const RelayLaunch &L, int sms, cudaStream_t stream)
 
 } // namespace
 
-#define SLCS_RELAY_SHAPES(X) X(1, 4, 3) X(2, 4, 3) X(4, 2, 3) X(8, 2, 3) X(8, 4, 4) X(16, 4, 4)
+#define SLCS_RELAY_SHAPES(X) \
+    X(1, 4, 3) X(2, 4, 3) X(4, 2, 3) X(8, 2, 3) X(8, 4, 4) X(14, 4, 4) X(14, 4, 8) X(14, 4, 16)
 
 bool relay_supported(const RelayShape &s)
 {

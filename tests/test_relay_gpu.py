@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 # last ones reach the taller shapes and the tilings.
 SHAPES = [(1, 1), (1, 131), (131, 1), (32, 32), (33, 31), (64, 127), (96, 128), (97, 129), (128, 255), (129, 16),
           (192, 257), (193, 4), (384, 1000), (385, 1001), (769, 3), (1153, 515), (300, 20001), (20001, 300),
-          (9000, 2047), (120001, 33), (160001, 30), (70001, 300), (90, 70003)]
+          (9000, 2047), (116003, 2001), (120001, 33), (260001, 17), (600001, 13),
+          (70001, 300), (90, 70003)]
 
 
 @pytest.fixture(scope="module")
@@ -27,7 +28,8 @@ def test_relay_shapes(cuda, seen, m, n):
     import torch
     info = slcs.pair_plan_info(m, n)
     assert info["relay_tile_m"] > 0
-    seen.add((info["relay_tile_m"], info["relay_cols"], info["relay_strips"] > 1, info["relay_bands"] > 1))
+    seen.add((info["relay_tile_m"], info["relay_cols"], info["relay_warps"], info["relay_strips"] > 1,
+              info["relay_bands"] > 1))
     rng = np.random.default_rng(m * 7 + n)
     sigma = int(rng.choice([2, 4, 256]))
     a, b = rng.integers(0, sigma, m, dtype=np.uint8), rng.integers(0, sigma, n, dtype=np.uint8)
@@ -43,5 +45,6 @@ def test_relay_shapes(cuda, seen, m, n):
 
 def test_relay_shapes_reached(seen):
     """The sizes above reach every shape, strips and bands."""
-    assert {(t, c) for t, c, _, _ in seen} == {(1, 4), (2, 4), (4, 2), (8, 2), (8, 4), (16, 4)}
-    assert any(s for _, _, s, _ in seen) and any(r for _, _, _, r in seen)
+    assert {x[:3] for x in seen} == {(1, 4, 3), (2, 4, 3), (4, 2, 3), (8, 2, 3), (8, 4, 4), (14, 4, 4), (14, 4, 8),
+                                     (14, 4, 16)}
+    assert any(x[3] for x in seen) and any(x[4] for x in seen)
