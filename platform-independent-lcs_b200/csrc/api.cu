@@ -766,43 +766,154 @@ slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_
     return s;
 }
 
+// A stream and a page-locked buffer for one host-pointer call at a time.  A
+// call takes an idle one (or makes one) and gives it back; at most LANES_KEPT
+// stay.  (A stream made and destroyed per call, and pageable copies one by one,
+// cost a small pair about 125 us.)
+namespace {
+struct HostLane {
+    int device = -1;
+    cudaStream_t st = nullptr;
+    char *pinned = nullptr; // LANE_BYTES, or null when it could not be had
+};
+constexpr size_t LANE_BYTES = size_t(2) << 20;
+constexpr size_t LANES_KEPT = 4;
+std::mutex g_lane_mu;
+std::vector<HostLane> g_lanes;
+
+void drop_lane(HostLane &l)
+{
+    if (l.st) cudaStreamDestroy(l.st);
+    if (l.pinned) cudaFreeHost(l.pinned);
+    l = HostLane{};
+}
+
+slcs_status take_lane(HostLane *l)
+{
+    int dev = 0;
+    SLCS_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> g(g_lane_mu);
+        for (size_t i = 0; i < g_lanes.size(); ++i)
+            if (g_lanes[i].device == dev) {
+                *l = g_lanes[i];
+                g_lanes.erase(g_lanes.begin() + long(i));
+                return SLCS_OK;
+            }
+    }
+    l->device = dev;
+    SLCS_CUDA(cudaStreamCreateWithFlags(&l->st, cudaStreamNonBlocking));
+    if (cudaHostAlloc(reinterpret_cast<void **>(&l->pinned), LANE_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        l->pinned = nullptr;
+    }
+    return SLCS_OK;
+}
+
+// With its stream synchronised; after a failed call a lane is dropped.
+void give_lane(HostLane &l, bool good)
+{
+    if (good) {
+        std::lock_guard<std::mutex> g(g_lane_mu);
+        if (g_lanes.size() < LANES_KEPT) {
+            g_lanes.push_back(l);
+            return;
+        }
+    }
+    drop_lane(l);
+}
+
+// One pair from host memory: symbols of `width` bytes (1, or 4 for Words that
+// become bytes on the device).
+slcs_status comb_host(const void *a, int32_t m, const void *b, int32_t n, size_t width, int32_t *h_out, int32_t *v_out,
+                      const slcs_config *cfg)
+{
+    const bool words = width > 1;
+    HostLane lane;
+    slcs_status s = take_lane(&lane);
+    if (s != SLCS_OK) {
+        drop_lane(lane);
+        return s;
+    }
+    cudaStream_t st = lane.st;
+    (void)sm_count(); // per-device set-up (memory pool) before the first allocation
+    // Device: [a | b | strands | alphabet | a and b as bytes | symbol workspace];
+    // the lane's buffer holds a and b, then strands and alphabet, in the same layout.
+    const size_t na = width * size_t(m), nb = width * size_t(n);
+    const size_t o_b = align_up(na + 16, 256), in_bytes = o_b + nb;
+    const size_t o_out = align_up(in_bytes + 16, 256), n_out = sizeof(int32_t) * (size_t(m) + n);
+    const size_t o_alpha = o_out + n_out, out_bytes = n_out + (words ? sizeof(int32_t) : 0);
+    const size_t o_ab = align_up(o_out + out_bytes + 16, 256);
+    const size_t o_bb = o_ab + (words ? align_up(size_t(m) + 16, 256) : 0);
+    const size_t o_ws = o_bb + (words ? align_up(size_t(n) + 16, 256) : 0);
+    char *buf = nullptr;
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&buf), o_ws + (words ? symbols_workspace_bytes() : 0), st);
+    if (e != cudaSuccess) {
+        give_lane(lane, true);
+        return cuda_fail(e, "cudaMallocAsync");
+    }
+    char *pin = o_out + out_bytes <= LANE_BYTES ? lane.pinned : nullptr;
+    if (pin) {
+        if (m) std::memcpy(pin, a, na);
+        if (n) std::memcpy(pin + o_b, b, nb);
+        if (m > 0 || n > 0) e = cudaMemcpyAsync(buf, pin, in_bytes, cudaMemcpyHostToDevice, st);
+    } else {
+        if (m) e = cudaMemcpyAsync(buf, a, na, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && n) e = cudaMemcpyAsync(buf + o_b, b, nb, cudaMemcpyHostToDevice, st);
+    }
+    const uint8_t *da = reinterpret_cast<uint8_t *>(buf), *db = reinterpret_cast<uint8_t *>(buf + o_b);
+    int32_t *dout = reinterpret_cast<int32_t *>(buf + o_out), *dalpha = reinterpret_cast<int32_t *>(buf + o_alpha);
+    int32_t alphabet = 0;
+    if (words && e == cudaSuccess) {
+        uint8_t *ab = reinterpret_cast<uint8_t *>(buf + o_ab), *bb = reinterpret_cast<uint8_t *>(buf + o_bb);
+        s = symbols_to_bytes(reinterpret_cast<const int32_t *>(da), m, reinterpret_cast<const int32_t *>(db), n, ab, bb,
+                             dalpha, buf + o_ws, st);
+        da = ab;
+        db = bb;
+        // The alphabet decides before a long comb; a short one it comes back with.
+        if (s == SLCS_OK && !(pin && int64_t(m) * n < (int64_t(1) << 28))) {
+            e = cudaMemcpyAsync(&alphabet, dalpha, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        }
+    }
+    if (e == cudaSuccess && s == SLCS_OK && alphabet >= 0) {
+        s = slcs_comb_pair(da, m, db, n, dout, dout + m, cfg, st);
+        if (s == SLCS_OK && pin) {
+            if (out_bytes) e = cudaMemcpyAsync(pin + o_out, dout, out_bytes, cudaMemcpyDeviceToHost, st);
+        } else if (s == SLCS_OK) {
+            if (m) e = cudaMemcpyAsync(h_out, dout, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess && n)
+                e = cudaMemcpyAsync(v_out, dout + m, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
+        }
+    }
+    const cudaError_t f = cudaFreeAsync(buf, st);
+    if (e == cudaSuccess) e = f;
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess && s == SLCS_OK && pin) {
+        if (words) std::memcpy(&alphabet, pin + o_alpha, sizeof(alphabet));
+        if (alphabet >= 0) {
+            if (m) std::memcpy(h_out, pin + o_out, sizeof(int32_t) * m);
+            if (n) std::memcpy(v_out, pin + o_out + sizeof(int32_t) * m, sizeof(int32_t) * n);
+        }
+    }
+    give_lane(lane, e == cudaSuccess);
+    if (s != SLCS_OK) return s;
+    if (e != cudaSuccess) return cuda_fail(e, "symbol or strand copies");
+    if (alphabet < 0) return fail(SLCS_ERR_RANGE, "more than 256 distinct symbols in a and b");
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return slcs_device_status(dev, 1);
+}
+} // namespace
+
 slcs_status slcs_comb_pair_host(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n, int32_t *h_out,
                                 int32_t *v_out, const slcs_config *cfg)
 {
     if (m < 0 || n < 0) return fail(SLCS_ERR_INVALID, "m and n must be >= 0");
     if ((m > 0 && (!a || !h_out)) || (n > 0 && (!b || !v_out)))
         return fail(SLCS_ERR_INVALID, "null pointer for a non-empty side");
-    cudaStream_t st = nullptr;
-    SLCS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    const size_t ab = align_up(size_t(m) + 16, 256), bb = align_up(size_t(n) + 16, 256);
-    const size_t sb = sizeof(int32_t) * (size_t(m) + n + 4);
-    char *buf = nullptr;
-    slcs_status s = SLCS_OK;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&buf), ab + bb + sb, st);
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(st);
-        return cuda_fail(e, "cudaMallocAsync");
-    }
-    uint8_t *da = reinterpret_cast<uint8_t *>(buf);
-    uint8_t *db = reinterpret_cast<uint8_t *>(buf + ab);
-    int32_t *dout = reinterpret_cast<int32_t *>(buf + ab + bb);
-    if (m) e = cudaMemcpyAsync(da, a, m, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(db, b, n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
-        s = slcs_comb_pair(da, m, db, n, dout, dout + m, cfg, st);
-        if (s == SLCS_OK && m) e = cudaMemcpyAsync(h_out, dout, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, st);
-        if (s == SLCS_OK && e == cudaSuccess && n)
-            e = cudaMemcpyAsync(v_out, dout + m, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
-    }
-    cudaFreeAsync(buf, st);
-    cudaError_t e2 = cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-    if (s != SLCS_OK) return s;
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync");
-    if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamSynchronize");
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return slcs_device_status(dev, 1);
+    return comb_host(a, m, b, n, sizeof(uint8_t), h_out, v_out, cfg);
 }
 
 slcs_status slcs_symbols_to_bytes(const int32_t *a, int32_t m, const int32_t *b, int32_t n, uint8_t *a_out,
@@ -827,49 +938,7 @@ slcs_status slcs_comb_pair_words_host(const int32_t *a, int32_t m, const int32_t
     if ((m > 0 && (!a || !h_out)) || (n > 0 && (!b || !v_out)))
         return fail(SLCS_ERR_INVALID, "null pointer for a non-empty side");
     if (int64_t(m) + n > INT32_MAX) return fail(SLCS_ERR_RANGE, "m+n exceeds int32 strand ids");
-    cudaStream_t st = nullptr;
-    SLCS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    // [a words | b words | a bytes | b bytes | strands | alphabet | symbol workspace]
-    const size_t o_bw = align_up(sizeof(int32_t) * size_t(m), 256);
-    const size_t o_ab = o_bw + align_up(sizeof(int32_t) * size_t(n), 256);
-    const size_t o_bb = o_ab + align_up(size_t(m) + 16, 256);
-    const size_t o_out = o_bb + align_up(size_t(n) + 16, 256);
-    const size_t o_alpha = o_out + align_up(sizeof(int32_t) * (size_t(m) + n), 256);
-    const size_t o_ws = o_alpha + 256;
-    const size_t bytes = o_ws + symbols_workspace_bytes();
-    char *buf = nullptr;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&buf), bytes, st);
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(st);
-        return cuda_fail(e, "cudaMallocAsync");
-    }
-    int32_t *da = reinterpret_cast<int32_t *>(buf), *db = reinterpret_cast<int32_t *>(buf + o_bw);
-    uint8_t *ab = reinterpret_cast<uint8_t *>(buf + o_ab), *bb = reinterpret_cast<uint8_t *>(buf + o_bb);
-    int32_t *dout = reinterpret_cast<int32_t *>(buf + o_out), *dalpha = reinterpret_cast<int32_t *>(buf + o_alpha);
-    slcs_status s = SLCS_OK;
-    int32_t alphabet = 0;
-    if (m) e = cudaMemcpyAsync(da, a, sizeof(int32_t) * size_t(m), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(db, b, sizeof(int32_t) * size_t(n), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) s = symbols_to_bytes(da, m, db, n, ab, bb, dalpha, buf + o_ws, st);
-    if (e == cudaSuccess && s == SLCS_OK) e = cudaMemcpyAsync(&alphabet, dalpha, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && s == SLCS_OK) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess && s == SLCS_OK && alphabet < 0)
-        s = fail(SLCS_ERR_RANGE, "more than 256 distinct symbols in a and b");
-    if (e == cudaSuccess && s == SLCS_OK) {
-        s = slcs_comb_pair(ab, m, bb, n, dout, dout + m, cfg, st);
-        if (s == SLCS_OK && m) e = cudaMemcpyAsync(h_out, dout, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, st);
-        if (s == SLCS_OK && e == cudaSuccess && n)
-            e = cudaMemcpyAsync(v_out, dout + m, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
-    }
-    cudaFreeAsync(buf, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-    if (s != SLCS_OK) return s;
-    if (e != cudaSuccess) return cuda_fail(e, "symbol or strand copies");
-    if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamSynchronize");
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return slcs_device_status(dev, 1);
+    return comb_host(a, m, b, n, sizeof(int32_t), h_out, v_out, cfg);
 }
 
 static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_desc *pairs, int32_t npairs,
