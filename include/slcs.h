@@ -188,7 +188,7 @@ SLCS_API slcs_status slcs_symbols_to_bytes(const int32_t *a, int32_t m, const in
 /* One pair of Word symbols from host memory: copies the words in, maps them
  * to bytes on the device (slcs_symbols_to_bytes), combs, copies the strands
  * out and synchronises.  More than 256 distinct symbols give SLCS_ERR_RANGE
- * before any comb.  The entry point the reference-side procedure adapter
+ * and leave the outputs alone.  The entry point the reference-side procedure adapter
  * binds (src/algorithm_registry.cpp:59-73 hands it the Word arrays). */
 SLCS_API slcs_status slcs_comb_pair_words_host(const int32_t *a, int32_t m, const int32_t *b, int32_t n,
                                                int32_t *h_out, int32_t *v_out, const slcs_config *cfg);
@@ -297,7 +297,8 @@ SLCS_API int64_t slcs_permutation_hash(const int32_t *col_to_row, int32_t size);
 /* staggered_multiply<RowGlue> (src/braid_multiplication.hpp:273-407) of two
  * full permutations given as device row->col arrays; out_row_to_col receives
  * p_size + q_size - k entries.  Steady-ant recursion (204-270) runs on the
- * device; nodes at or below cfg->braid_cutoff are finished by one block. */
+ * device; nodes at or below cfg->braid_cutoff (0, or more than a block takes:
+ * 1200) are finished by one block. */
 SLCS_API slcs_status slcs_braid_multiply(const int32_t *p_row_to_col, int32_t p_size, const int32_t *q_row_to_col,
                                 int32_t q_size, int32_t k, int32_t row_glue, int32_t *out_row_to_col,
                                 const slcs_config *cfg, void *stream);

@@ -713,7 +713,7 @@ slcs_status slcs_comb_pair(const uint8_t *a, int32_t m, const uint8_t *b, int32_
         slcs_config rc{};
         rc.strips = pp.relay.strips;
         rc.bands = pp.relay.bands;
-        rc.braid_cutoff = cfg && cfg->braid_cutoff > 0 ? cfg->braid_cutoff : 256;
+        rc.braid_cutoff = cfg ? cfg->braid_cutoff : 0;
         rc.wait_ms = cfg ? cfg->wait_ms : 0;
         return comb_strips(a, m, b, n, h_out, v_out, &rc, 0, 0, &pp.relay.relay, st);
     }
@@ -1962,7 +1962,7 @@ slcs_status slcs_braid_multiply(const int32_t *p_r2c, int32_t p_size, const int3
         return fail(SLCS_ERR_INVALID, "null permutation pointer");
     if (p_size + q_size == 0) return SLCS_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 1024;
+    const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 0;
     (void)sm_count(); // per-device set-up (memory pool) before the first allocation
     size_t bytes = 0;
     braid_workspace_bytes(p_size, q_size, k, cutoff, &bytes);

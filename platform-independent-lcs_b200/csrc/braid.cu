@@ -17,9 +17,9 @@
 //     first waits for the tiles of the level above that hold its parent
 //     nodes; every wait is bounded.  The maps from child index to parent
 //     index are kept per level.
-//   * A node at or below the cutoff is finished by one thread block: it loads
-//     the node into shared memory (16-bit local indices) and runs every lower
-//     level of its subtree there, down and back up, with block-wide scans.
+//   * A node at or below the cutoff is finished by one thread block without
+//     further recursion: it passes the crossings of P's part into Q's, S / 2
+//     at a time, in S rounds of one packed compare-and-exchange (node_kernel).
 //   * Upward, a level scatters both children's products into the parent's
 //     rows and columns (inverse_mapping, 191-202) and, in the same pass, into
 //     the parent's result (the union of the two halves, 254-268) and into the
@@ -48,12 +48,6 @@ constexpr int PART_PER = 8;     // entries per thread of a partition tile
 // a short look-back chain) for large products, 256 (2048 entries) below.
 constexpr int PART_BIG_K = 1 << 19;
 __host__ __device__ constexpr int part_threads(int k) { return k >= PART_BIG_K ? 1024 : 256; }
-constexpr int SUB_THREADS = 512; // threads of the subtree block
-constexpr int SUB_MAX = 4096;   // largest node a block finishes in shared memory
-// Shared memory of a subtree block for nodes of up to maxn entries: two int32
-// word arrays and six int16 arrays.
-constexpr size_t subtree_smem(int maxn) { return size_t(maxn) * 4 * 2 + size_t(maxn) * 2 * 6; }
-
 __host__ __device__ __forceinline__ void node_of(int i, int level, int k, int &o, int &s)
 {
     o = 0;
@@ -639,216 +633,62 @@ __device__ __forceinline__ void ant_walk_warp(int dr, int dc, int delta, int s, 
 }
 
 // ---------------------------------------------------------------------------
-// block-wide scans for the subtree kernel
+// nodes at or below the cutoff
 // ---------------------------------------------------------------------------
-template <int THREADS>
-__device__ __forceinline__ void block_scan2(int &a, int &b, int *wa, int *wb)
-{
-    // inclusive scan of (a, b) across the block; returns exclusive values
-    const int va = a, vb = b;
-    for (int off = 1; off < 32; off <<= 1) {
-        int ya = __shfl_up_sync(FULL_MASK, a, off), yb = __shfl_up_sync(FULL_MASK, b, off);
-        if ((threadIdx.x & 31) >= off) {
-            a += ya;
-            b += yb;
-        }
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 31) {
-        wa[w] = a;
-        wb[w] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        int sa = threadIdx.x < THREADS / 32 ? wa[threadIdx.x] : 0;
-        int sb = threadIdx.x < THREADS / 32 ? wb[threadIdx.x] : 0;
-        for (int off = 1; off < 32; off <<= 1) {
-            int ya = __shfl_up_sync(FULL_MASK, sa, off), yb = __shfl_up_sync(FULL_MASK, sb, off);
-            if (threadIdx.x >= off) {
-                sa += ya;
-                sb += yb;
-            }
-        }
-        if (threadIdx.x < THREADS / 32) {
-            wa[threadIdx.x] = sa;
-            wb[threadIdx.x] = sb;
-        }
-    }
-    __syncthreads();
-    a = a - va + (w ? wa[w - 1] : 0);
-    b = b - vb + (w ? wb[w - 1] : 0);
-    __syncthreads();
-}
-
-struct SubArgs {
-    const int32_t *P; // level lc arrays (global)
+struct NodeArgs {
+    const int32_t *P; // level lc arrays (global): P's rows by column, Q's columns by row
     const int32_t *Q;
     int32_t *res;     // level lc result (global), node-local r2c
-    int32_t *maps;    // base of per-level map arrays: pmap of level l at maps + 2*k*l, qmap at + k
     int k, lc;
     const int32_t *bad;
 };
 
-// Nodes below a subtree block's node (size S): the halving tree of S.  When S
-// is a power of two every node of depth d has size S >> d and starts at a
-// multiple of it, so the lookups are bit operations; otherwise node_of walks
-// down from the top.
-struct SubNodes {
-    int S;
-    bool pow2;
-    __device__ __forceinline__ void at(int i, int d, int &o, int &s) const
-    {
-        if (pow2) {
-            s = S >> d;
-            o = i & ~(s - 1);
-        } else {
-            node_of(i, d, S, o, s);
-        }
-    }
-    // node nd (0-based, left to right) of depth d
-    __device__ __forceinline__ void nth(int nd, int d, int &o, int &s) const
-    {
-        if (pow2) {
-            s = S >> d;
-            o = nd * s;
-            return;
-        }
-        o = 0;
-        s = S;
-        for (int e = 0; e < d; ++e) {
-            const int h = s >> 1;
-            if ((nd >> (d - 1 - e)) & 1) {
-                o += h;
-                s -= h;
-            } else {
-                s = h;
-            }
-        }
-    }
-};
-
-// One block finishes the subtree of one node of level lc (size <= MAXN):
-// every deeper level, down then up, in shared memory (the per-level maps,
-// child index -> parent-local index, in global memory).  Smaller variants
-// (fewer threads, less shared memory) keep more blocks resident per SM when
-// the cutoff is small.
-// The walk of one node (offset po, size ps) inside a subtree block, cut into
-// segments like the walks of the levels above the cutoff: a delta table of
-// SUB_G + 1 grid lines per dimension (spacing B = ps / SUB_G, rounded up) is
-// counted and summed in shared memory, then thread q walks segment q: the
-// diagonals (E, E + B] with E = (q - ceil(ps / B)) B, from one row above
-// r*(E), the first row of diagonal E whose delta is >= 0 (a search of the
-// table along the diagonal, then a scan of at most B rows).  Every thread of
-// the block calls it (it synchronises the block).
-constexpr int SUB_G = 16;
-constexpr int SUB_TAB = (SUB_G + 1) * (SUB_G + 1);
-template <int THREADS>
-__device__ void sub_walk_segmented(const int32_t *CW, const int32_t *RW, int16_t *Res, int po, int ps, int32_t *Th,
-                                   int32_t *Tl)
+// One round element of a node: P's row that ends on middle position j in the
+// high half, the complement of the column where Q's row j ends in the low half.
+__device__ __forceinline__ uint32_t pass_low(uint32_t l, uint32_t r) { return l > r ? __vminu2(l, r) : l; }
+__device__ __forceinline__ uint32_t pass_high(uint32_t l, uint32_t r) { return l > r ? __vmaxu2(l, r) : r; }
+__device__ __forceinline__ void pass_pair(uint32_t &l, uint32_t &r)
 {
-    const int B = (ps + SUB_G - 1) / SUB_G;
-    const int G = ps / B, W = G + 1;
-    for (int i = threadIdx.x; i < W * W; i += THREADS) {
-        Th[i] = 0;
-        Tl[i] = 0;
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < ps; r += THREADS) {
-        const int w = CW[po + r];
-        const int bi = min(r / B, G), bj = min((w & INT_MAX) / B, G);
-        atomicAdd((w < 0 ? Th : Tl) + bi * W + bj, 1);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < W; i += THREADS) { // rows: hi exclusive prefix, lo inclusive suffix
-        int run = 0;
-        for (int j = 0; j < W; ++j) {
-            const int v = Th[i * W + j];
-            Th[i * W + j] = run;
-            run += v;
-        }
-        run = 0;
-        for (int j = G; j >= 0; --j) {
-            run += Tl[i * W + j];
-            Tl[i * W + j] = run;
-        }
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < W; j += THREADS) { // columns, then delta into the hi table
-        int run = 0;
-        for (int i = G; i >= 0; --i) {
-            run += Tl[i * W + j];
-            Tl[i * W + j] = run;
-        }
-        run = 0;
-        for (int i = 0; i < W; ++i) {
-            const int v = Th[i * W + j];
-            Th[i * W + j] = run - Tl[i * W + j];
-            run += v;
-        }
-    }
-    __syncthreads();
-    const int32_t *cw_ = CW + po, *rw_ = RW + po;
-    const int jmin = -((ps + B - 1) / B);
-    const int nseg = 2 * ((ps + B - 1) / B) + 2;
-    const int e0 = -(ps - 1);
-    for (int q = threadIdx.x; q < nseg; q += THREADS) {
-        const int E = (jmin + q) * B;
-        if (E > ps || E + B < e0) continue;
-        int dr, dc, delta;
-        if (E < e0) {
-            dr = ps - 1;
-            dc = 0;
-            delta = cw_[ps - 1] < 0 ? 0 : -1;
-        } else {
-            const int rlo = max(0, -E), rhi = min(ps, ps - E);
-            if (rlo > rhi) continue;
-            const int jj = E / B;
-            const int ilo = rlo / B, ihi = rhi / B;
-            int lo_i = ilo, hi_i = ihi + 1;
-            while (lo_i < hi_i) {
-                const int mid = (lo_i + hi_i) >> 1;
-                if (Th[mid * W + mid + jj] >= 0) hi_i = mid;
-                else lo_i = mid + 1;
-            }
-            int rstar = rlo;
-            int dval = Th[ilo * W + ilo + jj]; // delta(rlo, rlo + E): a grid point
-            if (lo_i != ilo) {
-                dval = Th[(lo_i - 1) * W + (lo_i - 1) + jj];
-                const int rend = min(lo_i * B, rhi);
-                rstar = rhi + 1;
-                for (int r = (lo_i - 1) * B; r < rend; ++r) {
-                    dval += word_inc(rw_[r + E], r) + word_inc(cw_[r], r + E + 1);
-                    if (dval >= 0) {
-                        rstar = r + 1;
-                        break;
-                    }
-                }
-            }
-            dr = rstar - 1;
-            dc = rstar + E;
-            if (rstar > rhi || dr < 0 || dc > ps) continue;
-            delta = dval - word_inc(cw_[dr], dc);
-        }
-        ant_walk(dr, dc, delta, ps, E + B, [&](int r) { return cw_[r]; }, [&](int c) { return rw_[c]; },
-                 [&](int r, int c) { Res[po + r] = int16_t(c); });
-    }
-    __syncthreads();
+    const uint32_t low = pass_low(l, r);
+    r = l + r - low; // both halves keep their sums
+    l = low;
 }
 
-// Segmented walks inside a subtree block: nodes of at least SUB_SEG_MIN
-// entries on levels of at most SUB_SEG_NODES nodes.
-constexpr int SUB_SEG_MIN = 64;
-constexpr int SUB_SEG_NODES = 4;
+// One block multiplies one node of level lc (size S <= NODE_MAX) by passing
+// P's crossings into Q one by one, without any recursion.  Odd-even
+// transposition sorts P's strands along the middle: every exchange is one
+// crossing of a reduced word of P taken off P's right end, and
+// sigma_j . R exchanges rows j and j + 1 of R unless those two strands have
+// crossed already.  With R's columns complemented both exchanges take the
+// smaller half to the left, so one packed minimum does them (4 instructions a
+// pair).  S rounds of S / 2 independent pairs: S^2 / 2 pairs in all, against
+// S log S steps of a recursion, whose walks and scans are serial chains.  A
+// 1024-entry node took 183 us as a shared-memory recursion and takes 32 us
+// here, bound by the ALU pipe (30 of its 40 instructions a lane per round run
+// at half rate); products of k = 1003 231 -> 75 us, 32768 486 -> 334 us
+// (MEASURED).  Larger nodes lose to one more level of the recursion: 2048
+// entries 93 us, against two of 1024 side by side and a level of about 45 us.
+//
+// A lane holds NODE_E consecutive entries: rounds of even pairs stay in the
+// lane, odd ones cross one lane boundary (two shuffles, both sides compute
+// their half).  With several warps each warp owns 30 lanes, and its outer two
+// lanes repeat the neighbours' edge lanes: a round spoils one more of their
+// entries from the outside, so NODE_E rounds pass before the edges are
+// exchanged through shared memory at one barrier.  NODE_E = 10 gives a
+// 1024-entry node four warps, one on each SM sub-partition (8 gave it five:
+// whole product of k = 1024 76 us against 67).
+constexpr int NODE_E = 10;
+constexpr int NODE_OWN = 30 * NODE_E; // entries a warp owns when a block has several
+constexpr int NODE_MAX = 1200;
+constexpr int NODE_WARPS = (NODE_MAX + NODE_OWN - 1) / NODE_OWN;
+inline int node_warps(int smax) { return smax <= 32 * NODE_E ? 1 : (smax + NODE_OWN - 1) / NODE_OWN; }
 
-// Blocks kept resident per SM (bounds the registers): 12, 5 and 2 for the
-// 128-, 256- and 512-thread variants.
-constexpr int subtree_min_blocks(int threads) { return threads <= 128 ? 12 : (threads <= 256 ? 5 : 2); }
-
-template <int MAXN, int THREADS>
-__global__ void __launch_bounds__(THREADS, subtree_min_blocks(THREADS)) subtree_kernel(SubArgs A)
+template <bool ONE_WARP>
+__global__ void __launch_bounds__(ONE_WARP ? 32 : NODE_WARPS * 32) node_kernel(NodeArgs A)
 {
     if (*A.bad) return;
-    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint16_t half[2 * (ONE_WARP ? 32 * NODE_E : NODE_MAX)]; // entry j: column half, row half
+    __shared__ __align__(8) uint32_t edge[ONE_WARP ? 1 : 2][ONE_WARP ? 1 : NODE_WARPS][2][NODE_E];
     // node of this block: descend lc levels following the bits of blockIdx.x
     int o = 0, S = A.k;
     for (int d = 0; d < A.lc; ++d) {
@@ -860,168 +700,61 @@ __global__ void __launch_bounds__(THREADS, subtree_min_blocks(THREADS)) subtree_
             S = h;
         }
     }
-    const SubNodes N{S, S > 0 && (S & (S - 1)) == 0};
-    int32_t *CW = reinterpret_cast<int32_t *>(smem); // row words of the node being walked
-    int32_t *RW = CW + MAXN;                         // column words
-    int16_t *Pa = reinterpret_cast<int16_t *>(RW + MAXN);
-    int16_t *Qa = Pa + MAXN;
-    int16_t *Pb = Qa + MAXN;
-    int16_t *Qb = Pb + MAXN;
-    int16_t *ResA = Qb + MAXN;
-    int16_t *ResB = ResA + MAXN;
-    __shared__ int wa[32], wb[32];
-    __shared__ int32_t sTh[SUB_TAB], sTl[SUB_TAB]; // delta table of a segmented walk
-    // map words of depth d below this block's node (child index -> parent-local index)
-    int32_t *maps0 = A.maps + size_t(2) * A.k * (A.lc + 1) + o;
-    auto pmap_of = [&](int d) { return maps0 + size_t(2) * A.k * d; };
-
-    for (int i = threadIdx.x; i < S; i += THREADS) {
-        Pa[i] = int16_t(A.P[o + i]);
-        Qa[i] = int16_t(A.Q[o + i]);
+    for (int i = threadIdx.x; i < S; i += blockDim.x) {
+        const int p = A.P[o + i], q = A.Q[o + i];
+        if (unsigned(p) < unsigned(S)) half[2 * p + 1] = uint16_t(i);
+        if (unsigned(q) < unsigned(S)) half[2 * q] = uint16_t(0xFFFF - i);
     }
     __syncthreads();
-
-    // depth of the subtree: levels until every node has size <= 1
-    int depth = 0;
-    for (int s = S; s > 1; s = s - (s >> 1)) ++depth;
-
-    constexpr int PER = MAXN / THREADS;
-    for (int d = 0; d < depth; ++d) {
-        int fp[PER], fq[PER], cp = 0, cq = 0;
-        const int i0 = threadIdx.x * PER;
+    const int lane = threadIdx.x & 31;
+    const int warp = ONE_WARP ? 0 : int(threadIdx.x >> 5), warps = ONE_WARP ? 1 : int(blockDim.x >> 5);
+    const int base = (ONE_WARP ? lane : warp * 30 + lane - 1) * NODE_E;
+    uint32_t x[NODE_E];
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int i = i0 + j;
-            fp[j] = fq[j] = 0;
-            if (i < S) {
-                int so, ss;
-                N.at(i, d, so, ss);
-                const int h = ss >> 1;
-                fp[j] = Pa[i] < h;
-                fq[j] = Qa[i] < h;
-            }
-            cp += fp[j];
-            cq += fq[j];
-        }
-        int ep = cp, eq = cq;
-        block_scan2<THREADS>(ep, eq, wa, wb);
-        // exclusive scan values stored in ResA/ResB (free during the descent)
+    for (int e = 0; e < NODE_E; ++e) {
+        const int j = base + e; // outside the node: words no neighbour exchanges with
+        x[e] = j < 0 ? 0u : j >= S ? 0xFFFFFFFFu : (uint32_t(half[2 * j + 1]) << 16 | half[2 * j]);
+    }
+    for (int t = 0; t < S; t += NODE_E) {
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int i = i0 + j;
-            if (i < S) {
-                ResA[i] = int16_t(ep);
-                ResB[i] = int16_t(eq);
+        for (int u = 0; u < NODE_E; u += 2) {
+#pragma unroll
+            for (int e = 0; e < NODE_E; e += 2) pass_pair(x[e], x[e + 1]);
+            uint32_t next = __shfl_down_sync(FULL_MASK, x[0], 1);
+            uint32_t prev = __shfl_up_sync(FULL_MASK, x[NODE_E - 1], 1);
+            if (ONE_WARP) {
+                if (lane == 31) next = 0xFFFFFFFFu;
+                if (lane == 0) prev = 0u;
             }
-            ep += fp[j];
-            eq += fq[j];
+#pragma unroll
+            for (int e = 1; e + 1 < NODE_E; e += 2) pass_pair(x[e], x[e + 1]);
+            x[NODE_E - 1] = pass_low(x[NODE_E - 1], next);
+            x[0] = pass_high(prev, x[0]);
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < S; i += THREADS) {
-            int so, ss;
-            N.at(i, d, so, ss);
-            const int h = ss >> 1, local = i - so;
-            const int p = Pa[i], q = Qa[i];
-            if (ss <= 1) {
-                Pb[i] = int16_t(p);
-                Qb[i] = int16_t(q);
-                pmap_of(d)[i] = 0;
-                pmap_of(d)[A.k + i] = 0;
-                continue;
+        if (!ONE_WARP) {
+            const int buf = (t / NODE_E) & 1;
+            if (lane == 1 || lane == 30) {
+                uint2 *to = reinterpret_cast<uint2 *>(edge[buf][warp][lane == 30]);
+#pragma unroll
+                for (int e = 0; e < NODE_E; e += 2) to[e / 2] = make_uint2(x[e], x[e + 1]);
             }
-            const int bp = ResA[i] - ResA[so], bq = ResB[i] - ResB[so];
-            const int pp = p < h ? so + bp : so + h + (local - bp);
-            const int pq = q < h ? so + bq : so + h + (local - bq);
-            Pb[pp] = int16_t(p < h ? p : p - h);
-            Qb[pq] = int16_t(q < h ? q : q - h);
-            pmap_of(d)[pp] = local;
-            pmap_of(d)[A.k + pq] = local;
-        }
-        __syncthreads();
-        int16_t *t = Pa;
-        Pa = Pb;
-        Pb = t;
-        t = Qa;
-        Qa = Qb;
-        Qb = t;
-    }
-
-    // leaves: every node of the deepest level has size 1 (product = identity)
-    for (int i = threadIdx.x; i < S; i += THREADS) ResB[i] = 0;
-    __syncthreads();
-
-    for (int d = depth - 1; d >= 0; --d) {
-        // glue: children at level d+1 into parents at level d
-        for (int i = threadIdx.x; i < S; i += THREADS) {
-            int po, ps, co, cs;
-            N.at(i, d, po, ps);
-            if (ps <= 1) {
-                ResA[i] = 0;
-                continue;
+            __syncthreads();
+            const int from = lane == 0 ? warp - 1 : warp + 1;
+            if ((lane == 0 || lane == 31) && from >= 0 && from < warps) {
+                const uint2 *in = reinterpret_cast<const uint2 *>(edge[buf][from][lane == 0]);
+#pragma unroll
+                for (int e = 0; e < NODE_E; e += 2) {
+                    const uint2 w = in[e / 2];
+                    x[e] = w.x;
+                    x[e + 1] = w.y;
+                }
             }
-            N.at(i, d + 1, co, cs);
-            const int prow = pmap_of(d)[i];
-            const int pcol = pmap_of(d)[A.k + co + ResB[i]];
-            const int hi = co != po ? INT_MIN : 0;
-            CW[po + prow] = pcol | hi;
-            RW[po + pcol] = prow | hi;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < S; i += THREADS) {
-            int po, ps;
-            N.at(i, d, po, ps);
-            if (ps > 1) ResA[i] = int16_t(CW[i] & INT_MAX);
-        }
-        __syncthreads();
-        // walks: the first levels (nodes of at least SUB_SEG_MIN entries, at
-        // most SUB_SEG_NODES of them) one node after the other, each cut into
-        // segments walked side by side; below, one thread per node (threads
-        // of a warp walking different nodes side by side)
-        const int nodes = 1 << d;
-        if (nodes <= SUB_SEG_NODES && (S >> d) >= SUB_SEG_MIN) {
-            for (int nd = 0; nd < nodes; ++nd) {
-                int po, ps;
-                N.nth(nd, d, po, ps);
-                if (ps > 1) sub_walk_segmented<THREADS>(CW, RW, ResA, po, ps, sTh, sTl);
-            }
-        } else {
-            for (int nd = threadIdx.x; nd < nodes; nd += THREADS) {
-                int po, ps;
-                N.nth(nd, d, po, ps);
-                if (ps <= 1) continue;
-                const int32_t *cw_ = CW + po, *rw_ = RW + po;
-                int16_t *res_ = ResA + po;
-                ant_walk(ps - 1, 0, cw_[ps - 1] < 0 ? 0 : -1, ps, INT_MAX, [&](int r) { return cw_[r]; },
-                         [&](int c) { return rw_[c]; }, [&](int r, int c) { res_[r] = int16_t(c); });
-            }
-        }
-        __syncthreads();
-        int16_t *t = ResA;
-        ResA = ResB;
-        ResB = t;
-    }
-    for (int i = threadIdx.x; i < S; i += THREADS) A.res[o + i] = S > 1 ? ResB[i] : 0;
-}
-
-// A subtree launch; variants above 48 KB of shared memory opt in once per device.
-template <int MAXN, int THREADS>
-slcs_status launch_subtree(const SubArgs &S, int blocks, cudaStream_t st)
-{
-    constexpr size_t smem = subtree_smem(MAXN);
-    if (smem > 48 * 1024) {
-        static bool attr[64] = {};
-        int dev = 0;
-        SLCS_CUDA(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 64) dev = 0;
-        if (!attr[dev]) {
-            SLCS_CUDA(cudaFuncSetAttribute(subtree_kernel<MAXN, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(smem)));
-            attr[dev] = true;
         }
     }
-    subtree_kernel<MAXN, THREADS><<<blocks, THREADS, smem, st>>>(S);
-    SLCS_CUDA(cudaGetLastError());
-    return SLCS_OK;
+    if (!ONE_WARP && (lane == 0 || lane == 31)) return;
+#pragma unroll
+    for (int e = 0; e < NODE_E; ++e)
+        if (base + e < S) A.res[o + base + e] = int32_t(0xFFFFu - (x[e] & 0xFFFFu));
 }
 
 // ---------------------------------------------------------------------------
@@ -1442,10 +1175,17 @@ __global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes
         [&](int r, int c) { A.res[o + r] = c; }, lane);
 }
 
-// Levels with short segments (B <= WALK_LANE_B) have many segments: one
-// lane per segment, all steps straight from global memory (L2), so that a
-// warp advances 32 walks at once instead of one.
+// Many short segments (B <= WALK_LANE_B, more of them than the device keeps
+// WALK_WARPS warps per SM for): one lane per segment, all steps straight from
+// global memory (L2), so that a warp advances 32 walks at once instead of one.
+// While every segment's warp is resident the warp's staged walk wins, since a
+// lane waits for L2 at most steps.  Whole products, MEASURED lanes -> warps
+// (combed strands / random permutations): k = 32768 334 -> 285 / 333 -> 312 us,
+// 131072 555 -> 476 / 555 -> 535, 524288 932 -> 853 / 1097 -> 1109 with the
+// levels of at most 10000 segments on warps; with all of its levels on warps
+// 905 / 1288.
 constexpr int WALK_LANE_B = 256;
+constexpr int WALK_WARPS = 64;
 
 __global__ void __launch_bounds__(256) walk_lanes_kernel(SegArgs A, int nodes)
 {
@@ -1763,31 +1503,24 @@ static size_t table_ints(int k, int cutoff)
 slcs_status braid_workspace_bytes(int p, int q, int k, int cutoff, size_t *bytes)
 {
     const int n = std::max(p, q);
-    const int levels = braid_levels(k);
     const size_t kk = size_t(std::max(k, 1));
-    if (cutoff <= 0) cutoff = 1024;
-    if (cutoff > SUB_MAX) cutoff = SUB_MAX;
+    if (cutoff <= 0) cutoff = NODE_MAX;
+    if (cutoff > NODE_MAX) cutoff = NODE_MAX;
+    const int lc = cutoff_level(k, cutoff);
     size_t b = 0;
     b += 4 * table_ints(k, cutoff) * sizeof(int32_t) + 512; // delta tables (hi, lo), two buffers
     b += 4 * kk * sizeof(int32_t);                         // P/Q ping-pong
-    b += 2 * kk * size_t(levels + 2) * sizeof(int32_t);    // maps per level
-    b += kk * size_t(levels + 2) * sizeof(int32_t);        // results per level
+    b += 2 * kk * size_t(lc + 2) * sizeof(int32_t);    // maps per level
+    b += kk * size_t(lc + 2) * sizeof(int32_t);        // results per level
     b += 2 * kk * sizeof(int32_t);                         // row and column words
     b += 2 * size_t(std::max(n, k)) * sizeof(int32_t);     // scans
     b += 2 * (size_t(std::max(n, k)) / SCAN_BS + 2) * sizeof(int32_t);
     b += size_t(p) * sizeof(int32_t) + size_t(q) * sizeof(int32_t); // inverses
     b += 2 * kk * sizeof(int32_t);                         // map_row, map_col
     b += 64 * 256 + 256;                                    // alignment slack, flag
-    b += size_t(levels + 1) * ((size_t(std::max(k, 1)) + 256 * PART_PER - 1) / (256 * PART_PER)) * 16 + 512; // partition tiles
+    b += size_t(lc + 1) * ((size_t(std::max(k, 1)) + 256 * PART_PER - 1) / (256 * PART_PER)) * 16 + 512; // partition tiles
     *bytes = b;
     return SLCS_OK;
-}
-
-int braid_levels(int k)
-{
-    int depth = 0;
-    for (int s = k; s > 1; s = s - (s >> 1)) ++depth;
-    return depth;
 }
 
 slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k, bool row_glue, int32_t *out,
@@ -1798,10 +1531,10 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
         SLCS_CUDA(cudaGetLastError());
         return SLCS_OK;
     }
-    if (cutoff <= 0) cutoff = 1024;
-    if (cutoff > SUB_MAX) cutoff = SUB_MAX;
+    if (cutoff <= 0) cutoff = NODE_MAX;
+    if (cutoff > NODE_MAX) cutoff = NODE_MAX;
     const int n = std::max(p, q);
-    const int levels = braid_levels(k);
+    const int lc = cutoff_level(k, cutoff); // first level whose nodes fit a block
     const size_t kk = size_t(k);
     char *cur = static_cast<char *>(ws);
     auto take = [&](size_t bytes) {
@@ -1810,8 +1543,8 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
         return r;
     };
     int32_t *PQ = reinterpret_cast<int32_t *>(take(4 * kk * 4));
-    int32_t *maps = reinterpret_cast<int32_t *>(take(2 * kk * size_t(levels + 2) * 4));
-    int32_t *res = reinterpret_cast<int32_t *>(take(kk * size_t(levels + 2) * 4));
+    int32_t *maps = reinterpret_cast<int32_t *>(take(2 * kk * size_t(lc + 2) * 4));
+    int32_t *res = reinterpret_cast<int32_t *>(take(kk * size_t(lc + 2) * 4));
     int32_t *C = reinterpret_cast<int32_t *>(take(kk * 4));
     int32_t *Rr = reinterpret_cast<int32_t *>(take(kk * 4));
     const size_t nscan = size_t(std::max(n, k));
@@ -1827,7 +1560,6 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
     // Error flag, then the partitions' tile words (one per tile and level),
     // their done flags, the ticket and the levels' done counts: zeroed by one
     // memset.
-    const int lc = cutoff_level(k, cutoff); // first level whose nodes fit a block
     const int part_bs = part_threads(k) * PART_PER;
     const int kb = int((kk + part_bs - 1) / part_bs);
     const size_t tile_words = size_t(lc) * size_t(kb);
@@ -1885,12 +1617,10 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
     {
         int smax = k; // largest node of level lc (floor/ceil halving)
         for (int l = 0; l < lc; ++l) smax = smax - (smax >> 1);
-        SubArgs S{Pcur, Qcur, res + kk * size_t(lc), maps, k, lc, bad};
-        slcs_status ss;
-        if (smax <= 256) ss = launch_subtree<256, 128>(S, 1 << lc, st);
-        else if (smax <= 1024) ss = launch_subtree<1024, 256>(S, 1 << lc, st);
-        else ss = launch_subtree<SUB_MAX, SUB_THREADS>(S, 1 << lc, st);
-        if (ss != SLCS_OK) return ss;
+        const NodeArgs N{Pcur, Qcur, res + kk * size_t(lc), k, lc, bad};
+        const int warps = node_warps(smax);
+        if (warps == 1) node_kernel<true><<<1 << lc, 32, 0, st>>>(N);
+        else node_kernel<false><<<1 << lc, warps * 32, 0, st>>>(N);
     }
     // Levels above: glue, union, walk.
     for (int l = lc - 1; l >= 0; --l) {
@@ -1924,7 +1654,7 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
         const int nseg = 2 * ((smax + B - 1) / B) + 2;
         SegArgs SA{C, Rr, tab_hi, res + kk * size_t(l), k, l, B, stride, nseg, bad};
         const long warps = long(nodes) * nseg;
-        if (B <= WALK_LANE_B) {
+        if (B <= WALK_LANE_B && warps > long(WALK_WARPS) * sm_count()) {
             walk_lanes_kernel<<<int((warps + 255) / 256), 256, 0, st>>>(SA, nodes);
         } else {
             const size_t wsm = size_t(4) * 2 * walk_win(B) * sizeof(int32_t);

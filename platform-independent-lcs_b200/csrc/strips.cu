@@ -251,7 +251,7 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         scr_off[size_t(t)] = scr_elems;
         scr_elems += relay ? relay_row_elems(d.m, d.n, *relay) : scratch_elems(d.m, d.n, tm);
     }
-    const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 1024;
+    const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 0;
     // Products glue strips with overlap = band height and bands with overlap
     // n; no side exceeds m + n.
     size_t braid_bytes = 0;
