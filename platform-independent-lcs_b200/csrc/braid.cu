@@ -63,6 +63,28 @@ __host__ __device__ __forceinline__ void node_of(int i, int level, int k, int &o
     }
 }
 
+// Node of level lc, left to right, that holds value v (or place v).
+__device__ __forceinline__ int leaf_of(int v, int lc, int k)
+{
+    int o = 0, s = k, nd = 0;
+    for (int d = 0; d < lc; ++d) {
+        const int h = s >> 1;
+        const bool right = v >= o + h;
+        nd = nd * 2 + right;
+        o += right ? h : 0;
+        s = right ? s - h : h;
+    }
+    return nd;
+}
+
+// Products whose level lc has at most FAN_LEAVES nodes partition every level
+// in one pass (fan_kernel), in tiles of FAN_TILE entries.
+constexpr int FAN_LEAVES = 128;
+constexpr int FAN_TILE = 1024;
+__host__ __device__ constexpr int fan_tiles(int k) { return (k + FAN_TILE - 1) / FAN_TILE; }
+// Up to this many slice blocks add their predecessors' counts themselves.
+constexpr int SLICE_DIRECT = 1024;
+
 // ---------------------------------------------------------------------------
 // device-wide exclusive scan of two flag sets (partition of P rows and Q cols)
 // ---------------------------------------------------------------------------
@@ -1300,9 +1322,11 @@ struct SliceArgs {
     int32_t *p_red;  // level-0 P (r2c, local)
     int32_t *q_red;  // level-0 Q (c2r, local)
     int32_t *map_row, *map_col;
-    int32_t *scanP, *scanQ, *bsumP, *bsumQ;
+    int32_t *bsumP, *bsumQ;
     int n; // max(p, q)
     int32_t *bad;
+    int32_t *fan_cnt; // counts for fan_kernel (null: not used), of lc levels
+    int lc;
 };
 
 __device__ __forceinline__ void slice_flags(const SliceArgs &A, int i, int &fp, int &fq)
@@ -1314,24 +1338,30 @@ __device__ __forceinline__ void slice_flags(const SliceArgs &A, int i, int &fp, 
 __global__ void __launch_bounds__(256) slice_count_kernel(SliceArgs A)
 {
     if (*A.bad) return;
-    const int base = blockIdx.x * SCAN_BS;
+    constexpr int PER = SCAN_BS / 256;
+    const int base = blockIdx.x * SCAN_BS + threadIdx.x;
     int cp = 0, cq = 0;
-    for (int i = base + threadIdx.x; i < min(base + SCAN_BS, A.n); i += blockDim.x) {
-        // Column i of P (row i of Q) must be the image of the row its
-        // inverse names: otherwise no entry hit it and the input repeats one.
-        if (i < A.p) {
-            const int r = A.P_c2r[i];
-            if (unsigned(r) >= unsigned(A.p) || A.P_r2c[r] != i) *A.bad = 1;
-        }
-        if (i < A.q) {
-            const int c = A.Q_c2r[i];
-            if (unsigned(c) >= unsigned(A.q) || A.Q_r2c[c] != i) *A.bad = 1;
-        }
+    bool wrong = false;
+    int rp[PER], rq[PER]; // all reads of a kind in flight at once
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = base + j * 256;
+        rp[j] = i < A.p ? A.P_c2r[i] : 0;
+        rq[j] = i < A.q ? A.Q_c2r[i] : 0;
+    }
+    // Column i of P (row i of Q) must be the image of the row its
+    // inverse names: otherwise no entry hit it and the input repeats one.
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int i = base + j * 256;
+        if (i < A.p) wrong |= unsigned(rp[j]) >= unsigned(A.p) || A.P_r2c[rp[j]] != i;
+        if (i < A.q) wrong |= unsigned(rq[j]) >= unsigned(A.q) || A.Q_r2c[rq[j]] != i;
         int fp, fq;
         slice_flags(A, i, fp, fq);
         cp += fp;
         cq += fq;
     }
+    if (wrong) *A.bad = 1;
     __shared__ int sp[8], sq[8];
     for (int off = 16; off; off >>= 1) {
         cp += __shfl_xor_sync(FULL_MASK, cp, off);
@@ -1375,13 +1405,34 @@ __global__ void __launch_bounds__(256) slice_write_kernel(SliceArgs A)
             xq += yq;
         }
     }
-    __shared__ int wp[8], wq[8];
+    __shared__ int wp[8], wq[8], before[2];
     if ((threadIdx.x & 31) == 31) {
         wp[threadIdx.x >> 5] = xp;
         wq[threadIdx.x >> 5] = xq;
     }
-    __syncthreads();
-    int op = A.bsumP[blockIdx.x], oq = A.bsumQ[blockIdx.x];
+    int op, oq;
+    if (gridDim.x <= SLICE_DIRECT) { // the block adds its predecessors' counts itself
+        int bp = 0, bq = 0;
+        for (unsigned t = threadIdx.x; t < blockIdx.x; t += 256) {
+            bp += A.bsumP[t];
+            bq += A.bsumQ[t];
+        }
+        if (threadIdx.x < 2) before[threadIdx.x] = 0;
+        __syncthreads();
+        bp = __reduce_add_sync(FULL_MASK, bp);
+        bq = __reduce_add_sync(FULL_MASK, bq);
+        if ((threadIdx.x & 31) == 0 && (bp | bq)) {
+            atomicAdd(before, bp);
+            atomicAdd(before + 1, bq);
+        }
+        __syncthreads();
+        op = before[0];
+        oq = before[1];
+    } else {
+        __syncthreads();
+        op = A.bsumP[blockIdx.x];
+        oq = A.bsumQ[blockIdx.x];
+    }
     for (int w = 0; w < (threadIdx.x >> 5); ++w) {
         op += wp[w];
         oq += wq[w];
@@ -1393,15 +1444,112 @@ __global__ void __launch_bounds__(256) slice_write_kernel(SliceArgs A)
         const int i = base + j;
         if (fp[j]) {
             A.map_row[op] = i;
-            A.p_red[op] = A.P_r2c[i] - A.c0;
+            const int v = A.P_r2c[i] - A.c0;
+            A.p_red[op] = v;
+            if (A.fan_cnt) atomicAdd(A.fan_cnt + ((op / FAN_TILE) << A.lc) + leaf_of(v, A.lc, A.k), 1);
             ++op;
         }
         if (fq[j]) {
             A.map_col[oq] = i;
-            A.q_red[oq] = A.Q_c2r[i] - A.r0;
+            const int v = A.Q_c2r[i] - A.r0;
+            A.q_red[oq] = v;
+            if (A.fan_cnt)
+                atomicAdd(A.fan_cnt + ((fan_tiles(A.k) + oq / FAN_TILE) << A.lc) + leaf_of(v, A.lc, A.k), 1);
             ++oq;
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// every level's partition at once
+//
+// An entry's place at level l is its node's start plus the number of earlier
+// entries in the same node, and its node follows from its value alone (nodes
+// are the same ranges of values as of places).  So no level needs the one
+// above: slice_write counts the entries of every (tile, node of level lc);
+// here a block of one tile adds the earlier tiles' counts and its own warps'
+// into prefix sums over the nodes of level lc, of which the count of any
+// level's node before a warp is a difference of two, and __match_any_sync
+// ranks a warp's entries within their node, level by level.  No block waits
+// for another.  At an overlap of 32768 (5 levels) the level-by-level
+// partitions took 59 us, waiting for one another; this takes 6 (MEASURED).
+// The tables grow with the tiles times the nodes, so products of more than
+// FAN_LEAVES nodes keep the level-by-level form.
+// ---------------------------------------------------------------------------
+struct FanArgs {
+    const int32_t *in; // level 0: P then Q (k entries each)
+    int32_t *out;      // level lc, node-local: P then Q
+    int32_t *maps;     // level l at maps + 2 k l: P's map, then Q's (levels 1 to lc)
+    const int32_t *cnt; // (P or Q, tile, node of level lc)
+    int k, lc;
+    const int32_t *bad;
+};
+
+__global__ void __launch_bounds__(FAN_TILE) fan_kernel(FanArgs A)
+{
+    if (*A.bad) return;
+    __shared__ int sums[FAN_TILE / 32][FAN_LEAVES + 1]; // per warp: entries before it, by node, then prefix sums
+    __shared__ int before[FAN_LEAVES];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int side = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
+    const int nl = 1 << A.lc;
+    const int i = tile * FAN_TILE + threadIdx.x;
+    const bool here = i < A.k;
+    const int v = here ? A.in[size_t(side) * A.k + i] : 0;
+    const int leaf = here ? leaf_of(v, A.lc, A.k) : -1;
+    for (int t = lane; t <= nl; t += 32) sums[warp][t] = 0;
+    if (threadIdx.x < nl) before[threadIdx.x] = 0;
+    __syncthreads();
+    {
+        const unsigned same = __match_any_sync(FULL_MASK, leaf);
+        if (here && lane == __ffs(same) - 1) sums[warp][leaf] = __popc(same);
+        const int32_t *cnt = A.cnt + ((size_t(side) * tiles) << A.lc);
+        int sum = 0;
+        for (int t = threadIdx.x >> A.lc; t < tile; t += FAN_TILE >> A.lc)
+            sum += cnt[(size_t(t) << A.lc) + (threadIdx.x & (nl - 1))];
+        if (sum) atomicAdd(before + (threadIdx.x & (nl - 1)), sum);
+    }
+    __syncthreads();
+    if (threadIdx.x < nl) {
+        int run = before[threadIdx.x];
+        for (int w = 0; w < FAN_TILE / 32; ++w) {
+            const int c = sums[w][threadIdx.x];
+            sums[w][threadIdx.x] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+    for (int base = 0, carry = 0; base <= nl; base += 32) { // exclusive prefix sums of the warp's row
+        const int t = base + lane, c = t < nl ? sums[warp][t] : 0;
+        int x = c;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(FULL_MASK, x, off);
+            if (lane >= off) x += y;
+        }
+        if (t <= nl) sums[warp][t] = carry + x - c;
+        carry += __shfl_sync(FULL_MASK, x, 31);
+    }
+    __syncwarp();
+    int o = 0, s = A.k, local = i; // the entry's node of level l and its place there
+    for (int l = 1; l <= A.lc; ++l) {
+        const int h = s >> 1;
+        if (v < o + h) {
+            s = h;
+        } else {
+            o += h;
+            s -= h;
+        }
+        const int nd = leaf >> (A.lc - l);
+        const unsigned same = __match_any_sync(FULL_MASK, nd);
+        if (here) {
+            const int first = nd << (A.lc - l);
+            const int place = sums[warp][first + (1 << (A.lc - l))] - sums[warp][first] +
+                              __popc(same & ((1u << lane) - 1));
+            A.maps[size_t(2) * A.k * l + size_t(side) * A.k + o + place] = local;
+            local = place;
+        }
+    }
+    if (here) A.out[size_t(side) * A.k + o + local] = v - o;
 }
 
 struct AssembleArgs {
@@ -1518,6 +1666,7 @@ slcs_status braid_workspace_bytes(int p, int q, int k, int cutoff, size_t *bytes
     b += size_t(p) * sizeof(int32_t) + size_t(q) * sizeof(int32_t); // inverses
     b += 2 * kk * sizeof(int32_t);                         // map_row, map_col
     b += 64 * 256 + 256;                                    // alignment slack, flag
+    b += size_t(2 * fan_tiles(std::min(k, FAN_LEAVES * NODE_MAX))) * FAN_LEAVES * sizeof(int32_t); // the fan's counts
     b += size_t(lc + 1) * ((size_t(std::max(k, 1)) + 256 * PART_PER - 1) / (256 * PART_PER)) * 16 + 512; // partition tiles
     *bytes = b;
     return SLCS_OK;
@@ -1562,8 +1711,10 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
     // memset.
     const int part_bs = part_threads(k) * PART_PER;
     const int kb = int((kk + part_bs - 1) / part_bs);
-    const size_t tile_words = size_t(lc) * size_t(kb);
-    const size_t sync_bytes = 256 + tile_words * 8 + tile_words * 4 + 256 + tile_words * 4;
+    const bool fan = lc > 0 && lc < 31 && (1 << lc) <= FAN_LEAVES;
+    const size_t tile_words = fan ? 0 : size_t(lc) * size_t(kb);
+    const size_t fan_words = fan ? size_t(2 * fan_tiles(k)) << lc : 0;
+    const size_t sync_bytes = 256 + tile_words * 8 + tile_words * 4 + 256 + tile_words * 4 + fan_words * 4;
     char *sync_area = take(sync_bytes);
     int32_t *bad = reinterpret_cast<int32_t *>(sync_area);
     unsigned long long *tiles = reinterpret_cast<unsigned long long *>(sync_area + 256);
@@ -1571,6 +1722,7 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
     int32_t *ticket = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12);
     int32_t *level_done = ticket + 1; // lc counts (lc <= 31 fits these 256 bytes)
     int32_t *scat = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12 + 256);
+    int32_t *fan_cnt = scat + tile_words; // the fan's counts in place of the tiles' words
     const size_t tints = table_ints(k, cutoff);
     // Two table buffers, each a level's hi then lo counts; levels alternate.
     int32_t *tabs = reinterpret_cast<int32_t *>(take(4 * tints * 4));
@@ -1594,14 +1746,20 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
     int32_t *Pcur = PQ, *Qcur = PQ + kk;
     {
         SliceArgs S{P, Q_c2r, P_c2r, Q, p, q, k, row_glue ? 0 : p - k, row_glue ? q - k : 0, Pcur, Qcur, map_row,
-                    map_col, scanP, scanQ, bsP, bsQ, n, bad};
+                    map_col, bsP, bsQ, n, bad, fan ? fan_cnt : nullptr, lc};
         slice_count_kernel<<<nbs, 256, 0, st>>>(S);
-        part_bsum_kernel<<<1, 1024, 0, st>>>(bsP, bsQ, nbs);
+        if (nbs > SLICE_DIRECT) part_bsum_kernel<<<1, 1024, 0, st>>>(bsP, bsQ, nbs);
         slice_write_kernel<<<nbs, 256, 0, st>>>(S);
     }
     // Levels above the cutoff: device-wide partitions, all in one launch
-    // (level l reads the even or odd pair of PQ's arrays and writes the other).
-    if (lc > 0) {
+    // (level by level, level l reads the even or odd pair of PQ's arrays and
+    // writes the other).
+    if (fan) {
+        const FanArgs G{PQ, PQ + 2 * kk, maps, fan_cnt, k, lc, bad};
+        fan_kernel<<<dim3(unsigned(fan_tiles(k)), 2), FAN_TILE, 0, st>>>(G);
+        Pcur = PQ + 2 * kk;
+        Qcur = PQ + 3 * kk;
+    } else if (lc > 0) {
         PartAllArgs G{PQ, maps, scanP, scanQ, k, lc, kb, (k & (k - 1)) == 0, tiles, done, ticket, level_done, scat,
                       bad, device_status_word()};
         const int threads = part_threads(k);
