@@ -654,6 +654,51 @@ __device__ __forceinline__ void ant_walk_warp(int dr, int dc, int delta, int s, 
     }
 }
 
+// The walk's rows side by side: on its way up the walk leaves row r at
+// c*(r), the first column with delta(r, c) = 0, whatever way it came, so a
+// segment's rows need not wait for one another.  Lane t of a group takes row
+// dr - t: delta(dr - t, dc) is the start's minus the increments of the rows
+// between (a warp scan), and c* is where the increments of the columns from dc
+// on have made up for it (counted from shared memory, every lane reading the
+// same column).  Rows and columns beyond the segment's last diagonal belong to
+// later segments, so the counts form a triangle of B^2 / 2.  A fresh point can
+// only lie at (r, c* - 1).  Needs -1 <= delta <= 0 and, unless dc is 0,
+// delta(dr, dc - 1) < 0, as on every start of a segment; col holds last + 1 -
+// (dc - dr) entries.
+template <typename RowW, typename ColW, typename Put>
+__device__ __forceinline__ void walk_rows(int dr, int dc, int delta, int last, int s, RowW rw, ColW cw, Put put,
+                                          int2 *col, int lane)
+{
+    const int most = last - (dc - dr); // row dr - t looks at columns dc to dc + most - t
+    if (most < 0) return;
+    for (int j = lane; j < most; j += 32) {
+        const int w = dc + j < s ? cw(dc + j) : 0;
+        col[j] = make_int2(w & INT_MAX, w < 0 ? 0 : -1);
+    }
+    __syncwarp();
+    int carry = -delta;
+    for (int t0 = 0; t0 <= min(most, dr); t0 += 32) {
+        const int t = t0 + lane, r = dr - t;
+        const int w = r >= 0 ? rw(r) : 0;
+        int need = t > 0 && r >= 0 ? word_inc(w, dc) : 0;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(FULL_MASK, need, off);
+            if (lane >= off) need += y;
+        }
+        need += carry;
+        carry = __shfl_sync(FULL_MASK, need, 31);
+        int c = dc;
+        const int cols = most - t0;
+#pragma unroll 8
+        for (int j = 0; j < cols; ++j) {
+            const int2 p = col[j];
+            c += need > 0;
+            need += ((p.x - r) ^ p.y) >> 31; // hi: row above r; lo: row r or below
+        }
+        if (r >= 0 && need <= 0 && c - r <= last && c > 0 && word_inc(w, c)) put(r, c - 1);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // nodes at or below the cutoff
 // ---------------------------------------------------------------------------
@@ -1063,6 +1108,8 @@ __device__ __forceinline__ int colinc(const SegArgs &A, int o, int c, int r)
 // level (dynamic shared memory, so that levels with short segments keep many
 // warps resident).
 constexpr int WALK_WIN = 1040;
+constexpr int WALK_LANE_B = 256;
+constexpr int WALK_ROW_B = 128; // segments up to this long walk their rows side by side
 __host__ __device__ inline int walk_win(int B) { return B + 12 < WALK_WIN ? B + 12 : WALK_WIN; }
 
 __global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes)
@@ -1157,6 +1204,13 @@ __global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes
         delta = dstart - rowinc(A, o, dr, dc);
     }
     (void)G;
+    if (B <= WALK_ROW_B) {
+        int2 *col = reinterpret_cast<int2 *>(walk_smem) + size_t(threadIdx.x >> 5) * B;
+        walk_rows(
+            dr, dc, delta, E + B, s, [&](int r) { return __ldg(A.CW + o + r); },
+            [&](int c) { return __ldg(A.RW + o + c); }, [&](int r, int c) { A.res[o + r] = c; }, col, lane);
+        return;
+    }
     // The segment walks at most B + 1 steps, each one row up or one column
     // right: rows [dr - B - 6, dr] and columns [dc - 1, dc + B + 5] cover
     // them.  The warp stages them (coalesced), then walks in shared memory.
@@ -1206,7 +1260,6 @@ __global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes
 // 131072 555 -> 476 / 555 -> 535, 524288 932 -> 853 / 1097 -> 1109 with the
 // levels of at most 10000 segments on warps; with all of its levels on warps
 // 905 / 1288.
-constexpr int WALK_LANE_B = 256;
 constexpr int WALK_WARPS = 64;
 
 __global__ void __launch_bounds__(256) walk_lanes_kernel(SegArgs A, int nodes)
@@ -1815,7 +1868,7 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
         if (B <= WALK_LANE_B && warps > long(WALK_WARPS) * sm_count()) {
             walk_lanes_kernel<<<int((warps + 255) / 256), 256, 0, st>>>(SA, nodes);
         } else {
-            const size_t wsm = size_t(4) * 2 * walk_win(B) * sizeof(int32_t);
+            const size_t wsm = size_t(4) * 2 * (B <= WALK_ROW_B ? B : walk_win(B)) * sizeof(int32_t);
             walk_segments_kernel<<<int((warps * 32 + 127) / 128), 128, wsm, st>>>(SA, nodes);
         }
     }
