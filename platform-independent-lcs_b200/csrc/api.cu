@@ -1968,7 +1968,8 @@ slcs_status slcs_braid_multiply(const int32_t *p_r2c, int32_t p_size, const int3
     braid_workspace_bytes(p_size, q_size, k, cutoff, &bytes);
     void *ws = nullptr;
     SLCS_CUDA(cudaMallocAsync(&ws, bytes, st));
-    slcs_status s = launch_braid(p_r2c, p_size, q_r2c, q_size, k, row_glue != 0, out_r2c, cutoff, ws, bytes, st);
+    const BraidJob job{p_r2c, p_size, q_r2c, q_size, out_r2c};
+    slcs_status s = launch_braids(&job, 1, k, row_glue != 0, cutoff, ws, bytes, st);
     SLCS_CUDA(cudaFreeAsync(ws, st));
     return s;
 }

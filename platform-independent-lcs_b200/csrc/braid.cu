@@ -48,6 +48,15 @@ constexpr int PART_PER = 8;     // entries per thread of a partition tile
 // a short look-back chain) for large products, 256 (2048 entries) below.
 constexpr int PART_BIG_K = 1 << 19;
 __host__ __device__ constexpr int part_threads(int k) { return k >= PART_BIG_K ? 1024 : 256; }
+
+// One launch of a kernel works on up to N products side by side (product z of
+// grid dimension z): the arguments of each.
+template <typename Args, int N>
+struct Many {
+    static_assert(N * sizeof(Args) <= 4000, "kernel arguments are limited to 4 KB");
+    Args of[N];
+};
+
 __host__ __device__ __forceinline__ void node_of(int i, int level, int k, int &o, int &s)
 {
     o = 0;
@@ -102,8 +111,13 @@ struct LevelArgs {
 
 
 // Exclusive scan of the block sums (one block; the count is k / SCAN_BS).
-__global__ void __launch_bounds__(1024) part_bsum_kernel(int32_t *bp, int32_t *bq, int nb)
+struct BsumArgs {
+    int32_t *bp, *bq;
+};
+template <int N>
+__global__ void __launch_bounds__(1024) part_bsum_kernel(const __grid_constant__ Many<BsumArgs, N> M, int nb)
 {
+    int32_t *bp = M.of[blockIdx.z].bp, *bq = M.of[blockIdx.z].bq;
     __shared__ int wp[32], wq[32];
     __shared__ int carry_p, carry_q;
     if (threadIdx.x == 0) carry_p = carry_q = 0;
@@ -440,9 +454,10 @@ __device__ __forceinline__ bool part_tile(const FusedArgs &F, int tile, bool loc
     return true;
 }
 
-template <int PART_THREADS>
-__global__ void __launch_bounds__(PART_THREADS) part_levels_kernel(PartAllArgs G)
+template <int PART_THREADS, int N>
+__global__ void __launch_bounds__(PART_THREADS) part_levels_kernel(const __grid_constant__ Many<PartAllArgs, N> M)
 {
+    const PartAllArgs &G = M.of[blockIdx.z];
     constexpr int PART_BS = PART_THREADS * PART_PER;
     __shared__ PartSmem<PART_THREADS> S;
     __shared__ int s_ticket;
@@ -750,9 +765,11 @@ constexpr int NODE_MAX = 1200;
 constexpr int NODE_WARPS = (NODE_MAX + NODE_OWN - 1) / NODE_OWN;
 inline int node_warps(int smax) { return smax <= 32 * NODE_E ? 1 : (smax + NODE_OWN - 1) / NODE_OWN; }
 
-template <bool ONE_WARP>
-__global__ void __launch_bounds__(ONE_WARP ? 32 : NODE_WARPS * 32) node_kernel(NodeArgs A)
+template <bool ONE_WARP, int N>
+__global__ void __launch_bounds__(ONE_WARP ? 32 : NODE_WARPS * 32)
+    node_kernel(const __grid_constant__ Many<NodeArgs, N> M)
 {
+    const NodeArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     __shared__ uint16_t half[2 * (ONE_WARP ? 32 * NODE_E : NODE_MAX)]; // entry j: column half, row half
     __shared__ __align__(8) uint32_t edge[ONE_WARP ? 1 : 2][ONE_WARP ? 1 : NODE_WARPS][2][NODE_E];
@@ -846,8 +863,10 @@ struct GlueArgs {
     long long nclear;
 };
 
-__global__ void __launch_bounds__(256) glue_kernel(GlueArgs A)
+template <int N>
+__global__ void __launch_bounds__(256) glue_kernel(const __grid_constant__ Many<GlueArgs, N> M)
 {
+    const GlueArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < A.nclear;
          i += (long long)gridDim.x * blockDim.x)
@@ -937,8 +956,10 @@ __device__ __forceinline__ void node_by_index(int nd, int level, int k, int &o, 
 // inclusive suffix of the lo counts along the row, 32 columns per step, the
 // two scans side by side (hi from the left, lo from the right) with the next
 // step's words read before this step's scan.
-__global__ void __launch_bounds__(256) table_rows_kernel(TableArgs A, int nodes)
+template <int N>
+__global__ void __launch_bounds__(256) table_rows_kernel(const __grid_constant__ Many<TableArgs, N> M, int nodes)
 {
+    const TableArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     const int lane = threadIdx.x & 31;
     const long wid = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -984,9 +1005,10 @@ __global__ void __launch_bounds__(256) table_rows_kernel(TableArgs A, int nodes)
 // of at most TCOL_SMALL_ROWS rows) 32 columns x 8 chunks.
 constexpr int TCOL_PER = (WALK_GMAX + 1 + 63) / 64; // rows of a chunk, at most
 constexpr int TCOL_SMALL_ROWS = 8 * TCOL_PER;
-template <int COLS, int CHUNKS>
-__global__ void __launch_bounds__(COLS * CHUNKS) table_cols_kernel(TableArgs A, int nodes)
+template <int COLS, int CHUNKS, int N>
+__global__ void __launch_bounds__(COLS * CHUNKS) table_cols_kernel(const __grid_constant__ Many<TableArgs, N> M, int nodes)
 {
+    const TableArgs &A = M.of[blockIdx.z];
     constexpr int TCOL_COLS = COLS, TCOL_CHUNKS = CHUNKS;
     if (*A.bad) return;
     const int colblocks = (A.stride + TCOL_COLS - 1) / TCOL_COLS;
@@ -1037,8 +1059,10 @@ __global__ void __launch_bounds__(COLS * CHUNKS) table_cols_kernel(TableArgs A, 
 // finishes the whole table in shared memory (row pass, then column pass):
 // delta(iB, jB) = #{hi blocks above-left} - #{lo blocks at or below-right}.
 constexpr int SMALL_TABLE = 4096;
-__global__ void __launch_bounds__(256) table_small_kernel(TableArgs A, int nodes)
+template <int N>
+__global__ void __launch_bounds__(256) table_small_kernel(const __grid_constant__ Many<TableArgs, N> M, int nodes)
 {
+    const TableArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     __shared__ int32_t hs[SMALL_TABLE], ls[SMALL_TABLE];
     const int nd = blockIdx.x;
@@ -1112,8 +1136,10 @@ constexpr int WALK_LANE_B = 256;
 constexpr int WALK_ROW_B = 128; // segments up to this long walk their rows side by side
 __host__ __device__ inline int walk_win(int B) { return B + 12 < WALK_WIN ? B + 12 : WALK_WIN; }
 
-__global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes)
+template <int N>
+__global__ void __launch_bounds__(128) walk_segments_kernel(const __grid_constant__ Many<SegArgs, N> M, int nodes)
 {
+    const SegArgs &A = M.of[blockIdx.z];
     extern __shared__ int32_t walk_smem[];
     if (*A.bad) return;
     const int lane = threadIdx.x & 31;
@@ -1262,8 +1288,10 @@ __global__ void __launch_bounds__(128) walk_segments_kernel(SegArgs A, int nodes
 // 905 / 1288.
 constexpr int WALK_WARPS = 64;
 
-__global__ void __launch_bounds__(256) walk_lanes_kernel(SegArgs A, int nodes)
+template <int N>
+__global__ void __launch_bounds__(256) walk_lanes_kernel(const __grid_constant__ Many<SegArgs, N> M, int nodes)
 {
+    const SegArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     const long gid = long(blockIdx.x) * blockDim.x + threadIdx.x;
     if (gid >= long(nodes) * A.nseg) return;
@@ -1352,9 +1380,21 @@ __global__ void __launch_bounds__(256) walk_lanes_kernel(SegArgs A, int nodes)
 // launch; an entry outside [0, n) raises *bad.  A column that no entry hits
 // keeps whatever Pc / Qc held: slice_count_kernel detects it (a repeat in
 // the input leaves some column unhit).
-__global__ void inverse_pair_kernel(const int32_t *P, int32_t *Pc, int p, const int32_t *Q, int32_t *Qc, int q,
-                                    int32_t *bad)
+struct InverseArgs {
+    const int32_t *P;
+    int32_t *Pc;
+    const int32_t *Q;
+    int32_t *Qc;
+    int p, q;
+    int32_t *bad;
+};
+template <int N>
+__global__ void __launch_bounds__(256) inverse_pair_kernel(const __grid_constant__ Many<InverseArgs, N> M)
 {
+    const InverseArgs &A = M.of[blockIdx.z];
+    const int32_t *P = A.P, *Q = A.Q;
+    int32_t *Pc = A.Pc, *Qc = A.Qc, *bad = A.bad;
+    const int p = A.p, q = A.q;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < p + q; t += gridDim.x * blockDim.x) {
         const bool in_p = t < p;
         const int i = in_p ? t : t - p, n = in_p ? p : q;
@@ -1388,8 +1428,10 @@ __device__ __forceinline__ void slice_flags(const SliceArgs &A, int i, int &fp, 
     fq = i < A.q && A.Q_c2r[i] >= A.r0 && A.Q_c2r[i] < A.r0 + A.k;
 }
 
-__global__ void __launch_bounds__(256) slice_count_kernel(SliceArgs A)
+template <int N>
+__global__ void __launch_bounds__(256) slice_count_kernel(const __grid_constant__ Many<SliceArgs, N> M)
 {
+    const SliceArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     constexpr int PER = SCAN_BS / 256;
     const int base = blockIdx.x * SCAN_BS + threadIdx.x;
@@ -1436,8 +1478,10 @@ __global__ void __launch_bounds__(256) slice_count_kernel(SliceArgs A)
     }
 }
 
-__global__ void __launch_bounds__(256) slice_write_kernel(SliceArgs A)
+template <int N>
+__global__ void __launch_bounds__(256) slice_write_kernel(const __grid_constant__ Many<SliceArgs, N> M)
 {
+    const SliceArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     constexpr int PER = SCAN_BS / 256;
     const int base = blockIdx.x * SCAN_BS + threadIdx.x * PER;
@@ -1538,8 +1582,10 @@ struct FanArgs {
     const int32_t *bad;
 };
 
-__global__ void __launch_bounds__(FAN_TILE) fan_kernel(FanArgs A)
+template <int N>
+__global__ void __launch_bounds__(FAN_TILE) fan_kernel(const __grid_constant__ Many<FanArgs, N> M)
 {
+    const FanArgs &A = M.of[blockIdx.z];
     if (*A.bad) return;
     __shared__ int sums[FAN_TILE / 32][FAN_LEAVES + 1]; // per warp: entries before it, by node, then prefix sums
     __shared__ int before[FAN_LEAVES];
@@ -1616,8 +1662,10 @@ struct AssembleArgs {
     uint32_t *status;   // device status word: DEV_ERR_INPUT when the product failed
 };
 
-__global__ void __launch_bounds__(256) assemble_kernel(AssembleArgs A)
+template <int N>
+__global__ void __launch_bounds__(256) assemble_kernel(const __grid_constant__ Many<AssembleArgs, N> M)
 {
+    const AssembleArgs &A = M.of[blockIdx.z];
     if (*A.bad) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(A.status, DEV_ERR_INPUT);
         return;
@@ -1721,21 +1769,25 @@ slcs_status braid_workspace_bytes(int p, int q, int k, int cutoff, size_t *bytes
     b += 64 * 256 + 256;                                    // alignment slack, flag
     b += size_t(2 * fan_tiles(std::min(k, FAN_LEAVES * NODE_MAX))) * FAN_LEAVES * sizeof(int32_t); // the fan's counts
     b += size_t(lc + 1) * ((size_t(std::max(k, 1)) + 256 * PART_PER - 1) / (256 * PART_PER)) * 16 + 512; // partition tiles
-    *bytes = b;
+    *bytes = (b + 255) / 256 * 256;
     return SLCS_OK;
 }
 
-slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k, bool row_glue, int32_t *out,
-                         int cutoff, void *ws, size_t ws_bytes, cudaStream_t st)
+namespace {
+
+// Products jobs[0..count) of one overlap k >= 1, each with ws_bytes of
+// workspace one after another: every step of them in one launch.
+template <int N>
+slcs_status launch_many(const BraidJob *jobs, int count, int k, bool row_glue, int cutoff, void *ws, size_t ws_bytes,
+                        cudaStream_t st)
 {
-    if (k == 0) {
-        direct_sum_kernel<<<blocks_for(p + q, 256), 256, 0, st>>>(P, Q, p, q, row_glue, out);
-        SLCS_CUDA(cudaGetLastError());
-        return SLCS_OK;
+    if (cutoff <= 0 || cutoff > NODE_MAX) cutoff = NODE_MAX;
+    int pmax = 0, qmax = 0; // one layout for all: of the largest sizes
+    for (int z = 0; z < count; ++z) {
+        pmax = std::max(pmax, jobs[z].p);
+        qmax = std::max(qmax, jobs[z].q);
     }
-    if (cutoff <= 0) cutoff = NODE_MAX;
-    if (cutoff > NODE_MAX) cutoff = NODE_MAX;
-    const int n = std::max(p, q);
+    const int n = std::max(pmax, qmax);
     const int lc = cutoff_level(k, cutoff); // first level whose nodes fit a block
     const size_t kk = size_t(k);
     char *cur = static_cast<char *>(ws);
@@ -1744,138 +1796,190 @@ slcs_status launch_braid(const int32_t *P, int p, const int32_t *Q, int q, int k
         cur += (bytes + 255) / 256 * 256;
         return r;
     };
-    int32_t *PQ = reinterpret_cast<int32_t *>(take(4 * kk * 4));
-    int32_t *maps = reinterpret_cast<int32_t *>(take(2 * kk * size_t(lc + 2) * 4));
-    int32_t *res = reinterpret_cast<int32_t *>(take(kk * size_t(lc + 2) * 4));
-    int32_t *C = reinterpret_cast<int32_t *>(take(kk * 4));
-    int32_t *Rr = reinterpret_cast<int32_t *>(take(kk * 4));
+    auto take_ints = [&](size_t n) { return reinterpret_cast<int32_t *>(take(n * sizeof(int32_t))); };
+    // The first product's arrays; another's lie a multiple of ws_bytes further.
+    int32_t *PQ0 = take_ints(4 * kk);
+    int32_t *maps0 = take_ints(2 * kk * size_t(lc + 2));
+    int32_t *res0 = take_ints(kk * size_t(lc + 2));
+    int32_t *C0 = take_ints(kk), *Rr0 = take_ints(kk);
     const size_t nscan = size_t(std::max(n, k));
-    int32_t *scanP = reinterpret_cast<int32_t *>(take(nscan * 4));
-    int32_t *scanQ = reinterpret_cast<int32_t *>(take(nscan * 4));
+    int32_t *scanP0 = take_ints(nscan), *scanQ0 = take_ints(nscan);
     const int nbs = int((nscan + SCAN_BS - 1) / SCAN_BS);
-    int32_t *bsP = reinterpret_cast<int32_t *>(take(size_t(nbs + 1) * 4));
-    int32_t *bsQ = reinterpret_cast<int32_t *>(take(size_t(nbs + 1) * 4));
-    int32_t *P_c2r = reinterpret_cast<int32_t *>(take(size_t(p) * 4));
-    int32_t *Q_c2r = reinterpret_cast<int32_t *>(take(size_t(q) * 4));
-    int32_t *map_row = reinterpret_cast<int32_t *>(take(kk * 4));
-    int32_t *map_col = reinterpret_cast<int32_t *>(take(kk * 4));
+    int32_t *bsP0 = take_ints(size_t(nbs + 1)), *bsQ0 = take_ints(size_t(nbs + 1));
+    int32_t *P_c2r0 = take_ints(size_t(pmax)), *Q_c2r0 = take_ints(size_t(qmax));
+    int32_t *map_row0 = take_ints(kk), *map_col0 = take_ints(kk);
     // Error flag, then the partitions' tile words (one per tile and level),
-    // their done flags, the ticket and the levels' done counts: zeroed by one
-    // memset.
+    // their done flags, the ticket and the levels' done counts, or the fan's
+    // counts: zeroed by one memset.
     const int part_bs = part_threads(k) * PART_PER;
     const int kb = int((kk + part_bs - 1) / part_bs);
     const bool fan = lc > 0 && lc < 31 && (1 << lc) <= FAN_LEAVES;
     const size_t tile_words = fan ? 0 : size_t(lc) * size_t(kb);
     const size_t fan_words = fan ? size_t(2 * fan_tiles(k)) << lc : 0;
     const size_t sync_bytes = 256 + tile_words * 8 + tile_words * 4 + 256 + tile_words * 4 + fan_words * 4;
-    char *sync_area = take(sync_bytes);
-    int32_t *bad = reinterpret_cast<int32_t *>(sync_area);
-    unsigned long long *tiles = reinterpret_cast<unsigned long long *>(sync_area + 256);
-    int32_t *done = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 8);
-    int32_t *ticket = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12);
-    int32_t *level_done = ticket + 1; // lc counts (lc <= 31 fits these 256 bytes)
-    int32_t *scat = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12 + 256);
-    int32_t *fan_cnt = scat + tile_words; // the fan's counts in place of the tiles' words
+    char *sync0 = take(sync_bytes);
     const size_t tints = table_ints(k, cutoff);
     // Two table buffers, each a level's hi then lo counts; levels alternate.
-    int32_t *tabs = reinterpret_cast<int32_t *>(take(4 * tints * 4));
+    int32_t *tabs0 = take_ints(4 * tints);
     if (size_t(cur - static_cast<char *>(ws)) > ws_bytes) return fail(SLCS_ERR_ALLOC, "braid workspace too small");
 
+    const unsigned nz = unsigned(count);
+    auto at = [&](auto *p, int z) { return reinterpret_cast<decltype(p)>(reinterpret_cast<char *>(p) + ws_bytes * size_t(z)); };
+    auto bad_of = [&](int z) { return reinterpret_cast<int32_t *>(at(sync0, z)); };
     // Level l's tables: entries of each of the two, and place in the buffer
     // of its parity.
     auto level_tables = [&](int l, size_t *tentries) {
         int B, stride;
         walk_grid(k, l, B, stride);
         *tentries = (size_t(1) << l) * size_t(stride) * size_t(stride);
-        return tabs + size_t(l & 1) * 2 * tints;
+        return tabs0 + size_t(l & 1) * 2 * tints;
     };
-    SLCS_CUDA(cudaMemsetAsync(sync_area, 0, sync_bytes, st));
+    auto zero = [&](void *p, size_t bytes) {
+        if (count > 1 && ws_bytes < (size_t(1) << 30)) // within the pitch limit
+            return cudaMemset2DAsync(p, ws_bytes, 0, bytes, size_t(count), st);
+        cudaError_t e = cudaSuccess;
+        for (int z = 0; z < count && e == cudaSuccess; ++z)
+            e = cudaMemsetAsync(static_cast<char *>(p) + ws_bytes * size_t(z), 0, bytes, st);
+        return e;
+    };
+    SLCS_CUDA(zero(sync0, sync_bytes));
     if (lc > 0) { // the deepest level's tables; each level's glue clears the next level's
         size_t te = 0;
         int32_t *t0 = level_tables(lc - 1, &te);
-        SLCS_CUDA(cudaMemsetAsync(t0, 0, 2 * te * sizeof(int32_t), st));
+        SLCS_CUDA(zero(t0, 2 * te * sizeof(int32_t)));
     }
-    inverse_pair_kernel<<<blocks_for(long(p) + q, 256), 256, 0, st>>>(P, P_c2r, p, Q, Q_c2r, q, bad);
-    int32_t *Pcur = PQ, *Qcur = PQ + kk;
     {
-        SliceArgs S{P, Q_c2r, P_c2r, Q, p, q, k, row_glue ? 0 : p - k, row_glue ? q - k : 0, Pcur, Qcur, map_row,
-                    map_col, bsP, bsQ, n, bad, fan ? fan_cnt : nullptr, lc};
-        slice_count_kernel<<<nbs, 256, 0, st>>>(S);
-        if (nbs > SLICE_DIRECT) part_bsum_kernel<<<1, 1024, 0, st>>>(bsP, bsQ, nbs);
-        slice_write_kernel<<<nbs, 256, 0, st>>>(S);
+        Many<InverseArgs, N> I{};
+        Many<SliceArgs, N> S{};
+        Many<BsumArgs, N> U{};
+        for (int z = 0; z < count; ++z) {
+            const BraidJob &j = jobs[z];
+            int32_t *P_c2r = at(P_c2r0, z), *Q_c2r = at(Q_c2r0, z), *PQ = at(PQ0, z);
+            I.of[z] = InverseArgs{j.P, P_c2r, j.Q, Q_c2r, j.p, j.q, bad_of(z)};
+            int32_t *fan_cnt = reinterpret_cast<int32_t *>(at(sync0, z) + 512);
+            S.of[z] = SliceArgs{j.P, Q_c2r, P_c2r, j.Q, j.p, j.q, k, row_glue ? 0 : j.p - k, row_glue ? j.q - k : 0,
+                                PQ, PQ + kk, at(map_row0, z), at(map_col0, z), at(bsP0, z), at(bsQ0, z),
+                                std::max(j.p, j.q), bad_of(z), fan ? fan_cnt : nullptr, lc};
+            U.of[z] = BsumArgs{at(bsP0, z), at(bsQ0, z)};
+        }
+        inverse_pair_kernel<N><<<dim3(unsigned(blocks_for(long(pmax) + qmax, 256)), 1, nz), 256, 0, st>>>(I);
+        slice_count_kernel<N><<<dim3(unsigned(nbs), 1, nz), 256, 0, st>>>(S);
+        if (nbs > SLICE_DIRECT) part_bsum_kernel<N><<<dim3(1, 1, nz), 1024, 0, st>>>(U, nbs);
+        slice_write_kernel<N><<<dim3(unsigned(nbs), 1, nz), 256, 0, st>>>(S);
     }
     // Levels above the cutoff: device-wide partitions, all in one launch
     // (level by level, level l reads the even or odd pair of PQ's arrays and
     // writes the other).
+    int32_t *cur0 = PQ0; // P then Q of level lc
     if (fan) {
-        const FanArgs G{PQ, PQ + 2 * kk, maps, fan_cnt, k, lc, bad};
-        fan_kernel<<<dim3(unsigned(fan_tiles(k)), 2), FAN_TILE, 0, st>>>(G);
-        Pcur = PQ + 2 * kk;
-        Qcur = PQ + 3 * kk;
+        Many<FanArgs, N> G{};
+        for (int z = 0; z < count; ++z) {
+            int32_t *PQ = at(PQ0, z);
+            G.of[z] = FanArgs{PQ, PQ + 2 * kk, at(maps0, z), reinterpret_cast<int32_t *>(at(sync0, z) + 512), k, lc,
+                              bad_of(z)};
+        }
+        fan_kernel<N><<<dim3(unsigned(fan_tiles(k)), 2, nz), FAN_TILE, 0, st>>>(G);
+        cur0 = PQ0 + 2 * kk;
     } else if (lc > 0) {
-        PartAllArgs G{PQ, maps, scanP, scanQ, k, lc, kb, (k & (k - 1)) == 0, tiles, done, ticket, level_done, scat,
-                      bad, device_status_word()};
+        Many<PartAllArgs, N> G{};
+        for (int z = 0; z < count; ++z) {
+            char *sync_area = at(sync0, z);
+            int32_t *ticket = reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12);
+            G.of[z] = PartAllArgs{at(PQ0, z), at(maps0, z), at(scanP0, z), at(scanQ0, z), k, lc, kb,
+                                  (k & (k - 1)) == 0, reinterpret_cast<unsigned long long *>(sync_area + 256),
+                                  reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 8), ticket,
+                                  ticket + 1, // lc counts (lc <= 31 fits these 256 bytes)
+                                  reinterpret_cast<int32_t *>(sync_area + 256 + tile_words * 12 + 256), bad_of(z),
+                                  device_status_word()};
+        }
         const int threads = part_threads(k);
         const long grid = std::min<long>(long(lc) * kb, long(sm_count()) * (2048 / threads));
-        if (threads == 1024) part_levels_kernel<1024><<<int(grid), 1024, 0, st>>>(G);
-        else part_levels_kernel<256><<<int(grid), 256, 0, st>>>(G);
-        if (lc & 1) {
-            Pcur = PQ + 2 * kk;
-            Qcur = PQ + 3 * kk;
-        }
+        if (threads == 1024) part_levels_kernel<1024, N><<<dim3(unsigned(grid), 1, nz), 1024, 0, st>>>(G);
+        else part_levels_kernel<256, N><<<dim3(unsigned(grid), 1, nz), 256, 0, st>>>(G);
+        if (lc & 1) cur0 = PQ0 + 2 * kk;
     }
-    // Nodes of level lc: one block each, down to the leaves and back.
+    // Nodes of level lc: one block each.
     {
         int smax = k; // largest node of level lc (floor/ceil halving)
         for (int l = 0; l < lc; ++l) smax = smax - (smax >> 1);
-        const NodeArgs N{Pcur, Qcur, res + kk * size_t(lc), k, lc, bad};
+        Many<NodeArgs, N> G{};
+        for (int z = 0; z < count; ++z)
+            G.of[z] = NodeArgs{at(cur0, z), at(cur0, z) + kk, at(res0, z) + kk * size_t(lc), k, lc, bad_of(z)};
         const int warps = node_warps(smax);
-        if (warps == 1) node_kernel<true><<<1 << lc, 32, 0, st>>>(N);
-        else node_kernel<false><<<1 << lc, warps * 32, 0, st>>>(N);
+        const dim3 grid(1u << lc, 1, nz);
+        if (warps == 1) node_kernel<true, N><<<grid, 32, 0, st>>>(G);
+        else node_kernel<false, N><<<grid, warps * 32, 0, st>>>(G);
     }
     // Levels above: glue, union, walk.
     for (int l = lc - 1; l >= 0; --l) {
         int B, stride;
         walk_grid(k, l, B, stride);
         const int nodes = 1 << l;
+        int smax = k;
+        for (int d = 0; d < l; ++d) smax = smax - (smax >> 1);
+        const int nseg = 2 * ((smax + B - 1) / B) + 2;
         // hi and lo counts of the level side by side (zeroed by the memset
         // above or by the glue one level down), filled by the glue as it
         // places the points
         size_t tentries = 0, next_entries = 0;
-        int32_t *tab_hi = level_tables(l, &tentries);
-        int32_t *lvl_lo = tab_hi + tentries;
-        int32_t *next = l > 0 ? level_tables(l - 1, &next_entries) : nullptr;
-        GlueArgs G{res + kk * size_t(l + 1), maps + 2 * kk * size_t(l + 1), maps + 2 * kk * size_t(l + 1) + kk,
-                   C, Rr, res + kk * size_t(l), k, l, bad, tab_hi, lvl_lo, B, stride, next,
-                   (long long)(2 * next_entries)};
-        glue_kernel<<<blocks_for(k, 256), 256, 0, st>>>(G);
-        TableArgs TA{C, tab_hi, lvl_lo, k, l, B, stride, bad};
+        int32_t *tab0 = level_tables(l, &tentries);
+        int32_t *next0 = l > 0 ? level_tables(l - 1, &next_entries) : nullptr;
+        Many<GlueArgs, N> G{};
+        Many<TableArgs, N> TA{};
+        Many<SegArgs, N> SA{};
+        for (int z = 0; z < count; ++z) {
+            int32_t *C = at(C0, z), *Rr = at(Rr0, z), *tab = at(tab0, z), *lo = tab + tentries;
+            int32_t *maps = at(maps0, z) + 2 * kk * size_t(l + 1), *res = at(res0, z) + kk * size_t(l);
+            G.of[z] = GlueArgs{res + kk, maps, maps + kk, C, Rr, res, k, l, bad_of(z), tab, lo, B, stride,
+                               next0 ? at(next0, z) : nullptr, (long long)(2 * next_entries)};
+            TA.of[z] = TableArgs{C, tab, lo, k, l, B, stride, bad_of(z)};
+            SA.of[z] = SegArgs{C, Rr, tab, res, k, l, B, stride, nseg, bad_of(z)};
+        }
+        glue_kernel<N><<<dim3(unsigned(blocks_for(k, 256)), 1, nz), 256, 0, st>>>(G);
         if (size_t(stride) * stride <= size_t(SMALL_TABLE)) {
-            table_small_kernel<<<nodes, 256, 0, st>>>(TA, nodes);
+            table_small_kernel<N><<<dim3(unsigned(nodes), 1, nz), 256, 0, st>>>(TA, nodes);
         } else {
             const int rows = nodes * stride;
-            table_rows_kernel<<<int((long(rows) * 32 + 255) / 256), 256, 0, st>>>(TA, nodes);
+            table_rows_kernel<N><<<dim3(unsigned((long(rows) * 32 + 255) / 256), 1, nz), 256, 0, st>>>(TA, nodes);
             if (stride <= TCOL_SMALL_ROWS)
-                table_cols_kernel<32, 8><<<nodes * ((stride + 31) / 32), 256, 0, st>>>(TA, nodes);
+                table_cols_kernel<32, 8, N><<<dim3(unsigned(nodes * ((stride + 31) / 32)), 1, nz), 256, 0, st>>>(TA, nodes);
             else
-                table_cols_kernel<4, 64><<<nodes * ((stride + 3) / 4), 256, 0, st>>>(TA, nodes);
+                table_cols_kernel<4, 64, N><<<dim3(unsigned(nodes * ((stride + 3) / 4)), 1, nz), 256, 0, st>>>(TA, nodes);
         }
-        int smax = k;
-        for (int d = 0; d < l; ++d) smax = smax - (smax >> 1);
-        const int nseg = 2 * ((smax + B - 1) / B) + 2;
-        SegArgs SA{C, Rr, tab_hi, res + kk * size_t(l), k, l, B, stride, nseg, bad};
         const long warps = long(nodes) * nseg;
-        if (B <= WALK_LANE_B && warps > long(WALK_WARPS) * sm_count()) {
-            walk_lanes_kernel<<<int((warps + 255) / 256), 256, 0, st>>>(SA, nodes);
+        if (B <= WALK_LANE_B && warps * count > long(WALK_WARPS) * sm_count()) {
+            walk_lanes_kernel<N><<<dim3(unsigned((warps + 255) / 256), 1, nz), 256, 0, st>>>(SA, nodes);
         } else {
             const size_t wsm = size_t(4) * 2 * (B <= WALK_ROW_B ? B : walk_win(B)) * sizeof(int32_t);
-            walk_segments_kernel<<<int((warps * 32 + 127) / 128), 128, wsm, st>>>(SA, nodes);
+            walk_segments_kernel<N><<<dim3(unsigned((warps * 32 + 127) / 128), 1, nz), 128, wsm, st>>>(SA, nodes);
         }
     }
-    AssembleArgs A{P, P_c2r, Q, res, map_row, map_col, out, p, q, k, row_glue, bad, device_status_word()};
-    assemble_kernel<<<blocks_for(long(p) + q + k, 256), 256, 0, st>>>(A);
+    Many<AssembleArgs, N> A{};
+    for (int z = 0; z < count; ++z) {
+        const BraidJob &j = jobs[z];
+        A.of[z] = AssembleArgs{j.P, at(P_c2r0, z), j.Q, at(res0, z), at(map_row0, z), at(map_col0, z), j.out, j.p, j.q,
+                               k, row_glue, bad_of(z), device_status_word()};
+    }
+    assemble_kernel<N><<<dim3(unsigned(blocks_for(long(pmax) + qmax + k, 256)), 1, nz), 256, 0, st>>>(A);
     SLCS_CUDA(cudaGetLastError());
     return SLCS_OK;
+}
+
+} // namespace
+
+slcs_status launch_braids(const BraidJob *jobs, int count, int k, bool row_glue, int cutoff, void *ws, size_t ws_bytes,
+                          cudaStream_t st)
+{
+    if (k == 0) {
+        for (int z = 0; z < count; ++z) {
+            const BraidJob &j = jobs[z];
+            direct_sum_kernel<<<blocks_for(j.p + j.q, 256), 256, 0, st>>>(j.P, j.Q, j.p, j.q, row_glue, j.out);
+        }
+        SLCS_CUDA(cudaGetLastError());
+        return SLCS_OK;
+    }
+    if (count == 1) return launch_many<1>(jobs, 1, k, row_glue, cutoff, ws, ws_bytes, st);
+    return launch_many<BRAID_MANY>(jobs, count, k, row_glue, cutoff, ws, ws_bytes, st);
 }
 
 } // namespace slcs

@@ -36,6 +36,7 @@
 //     a masked row has a symbol nothing matches and h = -1 (never swaps), a
 //     masked column likewise and v = INT_MAX (never swaps), so edge tiles need
 //     no host fixup.
+#include <algorithm>
 #include <climits>
 #include <mutex>
 #include <type_traits>
@@ -594,6 +595,18 @@ __global__ void strands_to_perm_kernel(const int32_t *__restrict__ h, int32_t m,
     }
 }
 
+// The same for every pair of a batch (grid dimension y), each at its
+// out_off in both arrays: row -> col only.
+__global__ void batch_to_perm_kernel(const PairDev *__restrict__ pairs, const int32_t *__restrict__ strands, int32_t *r2c)
+{
+    const PairDev d = pairs[blockIdx.y];
+    const int32_t size = d.m + d.n;
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < size; i += gridDim.x * blockDim.x) {
+        const int32_t id = strands[d.out_off + i];
+        if (id >= 0 && id < size) r2c[d.out_off + id] = i < d.m ? d.n + i : i - d.m;
+    }
+}
+
 // Balanced launch: when every stripe can be resident at once, each SM gets
 // one block of ceil(stripes / SMs) warps, so no SM hosts more stripes than
 // another by more than one.  (With several blocks per SM, tickets went to
@@ -786,6 +799,20 @@ slcs_status launch_strands_to_perm(const int32_t *h, int32_t m, const int32_t *v
     int blocks = int((size + 255) / 256);
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     strands_to_perm_kernel<<<blocks, 256, 0, stream>>>(h, m, v, n, r2c, c2r);
+    SLCS_CUDA(cudaGetLastError());
+    return SLCS_OK;
+}
+
+slcs_status launch_batch_to_perm(const PairDev *pairs, int32_t npairs, int64_t total, const int32_t *strands,
+                                 int32_t *r2c, cudaStream_t st)
+{
+    const int64_t each = std::max<int64_t>(1, total / npairs / 1024);
+    constexpr int32_t MOST = 65535; // grid dimension y
+    for (int32_t p0 = 0; p0 < npairs; p0 += MOST) {
+        const int32_t np = std::min(MOST, npairs - p0);
+        const dim3 grid(unsigned(std::min<int64_t>(each, std::max(1, 2368 / np))), unsigned(np));
+        batch_to_perm_kernel<<<grid, 256, 0, st>>>(pairs + p0, strands, r2c);
+    }
     SLCS_CUDA(cudaGetLastError());
     return SLCS_OK;
 }

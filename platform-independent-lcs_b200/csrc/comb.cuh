@@ -118,4 +118,9 @@ slcs_status launch_batch_hash(const PairDev *pairs, int32_t npairs, const int32_
 slcs_status launch_strands_to_perm(const int32_t *h, int32_t m, const int32_t *v, int32_t n,
                                    int32_t *row_to_col, int32_t *col_to_row, cudaStream_t stream);
 
+// Strands of every pair (device descriptors, `total` strands in all) -> its
+// row -> col array at the same place of r2c.
+slcs_status launch_batch_to_perm(const PairDev *pairs, int32_t npairs, int64_t total, const int32_t *strands,
+                                 int32_t *r2c, cudaStream_t st);
+
 } // namespace slcs

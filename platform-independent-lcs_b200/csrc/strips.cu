@@ -18,6 +18,7 @@
 // at once; strips multiply the chains of a short pair, so that they fill the
 // GPU.  Column strips are also the per-GPU unit of the multi-GPU split.
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -46,11 +47,11 @@ __global__ void perm_to_strands_kernel(const int32_t *__restrict__ r2c, int32_t 
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Products of one tree level are independent: they run side by side on a
-// small pool of streams per device (created once, never destroyed), each
-// with its own braid workspace, forked from and joined back to the caller's
-// stream with events.
-constexpr int MAX_SIDE = 8;
+// Batches of products of one tree level (bands of unequal heights, more
+// products than a batch takes) run side by side on a small pool of streams per
+// device (created once, never destroyed), each with its own braid workspace,
+// forked from and joined back to the caller's stream with events.
+constexpr int MAX_SIDE = 4;
 std::mutex g_side_mu;
 std::vector<cudaStream_t> g_side[64];
 
@@ -70,33 +71,82 @@ slcs_status side_streams(int count, cudaStream_t *out)
     return SLCS_OK;
 }
 
+// A permutation in one of the two strand buffers.
 struct Perm {
-    int32_t *p;
-    int64_t size;
+    int64_t off, size;
 };
 
-// One level of a merge tree at a time: in every job's list, neighbours are
-// multiplied (products round robin on the side streams, each stream with its
-// own braid workspace, forked from and joined back to the caller's stream)
-// and an odd last entry is copied; each list is replaced by its products,
-// which are written one after another from `dst`.
-struct Merger {
+// One level of a merge tree: in every job's list, neighbours are multiplied
+// and an odd last entry is copied; each list is replaced by its results, laid
+// one after another in the other buffer.  Products of one overlap go into the
+// same launches, BRAID_MANY at most.
+struct Level {
     struct Job {
         std::vector<Perm> *list;
         int32_t k;     // overlap of every product of the list
         bool row_glue; // staggered_multiply<true> (bands) or <false> (strips)
     };
+    struct Batch {
+        int32_t k;
+        bool row_glue;
+        std::vector<Perm> p, q, out;
+    };
+    std::vector<Batch> batches;
+    std::vector<Perm> copy_from, copy_to;
+
+    explicit Level(std::vector<Job> &&jobs)
+    {
+        int64_t off = 0;
+        for (Job &J : jobs) {
+            std::vector<Perm> out, &lv = *J.list;
+            for (size_t i = 0; i < lv.size(); i += 2) {
+                if (i + 1 < lv.size()) {
+                    if (batches.empty() || batches.back().k != J.k || batches.back().row_glue != J.row_glue ||
+                        batches.back().p.size() >= size_t(BRAID_MANY))
+                        batches.push_back(Batch{J.k, J.row_glue, {}, {}, {}});
+                    Batch *it = &batches.back();
+                    out.push_back({off, lv[i].size + lv[i + 1].size - J.k});
+                    it->p.push_back(lv[i]);
+                    it->q.push_back(lv[i + 1]);
+                    it->out.push_back(out.back());
+                } else {
+                    out.push_back({off, lv[i].size});
+                    copy_from.push_back(lv[i]);
+                    copy_to.push_back(out.back());
+                }
+                off += out.back().size;
+            }
+            lv.swap(out);
+        }
+    }
+    // Workspace of one product of a batch.
+    static size_t product_bytes(const Batch &B, int cutoff)
+    {
+        int64_t p = 0, q = 0;
+        for (const Perm &x : B.p) p = std::max(p, x.size);
+        for (const Perm &x : B.q) q = std::max(q, x.size);
+        size_t bytes = 0;
+        braid_workspace_bytes(int(p), int(q), B.k, cutoff, &bytes);
+        return bytes;
+    }
+};
+
+// Runs the levels: a level of one batch on the caller's stream, the batches
+// of others round robin on the side streams (forked from and joined back to
+// the caller's), each stream with its own workspace.
+struct Merger {
     cudaStream_t st;
     cudaStream_t *side;
     int par;
     int cutoff;
     char *ws;
-    size_t ws_bytes;
+    size_t ws_bytes; // of one side stream
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[MAX_SIDE] = {};
 
     slcs_status create()
     {
+        if (par < 2) return SLCS_OK;
         SLCS_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
         for (int j = 0; j < par; ++j) SLCS_CUDA(cudaEventCreateWithFlags(&join[j], cudaEventDisableTiming));
         return SLCS_OK;
@@ -107,44 +157,40 @@ struct Merger {
         for (int j = 0; j < par; ++j)
             if (join[j]) cudaEventDestroy(join[j]);
     }
+    slcs_status batch(const Level::Batch &B, const int32_t *src, int32_t *dst, int slot, cudaStream_t t)
+    {
+        BraidJob jobs[BRAID_MANY];
+        const int count = int(B.p.size());
+        for (int z = 0; z < count; ++z)
+            jobs[z] = BraidJob{src + B.p[size_t(z)].off, int(B.p[size_t(z)].size), src + B.q[size_t(z)].off,
+                               int(B.q[size_t(z)].size), dst + B.out[size_t(z)].off};
+        return launch_braids(jobs, count, B.k, B.row_glue, cutoff, ws + ws_bytes * size_t(slot),
+                             Level::product_bytes(B, cutoff), t);
+    }
     // On an error the streams already forked are still joined back, so that
     // the caller's stream does not run ahead of (and free the workspace of)
     // products still in flight.
-    slcs_status level(std::vector<Job> &jobs, int32_t *dst)
+    slcs_status level(const Level &L, const int32_t *src, int32_t *dst)
     {
-        SLCS_CUDA(cudaEventRecord(fork, st));
         slcs_status s = SLCS_OK;
         auto cu = [&](cudaError_t e, const char *what) {
             if (s == SLCS_OK && e != cudaSuccess) s = cuda_fail(e, what);
         };
-        int used = 0, turn = 0;
-        int64_t off = 0;
-        for (Job &J : jobs) {
-            std::vector<Perm> &lv = *J.list;
-            std::vector<Perm> out;
-            for (size_t i = 0; i < lv.size() && s == SLCS_OK; i += 2) {
-                if (i + 1 < lv.size()) {
-                    const int j = turn++ % par;
-                    if (j >= used) {
-                        cu(cudaStreamWaitEvent(side[j], fork, 0), "fork wait");
-                        used = j + 1;
-                    }
-                    const int64_t size = lv[i].size + lv[i + 1].size - J.k;
-                    if (s == SLCS_OK)
-                        s = launch_braid(lv[i].p, int(lv[i].size), lv[i + 1].p, int(lv[i + 1].size), J.k,
-                                         J.row_glue, dst + off, cutoff, ws + ws_bytes * size_t(j), ws_bytes, side[j]);
-                    out.push_back({dst + off, size});
-                    off += size;
-                } else {
-                    cu(cudaMemcpyAsync(dst + off, lv[i].p, sizeof(int32_t) * size_t(lv[i].size),
-                                       cudaMemcpyDeviceToDevice, st),
-                       "odd part copy");
-                    out.push_back({dst + off, lv[i].size});
-                    off += lv[i].size;
-                }
+        const bool forked = L.batches.size() > 1;
+        int used = 0;
+        if (forked) cu(cudaEventRecord(fork, st), "fork");
+        for (size_t i = 0; i < L.batches.size() && s == SLCS_OK; ++i) {
+            const int j = forked ? int(i) % par : 0;
+            if (forked && j >= used) {
+                cu(cudaStreamWaitEvent(side[j], fork, 0), "fork wait");
+                used = j + 1;
             }
-            lv.swap(out);
+            if (s == SLCS_OK) s = batch(L.batches[i], src, dst, j, forked ? side[j] : st);
         }
+        for (size_t i = 0; i < L.copy_from.size(); ++i)
+            cu(cudaMemcpyAsync(dst + L.copy_to[i].off, src + L.copy_from[i].off,
+                               sizeof(int32_t) * size_t(L.copy_from[i].size), cudaMemcpyDeviceToDevice, st),
+               "odd part copy");
         for (int j = 0; j < used; ++j) {
             const cudaError_t e1 = cudaEventRecord(join[j], side[j]);
             const cudaError_t e2 = e1 == cudaSuccess ? cudaStreamWaitEvent(st, join[j], 0) : e1;
@@ -252,10 +298,31 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         scr_elems += relay ? relay_row_elems(d.m, d.n, *relay) : scratch_elems(d.m, d.n, tm);
     }
     const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 0;
-    // Products glue strips with overlap = band height and bands with overlap
-    // n; no side exceeds m + n.
-    size_t braid_bytes = 0;
-    braid_workspace_bytes(int(int64_t(m) + n), int(int64_t(m) + n), std::max(m, n), cutoff, &braid_bytes);
+    // The merge tree: strips of every band glue with overlap = band height
+    // (column glue), all bands side by side; then the bands glue with overlap
+    // n (row glue).  Each level writes into the buffer the previous one did not.
+    std::vector<Level> levels;
+    std::vector<Perm> col;
+    {
+        std::vector<std::vector<Perm>> rows(static_cast<size_t>(R));
+        for (int t = 0; t < T; ++t) {
+            const slcs_pair_desc &d = pd[size_t(t)];
+            rows[size_t(t / S)].push_back({d.out_offset, int64_t(d.m) + d.n});
+        }
+        while (rows[0].size() > 1) {
+            std::vector<Level::Job> jobs;
+            for (int r = 0; r < R; ++r) jobs.push_back({&rows[size_t(r)], hgt[size_t(r)], false});
+            levels.emplace_back(std::move(jobs));
+        }
+        for (int r = 0; r < R; ++r) col.push_back(rows[size_t(r)][0]);
+        while (col.size() > 1) levels.emplace_back(std::vector<Level::Job>{{&col, n, true}});
+    }
+    size_t braid_bytes = 0, most = 1; // workspace of a side stream; batches of a level
+    for (const Level &L : levels) {
+        most = std::max(most, L.batches.size());
+        for (const Level::Batch &B : L.batches)
+            braid_bytes = std::max(braid_bytes, Level::product_bytes(B, cutoff) * B.p.size());
+    }
     // Workspace: descriptors, tasks, scratch offsets, counters, scratch,
     // strands / permutations (two buffers of S*m+R*n), braid workspaces.
     const size_t o_pairs = 0;
@@ -270,9 +337,7 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     const size_t o_x = align256(o_scr + (relay ? 0 : scr_bytes + 16));
     const size_t o_y = align256(o_x + sizeof(int32_t) * size_t(total));
     const size_t o_braid = align256(o_y + sizeof(int32_t) * size_t(total));
-    const int most = std::max(R * (S / 2), R / 2); // products of the widest merge level
-    const int par = std::max(1, std::min(MAX_SIDE, most));
-    braid_bytes = align256(braid_bytes);
+    const int par = int(std::min(size_t(MAX_SIDE), most));
     const size_t bytes = o_braid + braid_bytes * size_t(par);
     char *ws = nullptr;
     SLCS_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&ws), bytes, st));
@@ -280,12 +345,12 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     auto cu = [&](cudaError_t e, const char *what) {
         if (s == SLCS_OK && e != cudaSuccess) s = cuda_fail(e, what);
     };
-    // Host vectors are pageable: each copy has left them when it returns.
-    cu(cudaMemcpyAsync(ws + o_pairs, pd.data(), sizeof(PairDev) * size_t(T), cudaMemcpyHostToDevice, st), "pairs");
-    cu(cudaMemcpyAsync(ws + o_tasks, tasks.data(), sizeof(int2) * tasks.size(), cudaMemcpyHostToDevice, st),
-       "tasks");
-    cu(cudaMemcpyAsync(ws + o_soff, scr_off.data(), sizeof(int64_t) * size_t(T), cudaMemcpyHostToDevice, st),
-       "scratch offsets");
+    // A pageable copy has left the vector when it returns.
+    std::vector<char> head(o_work);
+    std::memcpy(head.data() + o_pairs, pd.data(), sizeof(PairDev) * size_t(T));
+    std::memcpy(head.data() + o_tasks, tasks.data(), sizeof(int2) * tasks.size());
+    std::memcpy(head.data() + o_soff, scr_off.data(), sizeof(int64_t) * size_t(T));
+    cu(cudaMemcpyAsync(ws, head.data(), o_work, cudaMemcpyHostToDevice, st), "descriptors, tasks, scratch offsets");
     cu(cudaMemsetAsync(ws + o_work, 0, work_bytes, st), "counters");
     int32_t *X = reinterpret_cast<int32_t *>(ws + o_x);
     int32_t *Y = reinterpret_cast<int32_t *>(ws + o_y);
@@ -327,37 +392,19 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         s = launch_comb(L, tm, warps, st, nullptr);
     }
     // Strands of every tile -> its permutation (row -> col) in Y.
-    std::vector<Perm> tiles;
-    for (int t = 0; t < T && s == SLCS_OK; ++t) {
-        const slcs_pair_desc &d = pd[size_t(t)];
-        s = launch_strands_to_perm(X + d.out_offset, d.m, X + d.out_offset + d.m, d.n, Y + d.out_offset, nullptr, st);
-        tiles.push_back({Y + d.out_offset, int64_t(d.m) + d.n});
-    }
+    if (s == SLCS_OK)
+        s = launch_batch_to_perm(reinterpret_cast<const PairDev *>(ws + o_pairs), T, total, X, Y, st);
     cudaStream_t side[MAX_SIDE] = {};
-    if (s == SLCS_OK && T > 1) s = side_streams(par, side);
+    if (s == SLCS_OK && par > 1) s = side_streams(par, side);
     Merger M{st, side, par, cutoff, ws + o_braid, braid_bytes};
-    if (s == SLCS_OK && T > 1) s = M.create();
-    // Strips of every band glue with overlap = band height (column glue),
-    // all bands side by side; then the bands glue with overlap n (row glue).
-    // Each level writes into the buffer the previous one did not.
-    int32_t *dst = X;
-    std::vector<std::vector<Perm>> rows(static_cast<size_t>(R));
-    for (int r = 0; r < R; ++r) rows[size_t(r)].assign(tiles.begin() + r * S, tiles.begin() + (r + 1) * S);
-    while (s == SLCS_OK && rows[0].size() > 1) {
-        std::vector<Merger::Job> jobs;
-        for (int r = 0; r < R; ++r) jobs.push_back({&rows[size_t(r)], hgt[size_t(r)], false});
-        s = M.level(jobs, dst);
-        dst = (dst == X) ? Y : X;
-    }
-    std::vector<Perm> col;
-    for (int r = 0; r < R; ++r) col.push_back(rows[size_t(r)][0]);
-    while (s == SLCS_OK && col.size() > 1) {
-        std::vector<Merger::Job> jobs{{&col, n, true}};
-        s = M.level(jobs, dst);
-        dst = (dst == X) ? Y : X;
+    if (s == SLCS_OK) s = M.create();
+    int32_t *src = Y, *dst = X;
+    for (size_t l = 0; l < levels.size() && s == SLCS_OK; ++l) {
+        s = M.level(levels[l], src, dst);
+        std::swap(src, dst);
     }
     M.destroy();
-    if (s == SLCS_OK) s = perm_to_strands(col[0].p, m, n, h_out, v_out, st);
+    if (s == SLCS_OK) s = perm_to_strands(src + col[0].off, m, n, h_out, v_out, st);
     cudaFreeAsync(ws, st);
     return s;
 }
