@@ -192,15 +192,17 @@ constexpr double RELAY_GHZ = 1.965;     // the clock those cycles were measured 
 constexpr double RELAY_WARP_LAG = 40.0; // steps a warp starts after the warp above it
 constexpr double RELAY_HOP_LAG = 45.0;  // more steps for the hand-down to the next block
 
-// Microseconds of one braid product of overlap k inside a merge level (B200).
-double braid_us(double k)
+// Microseconds of a merge level of `count` braid products of overlap k, which
+// run in the same launches (B200): one product's time, and about 1.2 ns per
+// entry that the others add to it.
+double merge_us(double k, double count)
 {
     static const double log2k[] = {6, 8, 10, 12, 14, 16, 17, 20};
-    static const double us[] = {52, 97, 185, 266, 376, 542, 675, 1550};
+    static const double us[] = {38, 44, 60, 113, 166, 246, 334, 1206};
     const double x = std::log2(std::max(k, 64.0));
-    for (int i = 0; i < 6; ++i)
-        if (x < log2k[i + 1]) return us[i] + (us[i + 1] - us[i]) * (x - log2k[i]) / (log2k[i + 1] - log2k[i]);
-    return us[6] + (us[7] - us[6]) * (x - 17.0) / 3.0;
+    int i = 0;
+    while (i < 6 && x >= log2k[i + 1]) ++i;
+    return us[i] + (us[i + 1] - us[i]) * (x - log2k[i]) / (log2k[i + 1] - log2k[i]) + 0.0012 * k * (count - 1);
 }
 
 // The relay kernel's plan for one pair: shape, column strips and row bands
@@ -209,8 +211,7 @@ double braid_us(double k)
 // SMs combed 131072 x 131072 in 13.2 ms, 128 of (8, 4, 4) in 6.4 ms).
 // relay.tm == 0: no shape fits.  Predicted: a chain's steps (columns, then
 // the lags of its warps and blocks) at the shape's step time, and the merge
-// levels, each at least a product of its overlap and, when it holds several,
-// about 55 us of launches a product.
+// levels.
 struct RelayPlan {
     RelayShape relay{};
     int strips = 1, bands = 1;
@@ -228,8 +229,8 @@ RelayPlan plan_relay(int32_t m, int32_t n, int sms)
                 const double steps = double(n) / S / c.shape.tw + RELAY_WARP_LAG * stripes + RELAY_HOP_LAG * groups;
                 double us = 6.0 + steps * c.step / (RELAY_GHZ * 1e3);
                 if (R * S > 1) us += 20.0;
-                for (int p = S; p > 1; p /= 2) us += std::max(braid_us(double(m) / R) + 35.0, 55.0 * R * (p / 2));
-                for (int p = R; p > 1; p /= 2) us += std::max(braid_us(double(n)) + 35.0, 55.0 * (p / 2));
+                for (int p = S; p > 1; p /= 2) us += merge_us(double(m) / R, double(R) * (p / 2));
+                for (int p = R; p > 1; p /= 2) us += merge_us(double(n), p / 2);
                 if (best.relay.tm == 0 || us < best.us) best = RelayPlan{c.shape, S, R, us};
             }
     return best;
