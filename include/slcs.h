@@ -247,6 +247,7 @@ typedef struct {
      * say what a configuration naming a variant would get.                     */
     int32_t relay_groups;
     int32_t relay_all;
+    int32_t relay_duos; /* entries of two pairs a register holds (0: the relay kernel's registers hold one) */
 } slcs_plan_info;
 SLCS_API slcs_status slcs_batch_plan_info(const slcs_batch_plan *plan, slcs_plan_info *info);
 

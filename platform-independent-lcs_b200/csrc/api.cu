@@ -236,37 +236,132 @@ RelayPlan plan_relay(int32_t m, int32_t n, int sms)
     return best;
 }
 
+// The shapes with two pairs per register, and their steps.
+const RelayCost RELAY_DUO_COSTS[] = {{{2, 4, 3}, 92.0}, {{4, 4, 3}, 135.0}, {{8, 2, 3}, 160.0}, {{8, 4, 4}, 248.0}};
+
 // Instructions a combing warp of a relay shape issues per step (about; B200,
 // counted for (4, 4) and scaled by cells), the I/O warp about 12.
 double relay_issue(const RelayShape &s) { return 4.3 * s.tm * s.tw + 10.0 + 3.0 * s.tw; }
 
-// Microseconds the relay kernel takes for the pairs that `take` selects, with
-// the best shape: its longest chain plus its blocks' issue slots, spread over
-// the SMs (on B200 within a factor of 0.85 to 1.7 of sweeps from 64 reads to
-// 1,000 pairs of 9000 x 100 rows and columns).
-template <class Take>
-double batch_relay_us(const slcs_pair_desc *pairs, int32_t npairs, int sms, Take take, RelayShape *shape)
+// Pairs of a batch that the relay kernel combs: (m, n) each, or the larger m
+// and n of two pairs that share a register.
+using Sizes = std::vector<std::pair<int32_t, int32_t>>;
+
+// Longest chain (steps) and issue slots of a shape.
+struct RelayWork {
+    double chain = 0, slots = 0;
+    int64_t groups = 0;
+};
+RelayWork relay_work(const Sizes &sizes, const RelayShape &s)
+{
+    const double issue = relay_issue(s);
+    RelayWork w;
+    for (const auto &[m, n] : sizes) {
+        const int32_t stripes = (m + 32 * s.tm - 1) / (32 * s.tm);
+        const int32_t groups = (stripes + s.warps - 1) / s.warps;
+        const double own = double(n) / s.tw + 31.0; // steps of one warp
+        w.chain = std::max(w.chain, own + RELAY_WARP_LAG * stripes + RELAY_HOP_LAG * groups);
+        w.slots += stripes * own * issue + groups * (own + RELAY_WARP_LAG * (s.warps - 1)) * 12.0;
+        w.groups += groups;
+    }
+    return w;
+}
+
+// Microseconds the relay kernel takes for them, with the best shape: its
+// longest chain plus its blocks' issue slots, spread over the SMs (on B200
+// within a factor of 0.85 to 1.7 of sweeps from 64 reads to 1,000 pairs of
+// 9000 x 100 rows and columns).
+double batch_relay_us(const Sizes &sizes, int sms, RelayShape *shape)
 {
     double best = -1.0;
     for (const RelayCost &c : RELAY_COSTS) {
-        const RelayShape &s = c.shape;
-        const double issue = relay_issue(s);
-        double chain = 0, slots = 0;
-        for (int32_t p = 0; p < npairs; ++p) {
-            if (!take(p) || pairs[p].m == 0 || pairs[p].n == 0) continue;
-            const int32_t stripes = (pairs[p].m + 32 * s.tm - 1) / (32 * s.tm);
-            const int32_t groups = (stripes + s.warps - 1) / s.warps;
-            const double own = double(pairs[p].n) / s.tw + 31.0; // steps of one warp
-            chain = std::max(chain, own + RELAY_WARP_LAG * stripes + RELAY_HOP_LAG * groups);
-            slots += stripes * own * issue + groups * (own + RELAY_WARP_LAG * (s.warps - 1)) * 12.0;
-        }
-        const double us = 8.0 + 1.2 * (chain * c.step + slots / (4.0 * sms)) / (RELAY_GHZ * 1e3);
+        const RelayWork w = relay_work(sizes, c.shape);
+        const double us = 8.0 + 1.2 * (w.chain * c.step + w.slots / (4.0 * sms)) / (RELAY_GHZ * 1e3);
         if (best < 0 || us < best) {
             best = us;
-            *shape = s;
+            *shape = c.shape;
         }
     }
     return best;
+}
+
+// The same with contention by blocks: alone on its SM a block keeps its step;
+// on shared SMs each further block adds its issue to a chain's step, and with
+// many the slots count.  With two pairs per register within 0.87 to 1.12 of
+// thirteen batches (2 pairs of 600 x 8000 to 400 of 2000 x 2000), with one
+// 0.73 to 1.06.
+template <class Costs>
+double relay_shared_us(const Sizes &sizes, const Costs &costs, int sms, RelayShape *shape)
+{
+    double best = -1.0;
+    for (const RelayCost &c : costs) {
+        const RelayWork w = relay_work(sizes, c.shape);
+        const double blocks = std::ceil(double(w.groups) / sms);
+        double cycles = w.chain * c.step;
+        if (blocks > 1) {
+            const double crowded = w.chain * (c.step + 1.1 * (blocks - 1) * relay_issue(c.shape) * c.shape.warps / 4.0);
+            cycles = std::max(blocks <= 3 ? crowded : 0.0, cycles + 1.35 * w.slots / (4.0 * sms));
+        }
+        const double us = 8.0 + cycles / (RELAY_GHZ * 1e3);
+        if (best < 0 || us < best) {
+            best = us;
+            *shape = c.shape;
+        }
+    }
+    return best;
+}
+
+// How the relay kernel combs the pairs that `take` selects: one per register
+// or, when every pair's ids fit 15 bits and it is predicted faster, two,
+// neighbours in rows and then columns.  Two take half the instructions, but a
+// step of a lone chain 1.2 to 1.8 times as long: 96 pairs of up to 2900 x 3300
+// 309 -> 183 us, 30 of 9000 x 9000 1131 -> 542, 64 of 400 x 5000 112 -> 91;
+// 2 of 4000 x 4000 147 -> 194, which stay apart.
+struct BatchRelay {
+    RelayShape shape{};
+    std::vector<int2> duos; // empty: one pair per register
+    double us = 0.0;
+    int64_t groups = 0;
+};
+template <class Take>
+BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool may_two, int sms, Take take)
+{
+    BatchRelay B;
+    std::vector<int32_t> ids;
+    for (int32_t p = 0; p < npairs; ++p)
+        if (take(p) && pairs[p].m > 0 && pairs[p].n > 0) {
+            ids.push_back(p);
+            may_two = may_two && int64_t(pairs[p].m) + pairs[p].n <= PACKED16_MAX_IDS;
+        }
+    Sizes sizes;
+    for (int32_t p : ids) sizes.emplace_back(pairs[p].m, pairs[p].n);
+    B.us = batch_relay_us(sizes, sms, &B.shape);
+    if (may_two && ids.size() > 1) {
+        constexpr int32_t ROWS = 256; // pairs within so many rows are neighbours by columns
+        std::sort(ids.begin(), ids.end(), [&](int32_t x, int32_t y) {
+            const int32_t rx = pairs[x].m / ROWS, ry = pairs[y].m / ROWS;
+            return rx != ry ? rx > ry : pairs[x].n != pairs[y].n ? pairs[x].n > pairs[y].n : x < y;
+        });
+        std::vector<int2> duos;
+        Sizes both;
+        for (size_t i = 0; i < ids.size(); i += 2) {
+            const slcs_pair_desc &x = pairs[ids[i]];
+            const bool second = i + 1 < ids.size();
+            duos.push_back(make_int2(ids[i], second ? ids[i + 1] : -1));
+            both.emplace_back(second ? std::max(x.m, pairs[ids[i + 1]].m) : x.m,
+                              second ? std::max(x.n, pairs[ids[i + 1]].n) : x.n);
+        }
+        RelayShape one{}, two{};
+        const double us = relay_shared_us(both, RELAY_DUO_COSTS, sms, &two);
+        if (us < relay_shared_us(sizes, RELAY_COSTS, sms, &one)) {
+            B.us = us;
+            B.shape = two;
+            B.duos = std::move(duos);
+            sizes = std::move(both);
+        }
+    }
+    for (const auto &[m, n] : sizes) B.groups += relay_groups(m, B.shape);
+    return B;
 }
 
 // How slcs_comb_pair combs one pair: the effective configuration (algo
@@ -490,6 +585,8 @@ struct slcs_batch_plan {
     int32_t relay_sms = 0;      // SMs the couples leave to them
     int2 *d_relay = nullptr;    // (pair, group)
     int64_t *d_row_off = nullptr;
+    int2 *d_duos = nullptr;         // the relay's pairs of pairs (two per register)
+    int32_t nduos = 0;
     char *d_relay_ws = nullptr; // counters and hand-down rows, cleared by every run
     size_t relay_ws_bytes = 0;
     std::vector<slcs_pair_desc> empty_pairs; // pairs with m == 0 or n == 0
@@ -578,6 +675,8 @@ struct slcs_batch_plan {
         L.row_off = d_row_off;
         L.status = device_status_word();
         L.wait_ns = wait_ns;
+        L.two = nduos > 0;
+        L.duos = L.two ? d_duos : nullptr;
         return launch_relay(L, relay, sm_count(), st);
     }
 
@@ -1234,13 +1333,11 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     // the SMs holds all their groups.
     const int sms = sm_count();
     auto tall = [&](int32_t p) { return pairs[p].m > stream_rows; };
-    double tall_us = 0.0;
+    const bool may_two = P->stm > 0 && !(cfg && cfg->strand_bits == 32);
+    BatchRelay relay;
     if (P->stm > 0 && P->ntasks > 0) {
-        tall_us = batch_relay_us(pairs, npairs, sms, tall, &P->relay);
-        int64_t groups = 0;
-        for (int32_t p = 0; p < npairs; ++p)
-            if (tall(p) && pairs[p].n > 0) groups += relay_groups(pairs[p].m, P->relay);
-        if (groups <= sms / 4) P->relay_sms = int32_t(groups);
+        relay = plan_batch_relay(pairs, npairs, may_two, sms, tall);
+        if (relay.groups <= sms / 4) P->relay_sms = int32_t(relay.groups);
     }
     // Couples of the packed pairs and their bundles.
     std::vector<CoupleDev> couples;
@@ -1426,32 +1523,49 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
             steps += 0.33 * (pairs[p].n / double(P->tns) + 2.0);
         }
         double us = P->nstream > 0 ? (P->nstaged > 0 ? 25.0 : 10.0) + std::max(chain, steps / (4.0 * sms)) : 0.0;
-        us = P->relay_sms > 0 ? std::max(us, tall_us) : us + tall_us;
+        us = P->relay_sms > 0 ? std::max(us, relay.us) : us + relay.us;
         // (A chunk of a host run shares the GPU with the others: couples take less
         // of it.)
         const bool plain = chunk ? false : !cfg || (cfg->algo == SLCS_ALGO_AUTO && cfg->tile_m == 0 && cfg->tile_n == 0 &&
                                     cfg->warps == 0 && cfg->seg == 0 && cfg->blocks_per_sm == 0 &&
                                     cfg->strand_bits == 0 && cfg->pool_pct == 0);
-        RelayShape all{};
-        if (P->nstream == 0 || (plain && batch_relay_us(pairs, npairs, sms, [](int32_t) { return true; }, &all) < us)) {
+        BatchRelay all;
+        if (P->nstream > 0 && plain) all = plan_batch_relay(pairs, npairs, may_two, sms, [](int32_t) { return true; });
+        if (P->nstream == 0 || (plain && all.us < us)) {
             P->relay_all = P->nstream + P->ntasks > 0;
-            if (P->nstream > 0) P->relay = all;
+            if (P->nstream > 0) relay = std::move(all);
         }
     }
     if (P->relay_all || (P->stm > 0 && P->ntasks > 0)) {
-        const slcs_status rs = launch_relay(RelayLaunch{}, P->relay, sm_count(), PREPARE_ONLY);
+        P->relay = relay.shape;
+        P->nduos = int32_t(relay.duos.size());
+        RelayLaunch prepare{};
+        prepare.two = P->nduos > 0;
+        const slcs_status rs = launch_relay(prepare, P->relay, sm_count(), PREPARE_ONLY);
         if (rs != SLCS_OK) {
             delete P;
             return rs;
         }
         int64_t row_elems = 0;
-        row_off.assign(npairs, 0);
-        for (int32_t p : S.order) {
-            if (pairs[p].m == 0 || pairs[p].n == 0 || (!P->relay_all && pairs[p].m <= stream_rows)) continue;
-            const int32_t groups = relay_groups(pairs[p].m, P->relay);
-            for (int32_t g = 0; g < groups; ++g) relay_items.push_back(make_int2(p, g));
-            row_off[p] = row_elems;
-            row_elems += relay_row_elems(pairs[p].m, pairs[p].n, P->relay);
+        auto add = [&](int32_t i, int32_t m, int32_t n) { // pair or duo i
+            const int32_t groups = relay_groups(m, P->relay);
+            for (int32_t g = 0; g < groups; ++g) relay_items.push_back(make_int2(i, g));
+            row_off[size_t(i)] = row_elems;
+            row_elems += relay_row_elems(m, n, P->relay);
+        };
+        if (P->nduos > 0) { // sorted largest first
+            row_off.assign(relay.duos.size(), 0);
+            for (int32_t i = 0; i < P->nduos; ++i) {
+                const int2 d = relay.duos[size_t(i)];
+                const slcs_pair_desc &x = pairs[d.x], &y = pairs[d.y >= 0 ? d.y : d.x];
+                add(i, std::max(x.m, y.m), std::max(x.n, y.n));
+            }
+        } else {
+            row_off.assign(npairs, 0);
+            for (int32_t p : S.order) {
+                if (pairs[p].m == 0 || pairs[p].n == 0 || (!P->relay_all && pairs[p].m <= stream_rows)) continue;
+                add(p, pairs[p].m, pairs[p].n);
+            }
         }
         P->nrelay = int32_t(relay_items.size());
         P->relay_ws_bytes = 16 + sizeof(int2) * size_t(row_elems);
@@ -1480,6 +1594,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     upload(&P->d_pairs, pairs, size_t(npairs));
     upload(&P->d_relay, relay_items.data(), relay_items.size());
     upload(&P->d_row_off, row_off.data(), row_off.size());
+    upload(&P->d_duos, relay.duos.data(), size_t(P->nduos));
     upload(&P->d_seg_off, seg_off.data(), stream ? seg_off.size() : 0);
     upload(&P->d_seg_list, seg_list.data(), stream ? seg_list.size() : 0);
     upload(&P->d_pool_list, pool_list.data(), stream ? pool_list.size() : 0);
@@ -1511,6 +1626,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     rebase(P->d_pairs);
     rebase(P->d_relay);
     rebase(P->d_row_off);
+    rebase(P->d_duos);
     rebase(P->d_seg_off);
     rebase(P->d_seg_list);
     rebase(P->d_pool_list);
@@ -1604,6 +1720,7 @@ slcs_status slcs_batch_plan_info(const slcs_batch_plan *P, slcs_plan_info *info)
     info->packed_pairs = P->npacked;
     info->relay_groups = P->nrelay;
     info->relay_all = P->relay_all;
+    info->relay_duos = P->nduos;
     return SLCS_OK;
 }
 

@@ -1,21 +1,7 @@
 // couples.cu -- two pairs per register: the short pairs of a batch.
 //
-// A couple of pairs (A, B) is combed together: every symbol,
-// h and v register holds pair A in its low 16 bits and pair B in its high 16
-// bits, so one instruction works on two cells.  Strand ids are stored plus
-// one (1..32767); a masked row holds h = 0 and symbol 0x1FF, a masked column
-// v = 0x7FFF and symbol 0x100, so neither ever swaps.  The cell rule per half:
-//   x = a ^ b                    0 on a match (both below 0x200)
-//   far = fma.relu(x, -inf, 0)   on two 16-bit floats: 0 * -inf is NaN, which
-//                                relu turns into 0x7FFF; a positive x gives
-//                                -inf, which relu turns into 0
-//   h' = min(h + far, v)         unsigned halves, one VIADDMNMX
-//   v' = h + v - h'              as one 32-bit sum: the carries between the
-//                                halves cancel
-// On a match h + far is at least any v, so h' = v.  Seven integer instructions
-// (a carry-safe difference, a byte permute expanding its sign to a mask, two
-// bitwise selects) measured 5.50 cycles per warp and cell, these four 2.39
-// (one sub-partition, 4 warps of 16 rows per lane).
+// A couple of pairs (A, B) is combed together, one instruction for two cells
+// (cell16, cell.cuh).
 //
 // A warp combs a bundle: couples side by side, each on as many lanes as its
 // rows need at TM rows per lane, all started in the same step and of about the
@@ -43,26 +29,13 @@
 #include <algorithm>
 #include <climits>
 
+#include "cell.cuh"
 #include "couples.cuh"
 #include "occupancy.cuh"
 
 namespace slcs {
 
 namespace {
-
-__device__ __forceinline__ void cell16(uint32_t a, uint32_t b, uint32_t &h, uint32_t &v)
-{
-    uint32_t far;
-    asm("{\n\t.reg .b32 ninf, zero;\n\tmov.b32 ninf, 0xFF80FF80;\n\tmov.b32 zero, 0;\n\t"
-        "fma.rn.relu.bf16x2 %0, %1, ninf, zero;\n\t}"
-        : "=r"(far)
-        : "r"(a ^ b));
-    const uint32_t nh = __viaddmin_u16x2(h, far, v);
-    v = h + v - nh;
-    h = nh;
-}
-
-constexpr uint32_t MASKED_ROW16 = 0x01FF01FFu, MASKED_COLUMN16 = 0x01000100u;
 
 // Symbols c .. c + 3 of one pair as two packed words' low halves would hold
 // them: s[0..3], `mask` past n.  Whole-word loads where they are aligned.

@@ -26,6 +26,11 @@
 //     early.  Every wait is bounded as in the wavefront kernel.
 //   * Blocks take groups from a ticket counter; the group above a block's own
 //     was therefore claimed by a running block.
+//   * Batches whose ids fit 15 bits may put two pairs in a register (TWO, the
+//     packed cell rule of cell.cuh): half the instructions for batches that
+//     fill the SMs, which are bound by issue; a lone chain's step takes 1.2 to
+//     1.8 times as long.  96 pairs of up to 2900 x 3300 309 -> 183 us, 400 of
+//     2000 x 2000 538 -> 326, 30 of 9000 x 9000 1222 -> 540 (one B200).
 // What it measured on one B200, against the wavefront kernel with the same
 // cell rule: 4096 x 4096 728 -> 150 us ((TM, TW, W) = (4, 2, 3)), 20011 x 9973
 // 3.41 -> 0.51 ms, 65536 x 65536 5.2 -> 2.6 ms ((8, 2, 3), against 2 x 2
@@ -96,13 +101,43 @@ __device__ __forceinline__ void st_relaxed_pair(int2 *p, int x, int y)
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-template <int TM, int TW>
+// The cell rule in two steps, for one pair or two.
+template <bool TWO>
+__device__ __forceinline__ int match(uint32_t a, int b)
+{
+    if constexpr (TWO) return int(match16(a, uint32_t(b)));
+    else return match_far(a, uint32_t(b));
+}
+template <bool TWO>
+__device__ __forceinline__ void swap_if(int far, int &h, int &v)
+{
+    if constexpr (TWO) {
+        uint32_t x = uint32_t(h), y = uint32_t(v);
+        pass16(uint32_t(far), x, y);
+        h = int(x);
+        v = int(y);
+    } else {
+        pass(far, h, v);
+    }
+}
+template <bool TWO, int TM, int TW>
 __device__ __forceinline__ void matches(const uint32_t (&a)[TM], const int (&b)[TW], int (&far)[TM][TW])
 {
 #pragma unroll
     for (int j = 0; j < TW; ++j)
 #pragma unroll
-        for (int q = 0; q < TM; ++q) far[q][j] = match_far(a[q], uint32_t(b[j]));
+        for (int q = 0; q < TM; ++q) far[q][j] = match<TWO>(a[q], b[j]);
+}
+
+// Columns c .. c + 3 of b (n columns, `aligned` to 4 bytes).
+__device__ __forceinline__ uint32_t four_columns(const uint8_t *b, int c, int n, bool aligned)
+{
+    if (aligned && c + 4 <= n) return __ldg(reinterpret_cast<const uint32_t *>(b + c));
+    uint32_t x = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (c + j < n) x |= uint32_t(__ldg(b + c + j)) << (8 * j);
+    return x;
 }
 
 template <int TM, int TW, int W>
@@ -136,9 +171,11 @@ __device__ __forceinline__ void sync()
     asm volatile("bar.sync 1, %0;" ::"n"((W + 1) * 32) : "memory");
 }
 
-template <int TM, int TW, int W>
+template <int TM, int TW, int W, bool TWO>
 __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L)
 {
+    constexpr int NO_COLUMN = TWO ? int(MASKED_COLUMN16) : int(MASKED_COLUMN); // symbol of a masked column
+    constexpr int NO_V = TWO ? int(MASKED_V16) : INT_MAX;                      // and its strand
     using R = Relay<TM, TW, W>;
     constexpr int K = R::K, C = R::C, DI = R::DI, RING = R::RING, BRING = R::BRING, PF = R::PF, STAGES = R::STAGES;
     __shared__ __align__(16) typename R::Shared S;
@@ -154,12 +191,22 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
         }
         if (k >= L.nitems) break;
         const int2 it = L.items ? L.items[k] : make_int2(0, k);
-        const PairDev P = L.items ? L.pairs[it.x] : L.single;
-        const int m = P.m, n = P.n, group = it.y;
+        PairDev P, Q{};
+        if constexpr (TWO) {
+            const int2 d = L.duos[it.x];
+            P = L.pairs[d.x];
+            if (d.y >= 0) Q = L.pairs[d.y];
+        } else {
+            P = L.items ? L.pairs[it.x] : L.single;
+        }
+        const int m = TWO ? max(P.m, Q.m) : P.m, n = TWO ? max(P.n, Q.n) : P.n, group = it.y;
         const uint8_t *__restrict__ a = L.a_blob + P.a_off;
         const uint8_t *__restrict__ b = L.b_blob + P.b_off;
+        const uint8_t *__restrict__ a2 = L.a_blob + Q.a_off; // the second pair's
+        const uint8_t *__restrict__ b2 = L.b_blob + Q.b_off;
         int32_t *hout = L.out + P.out_off;
-        int32_t *vout = L.items ? hout + m : L.v_single;
+        int32_t *vout = L.items ? hout + P.m : L.v_single;
+        int32_t *hout2 = L.out + Q.out_off, *vout2 = hout2 + Q.m;
         int2 *row = L.rows + (L.row_off ? L.row_off[it.x] : 0);
         const int r_group = group * (32 * TM * W);
         const int last = min(W, (m - r_group + 32 * TM - 1) / (32 * TM)) - 1; // the last warp with rows
@@ -174,14 +221,20 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
             const int r0 = r_group + (w * 32 + lane) * TM;
 #pragma unroll
             for (int q = 0; q < TM; ++q) {
-                const bool in = r0 + q < m;
-                av[q] = in ? symbol_code(__ldg(a + r0 + q), 0) : MASKED_ROW;
-                hv[q] = in ? m - 1 - r0 - q : -1;
+                const int r = r0 + q;
+                if constexpr (TWO) {
+                    av[q] = (r < P.m ? uint32_t(__ldg(a + r)) : MASKED_ROW16 & 0xFFFFu) |
+                            (r < Q.m ? uint32_t(__ldg(a2 + r)) << 16 : MASKED_ROW16 & 0xFFFF0000u);
+                    hv[q] = max(P.m - r, 0) | max(Q.m - r, 0) << 16;
+                } else {
+                    av[q] = r < m ? symbol_code(__ldg(a + r), 0) : MASKED_ROW;
+                    hv[q] = r < m ? m - 1 - r : -1;
+                }
             }
 #pragma unroll
-            for (int j = 0; j < TW; ++j) vc[j] = INT_MAX;
+            for (int j = 0; j < TW; ++j) vc[j] = NO_V;
         }
-        for (int x = threadIdx.x; x < BRING * TW; x += (W + 1) * 32) (&S.codes[0][0])[x] = int(MASKED_COLUMN);
+        for (int x = threadIdx.x; x < BRING * TW; x += (W + 1) * 32) (&S.codes[0][0])[x] = NO_COLUMN;
         __syncthreads();
 
         if (w == W) {
@@ -191,16 +244,14 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
             // Symbols come a word of 4 per lane, 128 columns at a time.
             constexpr int SPAN = 128 / C;
             const bool aligned = (reinterpret_cast<uintptr_t>(b) & 3) == 0;
-            auto symbols = [&](int span) {
-                const int c = span * 128 + 4 * lane;
-                if (aligned && c + 4 <= n) return __ldg(reinterpret_cast<const uint32_t *>(b + c));
-                uint32_t x = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (c + j < n) x |= uint32_t(__ldg(b + c + j)) << (8 * j);
-                return x;
-            };
-            uint32_t word = symbols(0), word_next = symbols(1);
+            const bool aligned2 = (reinterpret_cast<uintptr_t>(b2) & 3) == 0;
+            uint32_t word = four_columns(b, 4 * lane, P.n, aligned);
+            uint32_t word_next = four_columns(b, 128 + 4 * lane, P.n, aligned);
+            uint32_t word2 = 0, word2_next = 0;
+            if constexpr (TWO) {
+                word2 = four_columns(b2, 4 * lane, Q.n, aligned2);
+                word2_next = four_columns(b2, 128 + 4 * lane, Q.n, aligned2);
+            }
             auto fetch = [&](int i) { // start the copy of the row entries of interval i
                 const int c = i * C + 2 * lane;
                 if (group && 2 * lane < C && c < n) cp_async_cg16(&S.stage[i & (STAGES - 1)][2 * lane], row + c);
@@ -220,6 +271,8 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 const int c = i * C + lane;
                 const bool in = lane < C && c < n;
                 int v = in ? m + c : INT_MAX;
+                if constexpr (TWO) // ids plus one
+                    v = (c < P.n ? P.m + c + 1 : 0x7FFF) | (c < Q.n ? Q.m + c + 1 : 0x7FFF) << 16;
                 if (group) {
                     cp_async_wait<PF - 1>();
                     __syncwarp();
@@ -233,15 +286,29 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                     if (in) v = e.x;
                 }
                 const uint32_t x = __shfl_sync(FULL_MASK, word, (i % SPAN) * (C / 4) + lane / 4);
+                uint32_t x2 = 0;
+                if constexpr (TWO) x2 = __shfl_sync(FULL_MASK, word2, (i % SPAN) * (C / 4) + lane / 4);
                 if (lane < C) {
                     const int blk = c / TW, j = c % TW;
                     S.strands[0][blk & (RING - 1)][j] = v;
-                    S.codes[blk & (BRING - 1)][j] =
-                        int(in ? symbol_code((x >> (8 * (lane & 3))) & 0xffu, 0) : MASKED_COLUMN);
+                    const uint32_t sym = (x >> (8 * (lane & 3))) & 0xffu;
+                    if constexpr (TWO) {
+                        const uint32_t sym2 = (x2 >> (8 * (lane & 3))) & 0xffu;
+                        S.codes[blk & (BRING - 1)][j] =
+                            int((c < P.n ? sym : MASKED_COLUMN16 & 0xFFFFu) |
+                                (c < Q.n ? sym2 << 16 : MASKED_COLUMN16 & 0xFFFF0000u));
+                    } else {
+                        S.codes[blk & (BRING - 1)][j] = int(in ? symbol_code(sym, 0) : MASKED_COLUMN);
+                    }
                 }
                 if (i % SPAN == SPAN - 1) {
+                    const int ahead = (i / SPAN + 2) * 128 + 4 * lane;
                     word = word_next;
-                    word_next = symbols(i / SPAN + 2);
+                    word_next = four_columns(b, ahead, P.n, aligned);
+                    if constexpr (TWO) {
+                        word2 = word2_next;
+                        word2_next = four_columns(b2, ahead, Q.n, aligned2);
+                    }
                 }
             };
             auto flush = [&](int i) { // the strands the last warp put out in interval i
@@ -250,8 +317,14 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 if (lane < C && c >= 0 && c < n) {
                     const int blk = c / TW, j = c % TW;
                     const int v = S.strands[last + 1][blk & (RING - 1)][j];
-                    if (bottom) vout[c] = v;
-                    else st_relaxed_pair(row + c, v, group + 1);
+                    if (!bottom) {
+                        st_relaxed_pair(row + c, v, group + 1);
+                    } else if constexpr (TWO) {
+                        if (c < P.n) vout[c] = (v & 0xFFFF) - 1;
+                        if (c < Q.n) vout2[c] = int(uint32_t(v) >> 16) - 1;
+                    } else {
+                        vout[c] = v;
+                    }
                 }
             };
 #pragma unroll
@@ -283,7 +356,7 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                     load_block<TW>(&S.codes[(base - lane) & (BRING - 1)][0], bc);
                     if constexpr (R::PIPE) {
                         int far[TM][TW], next[TM][TW];
-                        matches<TM, TW>(av, bc, far);
+                        matches<TWO, TM, TW>(av, bc, far);
                         load_block<TW>(&S.codes[(base + 1 - lane) & (BRING - 1)][0], bc);
 #pragma unroll
                         for (int s = 0; s < K; ++s) {
@@ -297,14 +370,14 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                             // wait for nothing, fill the gaps of this step's chain.
                             if (s + 1 < K) {
                                 load_block<TW>(in + (s + 1) * TW, vin);
-                                matches<TM, TW>(av, bc, next);
+                                matches<TWO, TM, TW>(av, bc, next);
                                 if (s + 2 < K) load_block<TW>(&S.codes[(base + s + 2 - lane) & (BRING - 1)][0], bc);
                             }
 #pragma unroll
                             for (int j = 0; j < TW; ++j) {
                                 int v = vi[j];
 #pragma unroll
-                                for (int q = 0; q < TM; ++q) pass(far[q][j], hv[q], v);
+                                for (int q = 0; q < TM; ++q) swap_if<TWO>(far[q][j], hv[q], v);
                                 vc[j] = v;
                             }
 #pragma unroll
@@ -331,7 +404,7 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                             for (int j = 0; j < TW; ++j) {
                                 int v = vi[j];
 #pragma unroll
-                                for (int q = 0; q < TM; ++q) cell<false>(av[q], uint32_t(bs[j]), hv[q], v);
+                                for (int q = 0; q < TM; ++q) swap_if<TWO>(match<TWO>(av[q], bs[j]), hv[q], v);
                                 vc[j] = v;
                             }
                             store_block_if<TW>(lane == 31, &S.strands[w + 1][(base + s - 31) & (RING - 1)][0], vc);
@@ -341,23 +414,28 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 }
                 for (int il = nw; il < ni - idle; ++il) {
                     // Past its last block: masked columns for the warp below.
-                    if (lane < C) S.strands[w + 1][(il * K - 31 + lane / TW) & (RING - 1)][lane % TW] = INT_MAX;
+                    if (lane < C) S.strands[w + 1][(il * K - 31 + lane / TW) & (RING - 1)][lane % TW] = NO_V;
                     sync<W>();
                 }
             }
             const int r0 = r_group + (w * 32 + lane) * TM;
 #pragma unroll
             for (int q = 0; q < TM; ++q)
-                if (r0 + q < m) hout[m - 1 - r0 - q] = hv[q];
+                if constexpr (TWO) {
+                    if (r0 + q < P.m) hout[P.m - 1 - r0 - q] = (hv[q] & 0xFFFF) - 1;
+                    if (r0 + q < Q.m) hout2[Q.m - 1 - r0 - q] = int(uint32_t(hv[q]) >> 16) - 1;
+                } else {
+                    if (r0 + q < m) hout[m - 1 - r0 - q] = hv[q];
+                }
         }
         if (!L.counters) break;
     }
 }
 
-template <int TM, int TW, int W>
+template <int TM, int TW, int W, bool TWO>
 slcs_status launch_shape(const RelayLaunch &L, int sms, cudaStream_t stream)
 {
-    constexpr auto kernel = relay_kernel<TM, TW, W>;
+    constexpr auto kernel = relay_kernel<TM, TW, W, TWO>;
     int occ = 1;
     const slcs_status os = occupancy_of<kernel>((W + 1) * 32, &occ);
     if (os != SLCS_OK || stream == PREPARE_ONLY) return os;
@@ -371,23 +449,22 @@ slcs_status launch_shape(const RelayLaunch &L, int sms, cudaStream_t stream)
 
 #define SLCS_RELAY_SHAPES(X) \
     X(1, 4, 3) X(2, 4, 3) X(4, 2, 3) X(8, 2, 3) X(8, 4, 4) X(14, 4, 4) X(14, 4, 8) X(14, 4, 16)
-
-bool relay_supported(const RelayShape &s)
-{
-#define SLCS_CASE(TM, TW, W) \
-    if (s.tm == TM && s.tw == TW && s.warps == W) return true;
-    SLCS_RELAY_SHAPES(SLCS_CASE)
-#undef SLCS_CASE
-    return false;
-}
+#define SLCS_RELAY_DUO_SHAPES(X) X(2, 4, 3) X(4, 4, 3) X(8, 2, 3) X(8, 4, 4)
 
 slcs_status launch_relay(const RelayLaunch &L, const RelayShape &s, int sms, cudaStream_t stream)
 {
     if (L.nitems <= 0 && stream != PREPARE_ONLY) return SLCS_OK;
 #define SLCS_CASE(TM, TW, W) \
-    if (s.tm == TM && s.tw == TW && s.warps == W) return launch_shape<TM, TW, W>(L, sms, stream);
-    SLCS_RELAY_SHAPES(SLCS_CASE)
+    if (s.tm == TM && s.tw == TW && s.warps == W) return launch_shape<TM, TW, W, false>(L, sms, stream);
+#define SLCS_CASE_TWO(TM, TW, W) \
+    if (s.tm == TM && s.tw == TW && s.warps == W) return launch_shape<TM, TW, W, true>(L, sms, stream);
+    if (L.two) {
+        SLCS_RELAY_DUO_SHAPES(SLCS_CASE_TWO)
+    } else {
+        SLCS_RELAY_SHAPES(SLCS_CASE)
+    }
 #undef SLCS_CASE
+#undef SLCS_CASE_TWO
     return fail(SLCS_ERR_UNSUPPORTED, "no such relay shape");
 }
 

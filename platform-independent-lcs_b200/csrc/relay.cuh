@@ -22,6 +22,11 @@ struct RelayLaunch {
     uint32_t *status;
     uint64_t wait_ns;
     PairDev single;
+    // Two pairs per register (ids of 15 bits): an item's pair is an entry of
+    // duos, two pairs (the second -1 for none) that share its groups, rows and
+    // columns (the larger of both); row_off per entry.  Otherwise null.
+    const int2 *duos; // device
+    bool two;         // duos is set (also with PREPARE_ONLY)
 };
 
 // Shape of the kernel: rows per lane, columns per step, warps that comb.
@@ -38,7 +43,6 @@ inline int64_t relay_row_elems(int32_t m, int32_t n, const RelayShape &s)
 {
     return relay_groups(m, s) > 1 ? (int64_t(n) + 1) / 2 * 2 : 0;
 }
-bool relay_supported(const RelayShape &s);
 slcs_status launch_relay(const RelayLaunch &L, const RelayShape &s, int sms, cudaStream_t stream);
 
 } // namespace slcs
