@@ -323,8 +323,10 @@ struct BatchRelay {
     double us = 0.0;
     int64_t groups = 0;
 };
+// With `budget_us`, the plan of fewest groups predicted to end within it, if any.
 template <class Take>
-BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool may_two, int sms, Take take)
+BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool may_two, int sms, Take take,
+                            double budget_us = 0.0)
 {
     BatchRelay B;
     std::vector<int32_t> ids;
@@ -333,7 +335,8 @@ BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool ma
             ids.push_back(p);
             may_two = may_two && int64_t(pairs[p].m) + pairs[p].n <= PACKED16_MAX_IDS;
         }
-    Sizes sizes;
+    Sizes sizes, both;
+    std::vector<int2> duos;
     for (int32_t p : ids) sizes.emplace_back(pairs[p].m, pairs[p].n);
     B.us = batch_relay_us(sizes, sms, &B.shape);
     if (may_two && ids.size() > 1) {
@@ -342,8 +345,6 @@ BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool ma
             const int32_t rx = pairs[x].m / ROWS, ry = pairs[y].m / ROWS;
             return rx != ry ? rx > ry : pairs[x].n != pairs[y].n ? pairs[x].n > pairs[y].n : x < y;
         });
-        std::vector<int2> duos;
-        Sizes both;
         for (size_t i = 0; i < ids.size(); i += 2) {
             const slcs_pair_desc &x = pairs[ids[i]];
             const bool second = i + 1 < ids.size();
@@ -356,11 +357,22 @@ BatchRelay plan_batch_relay(const slcs_pair_desc *pairs, int32_t npairs, bool ma
         if (us < relay_shared_us(sizes, RELAY_COSTS, sms, &one)) {
             B.us = us;
             B.shape = two;
-            B.duos = std::move(duos);
-            sizes = std::move(both);
+            B.duos = duos;
         }
     }
-    for (const auto &[m, n] : sizes) B.groups += relay_groups(m, B.shape);
+    B.groups = relay_work(B.duos.empty() ? sizes : both, B.shape).groups;
+    if (budget_us > 0) {
+        auto fewer = [&](const Sizes &of, const RelayCost &c, const std::vector<int2> &d) {
+            const RelayCost only[] = {c};
+            RelayShape shape{};
+            const double us = relay_shared_us(of, only, sms, &shape);
+            const int64_t groups = relay_work(of, shape).groups;
+            if (us <= budget_us && groups < B.groups) B = BatchRelay{shape, d, us, groups};
+        };
+        for (const RelayCost &c : RELAY_COSTS) fewer(sizes, c, {});
+        for (const RelayCost &c : RELAY_DUO_COSTS)
+            if (!duos.empty()) fewer(both, c, duos);
+    }
     return B;
 }
 
@@ -1389,6 +1401,16 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
         make_bundles(couples, 0, size_t(P->nstaged), tm, INT32_MAX, bundle_lanes);
         P->nstaged_bundles = int32_t(bundle_lanes.size() / 32);
         make_bundles(couples, size_t(P->nstaged), couples.size(), tm, BUNDLE_BLOCKS, bundle_lanes);
+        if (P->relay_sms > 0) {
+            // Beside couples the relay kernel need not be fast but few: its
+            // groups keep their SMs to themselves, and the couples take about
+            // 0.22 us a step and sub-partition.  (20,000 reads, 7 of
+            // them taller: 14 SMs for those 117 us, 4 SMs 106 us.)
+            double steps = 0;
+            for (size_t i = 0; i < bundle_lanes.size(); i += 32) steps += bundle_lanes[i].steps + 12.0;
+            relay = plan_batch_relay(pairs, npairs, may_two, sms, tall, 0.7 * 0.22 * steps / (4.0 * sms));
+            P->relay_sms = int32_t(relay.groups);
+        }
         deal_bundles(bundle_lanes, P->nstaged_bundles, 4 * (sm_count() - P->relay_sms), list_off);
         P->nlists = int32_t(list_off.size()) - 1;
     }
