@@ -11,12 +11,13 @@
 //     the node containing entry i at level l follows from i alone (node_of).
 //   * Downward, each level is a stable partition of every node: P's rows by
 //     column < s/2 (get_vert_slice, 5-19) and Q's columns by row < s/2
-//     (get_horz_slice, 22-36).  Above the cutoff every level's partition runs
-//     in one launch: single-pass tiles (they publish their counts and look
-//     back over their predecessors) take tickets level by level, and a tile
-//     first waits for the tiles of the level above that hold its parent
-//     nodes; every wait is bounded.  The maps from child index to parent
-//     index are kept per level.
+//     (get_horz_slice, 22-36); the maps from child index to parent index are
+//     kept per level.  An entry's place at every level follows from its value
+//     and counts, so products of up to 128 nodes write all levels in one pass
+//     (fan_kernel).  Larger ones go level by level in one launch: single-pass
+//     tiles (they publish their counts and look back over their predecessors)
+//     take tickets level by level, and a tile first waits for the tiles of the
+//     level above that hold its parent nodes; every wait is bounded.
 //   * A node at or below the cutoff is finished by one thread block without
 //     further recursion: it passes the crossings of P's part into Q's, S / 2
 //     at a time, in S rounds of one packed compare-and-exchange (node_kernel).
@@ -25,14 +26,15 @@
 //     the parent's result (the union of the two halves, 254-268) and into the
 //     block counts of the level's delta tables; then it walks the ant
 //     (123-189) over every node, which writes the fresh points on top.
-//   * Walks of small nodes run one thread per node.  A large node's walk is cut
-//     into segments that run concurrently: on every diagonal e = col - row the
-//     walk sits one row above r*(e-1), the first point of diagonal e-1 where
-//     the dominance difference (hi points above-left minus lo points
-//     below-right) is non-negative, so a segment can start anywhere once r* is
-//     known there (walk_lanes_kernel: one lane per segment for short segments;
-//     walk_segments_kernel: one warp per segment with the rows and columns it
-//     can touch staged in shared memory).
+//   * A node's walk is cut into segments that run concurrently: on every
+//     diagonal e = col - row the walk sits one row above r*(e-1), the first
+//     point of diagonal e-1 where the dominance difference (hi points above-left
+//     minus lo points below-right) is non-negative, so a segment can start
+//     anywhere once r* is known there.  One warp takes a segment: short ones
+//     row by row, every row independent of the others (walk_rows), long ones
+//     run by run from staged words (ant_walk_warp).  Many short segments take
+//     one lane each (walk_lanes_kernel).
+//   * Products of one overlap run side by side in the same launches.
 #include <climits>
 #include <cmath>
 #include <vector>
@@ -103,7 +105,6 @@ struct LevelArgs {
     int32_t *Pn, *Qn;  // next level
     int32_t *pmap, *qmap; // next level: child index -> parent-local index
     int32_t *scanP, *scanQ;
-    int32_t *bsumP, *bsumQ;
     int k, level;
     const int32_t *bad;
 };
@@ -510,7 +511,7 @@ __global__ void __launch_bounds__(PART_THREADS) part_levels_kernel(const __grid_
         const int lv = t / G.kb, tile = t % G.kb;
         int32_t *in = G.PQ + ((lv & 1) ? 2 * kk : 0), *nx = G.PQ + ((lv & 1) ? 0 : 2 * kk);
         int32_t *mp = G.maps + 2 * kk * size_t(lv + 1);
-        FusedArgs F{LevelArgs{in, in + kk, nx, nx + kk, mp, mp + kk, G.scanP, G.scanQ, nullptr, nullptr, G.k, lv,
+        FusedArgs F{LevelArgs{in, in + kk, nx, nx + kk, mp, mp + kk, G.scanP, G.scanQ, G.k, lv,
                               G.err},
                     G.tiles + size_t(lv) * G.kb, G.done + size_t(lv) * G.kb, G.err, G.status};
         const bool local = G.pow2 && (G.k >> lv) <= PART_BS; // the level's nodes fit inside tiles
