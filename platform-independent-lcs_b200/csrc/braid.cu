@@ -44,7 +44,10 @@
 namespace slcs {
 namespace {
 
-constexpr int SCAN_BS = 2048;   // elements per block of the device-wide scan
+// Entries per block of the slices: two a thread, since a block's time is its
+// chain of dependent reads (2048: products 1003 61 -> 54 us, 32768 198 -> 188;
+// 256: 1000 x 1000000 pairs 866 -> 936 us, each block then adds more counts).
+constexpr int SCAN_BS = 512;
 constexpr int PART_PER = 8;     // entries per thread of a partition tile
 // Threads of a partition tile: 1024 (8192 entries, one tile per SM at a time,
 // a short look-back chain) for large products, 256 (2048 entries) below.
@@ -94,7 +97,7 @@ constexpr int FAN_LEAVES = 128;
 constexpr int FAN_TILE = 1024;
 __host__ __device__ constexpr int fan_tiles(int k) { return (k + FAN_TILE - 1) / FAN_TILE; }
 // Up to this many slice blocks add their predecessors' counts themselves.
-constexpr int SLICE_DIRECT = 1024;
+constexpr int SLICE_DIRECT = 4096;
 
 // ---------------------------------------------------------------------------
 // device-wide exclusive scan of two flag sets (partition of P rows and Q cols)
@@ -954,9 +957,13 @@ __device__ __forceinline__ void node_by_index(int nd, int level, int k, int &o, 
 }
 
 // One warp per (node, row block): exclusive prefix of the hi counts and
-// inclusive suffix of the lo counts along the row, 32 columns per step, the
-// two scans side by side (hi from the left, lo from the right) with the next
-// step's words read before this step's scan.
+// inclusive suffix of the lo counts along the row, the two scans side by side
+// (hi from the left, lo from the right), ROW_STEPS groups of 32 columns at a
+// time: a lone warp's row is bound by the latency of its reads and shuffles,
+// so the groups' scans run side by side and the next ones' words are read before
+// them (one group at a time: products of overlap 32768 187 -> 183 us, 131072
+// 331 -> 316; eight: 183 and 320).
+constexpr int ROW_STEPS = 4;
 template <int N>
 __global__ void __launch_bounds__(256) table_rows_kernel(const __grid_constant__ Many<TableArgs, N> M, int nodes)
 {
@@ -973,27 +980,42 @@ __global__ void __launch_bounds__(256) table_rows_kernel(const __grid_constant__
     int32_t *hi = A.cnt_hi + size_t(nd) * A.stride * A.stride + size_t(bi) * A.stride;
     int32_t *lo = A.cnt_lo + size_t(nd) * A.stride * A.stride + size_t(bi) * A.stride;
     const int nch = G / 32 + 1; // steps of 32 columns over 0..G
-    int nh = lane <= G ? hi[lane] : 0;
-    int nl = (nch - 1) * 32 + lane <= G ? lo[(nch - 1) * 32 + lane] : 0;
+    int nh[ROW_STEPS], nl[ROW_STEPS];
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < ROW_STEPS; ++u) {
+            const int jh = (c0 + u) * 32 + lane, jl = (nch - 1 - c0 - u) * 32 + lane;
+            nh[u] = jh <= G ? hi[jh] : 0;
+            nl[u] = jl >= 0 && jl <= G ? lo[jl] : 0;
+        }
+    };
+    load(0);
     int carry_h = 0, carry_l = 0;
-    for (int c = 0; c < nch; ++c) {
-        const int jh = c * 32 + lane, jl = (nch - 1 - c) * 32 + lane;
-        const int vh = nh, vl = nl;
-        if (c + 1 < nch) {
-            nh = jh + 32 <= G ? hi[jh + 32] : 0;
-            nl = lo[jl - 32]; // jl - 32 <= G - 32 + 31 < G
+    for (int c0 = 0; c0 < nch; c0 += ROW_STEPS) {
+        int vh[ROW_STEPS], xh[ROW_STEPS], xl[ROW_STEPS]; // xl becomes the sum over lanes >= lane
+#pragma unroll
+        for (int u = 0; u < ROW_STEPS; ++u) {
+            vh[u] = xh[u] = nh[u];
+            xl[u] = nl[u];
         }
-        int xh = vh, xl = vl; // xl becomes the sum over lanes >= lane
-        for (int off = 1; off < 32; off <<= 1) {
-            const int yh = __shfl_up_sync(FULL_MASK, xh, off);
-            const int yl = __shfl_down_sync(FULL_MASK, xl, off);
-            if (lane >= off) xh += yh;
-            if (lane + off < 32) xl += yl;
+        if (c0 + ROW_STEPS < nch) load(c0 + ROW_STEPS);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+#pragma unroll
+            for (int u = 0; u < ROW_STEPS; ++u) {
+                const int yh = __shfl_up_sync(FULL_MASK, xh[u], off);
+                const int yl = __shfl_down_sync(FULL_MASK, xl[u], off);
+                if (lane >= off) xh[u] += yh;
+                if (lane + off < 32) xl[u] += yl;
+            }
+#pragma unroll
+        for (int u = 0; u < ROW_STEPS; ++u) {
+            const int jh = (c0 + u) * 32 + lane, jl = (nch - 1 - c0 - u) * 32 + lane;
+            if (jh <= G) hi[jh] = carry_h + xh[u] - vh[u];
+            if (jl >= 0 && jl <= G) lo[jl] = carry_l + xl[u];
+            carry_h += __shfl_sync(FULL_MASK, xh[u], 31);
+            carry_l += __shfl_sync(FULL_MASK, xl[u], 0);
         }
-        if (jh <= G) hi[jh] = carry_h + xh - vh;
-        if (jl <= G) lo[jl] = carry_l + xl;
-        carry_h += __shfl_sync(FULL_MASK, xh, 31);
-        carry_l += __shfl_sync(FULL_MASK, xl, 0);
     }
 }
 

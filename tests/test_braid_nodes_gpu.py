@@ -44,3 +44,10 @@ def test_partitions(cuda, k, cutoff):
     """Every level in one pass up to 128 nodes (one entry more: level by level), around its tiles of 1024."""
     rng = np.random.default_rng(k)
     _check(rng.permutation(k + 3), rng.permutation(k + 2500), k, cutoff)
+
+
+def test_many_slice_blocks(cuda):
+    """More blocks of the slices than add their predecessors' counts themselves."""
+    rng = np.random.default_rng(3)
+    _check(rng.permutation(2200000), rng.permutation(300), 57, None)
+    _check(rng.permutation(300), rng.permutation(2200000), 57, None)
