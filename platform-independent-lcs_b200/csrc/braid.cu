@@ -13,7 +13,7 @@
 //     column < s/2 (get_vert_slice, 5-19) and Q's columns by row < s/2
 //     (get_horz_slice, 22-36); the maps from child index to parent index are
 //     kept per level.  An entry's place at every level follows from its value
-//     and counts, so products of up to 128 nodes write all levels in one pass
+//     and counts, so products of up to 256 nodes write all levels in one pass
 //     (fan_kernel).  Larger ones go level by level in one launch: single-pass
 //     tiles (they publish their counts and look back over their predecessors)
 //     take tickets level by level, and a tile first waits for the tiles of the
@@ -93,7 +93,7 @@ __device__ __forceinline__ int leaf_of(int v, int lc, int k)
 
 // Products whose level lc has at most FAN_LEAVES nodes partition every level
 // in one pass (fan_kernel), in tiles of FAN_TILE entries.
-constexpr int FAN_LEAVES = 128;
+constexpr int FAN_LEAVES = 256;
 constexpr int FAN_TILE = 1024;
 __host__ __device__ constexpr int fan_tiles(int k) { return (k + FAN_TILE - 1) / FAN_TILE; }
 // Up to this many slice blocks add their predecessors' counts themselves.
@@ -1593,8 +1593,9 @@ __global__ void __launch_bounds__(256) slice_write_kernel(const __grid_constant_
 // ranks a warp's entries within their node, level by level.  No block waits
 // for another.  At an overlap of 32768 (5 levels) the level-by-level
 // partitions took 59 us, waiting for one another; this takes 6 (MEASURED).
-// The tables grow with the tiles times the nodes, so products of more than
-// FAN_LEAVES nodes keep the level-by-level form.
+// The counts grow with the tiles times the nodes, and the sums take 132 bytes of
+// shared memory a node, so products of more than FAN_LEAVES nodes keep the
+// level-by-level form (256 nodes instead of 128: 262144 569 -> 478 us).
 // ---------------------------------------------------------------------------
 struct FanArgs {
     const int32_t *in; // level 0: P then Q (k entries each)

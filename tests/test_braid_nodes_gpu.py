@@ -39,9 +39,10 @@ def test_cutoffs(cuda, cutoff):
 
 
 @pytest.mark.parametrize("k,cutoff", [(1023, 8), (1024, 8), (1025, 9), (1025, 8), (2049, 1024), (4801, 38), (4801, 37),
-                                      (153600, 1200), (153601, 1200)])
+                                      (153600, 1200), (153601, 1200), (4801, 19), (4801, 18),
+                                      (307200, 1200), (307201, 1200)])
 def test_partitions(cuda, k, cutoff):
-    """Every level in one pass up to 128 nodes (one entry more: level by level), around its tiles of 1024."""
+    """Every level in one pass up to 256 nodes (one entry more: level by level), around its tiles of 1024."""
     rng = np.random.default_rng(k)
     _check(rng.permutation(k + 3), rng.permutation(k + 2500), k, cutoff)
 
