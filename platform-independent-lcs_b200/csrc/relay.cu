@@ -21,9 +21,11 @@
 //     top, and writes out the ones that leave it at the bottom.
 //   * Blocks hand down through one row of (strand, group) words per pair.  The
 //     group number next to each strand says whose it is, so a reader needs no
-//     flag and no fence, and the row is reused in place by every group; it is
-//     copied two intervals ahead and polled only where the copy came too
-//     early.  Every wait is bounded as in the wavefront kernel.
+//     flag and no fence, and the row is reused in place by every group.  That
+//     holds only while a word is stored and loaded as one, so both sides use
+//     8-byte relaxed accesses and nothing else (a wider or asynchronous copy
+//     promises no such thing).  Entries are loaded ahead and polled only where
+//     that was too early.  Every wait is bounded as in the wavefront kernel.
 //   * Blocks take groups from a ticket counter; the group above a block's own
 //     was therefore claimed by a running block.
 //   * Batches whose ids fit 15 bits may put two pairs in a register (TWO, the
@@ -147,11 +149,19 @@ struct Relay {
     // Intervals a warp starts after the one above it: block t leaves lane 31
     // in interval (t + 31) / K and must be read in a later one, t / K + DI.
     static constexpr int DI = (30 + K) / K + 1;
-    static constexpr int PF = 2;                         // intervals the I/O warp copies row entries ahead
+    // How the I/O warp brings the row entries: LOADS words per lane for FETCH
+    // intervals at once, issued when the entries before them are delivered or,
+    // where intervals are shorter than an L2 round trip and a lane's word is
+    // only one of them (DEEP), that many intervals earlier.  A load waits for
+    // the one before it: with one per interval, two intervals ahead, 4096 x
+    // 4096 took 176 us and 1003 x 250007 482, so 152 and 434 (the latter 472
+    // without DEEP).
+    static constexpr bool DEEP = C == 32 && TM * TW < 32;
+    static constexpr int FETCH = DEEP ? 2 : 32 / C;
+    static constexpr int LOADS = FETCH * C / 32;
     // Matches computed one step ahead, while their registers are few (a step
     // of (8, 4): 217 -> 196 cycles in a register probe, of (4, 2) 77 -> 72).
     static constexpr bool PIPE = TM * TW <= 32;
-    static constexpr int STAGES = next_pow2(PF + 1);
     static constexpr int RING = 4 * K;                   // blocks of a ring between two warps
     // Blocks of symbols between the one being delivered and the one lane 31
     // of the last warp still combs.
@@ -159,7 +169,6 @@ struct Relay {
     struct Shared {
         int32_t strands[W + 1][RING][TW];
         int32_t codes[BRING][TW];
-        int2 stage[STAGES][C];
         int32_t item;
     };
 };
@@ -177,7 +186,7 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
     constexpr int NO_COLUMN = TWO ? int(MASKED_COLUMN16) : int(MASKED_COLUMN); // symbol of a masked column
     constexpr int NO_V = TWO ? int(MASKED_V16) : INT_MAX;                      // and its strand
     using R = Relay<TM, TW, W>;
-    constexpr int K = R::K, C = R::C, DI = R::DI, RING = R::RING, BRING = R::BRING, PF = R::PF, STAGES = R::STAGES;
+    constexpr int K = R::K, C = R::C, DI = R::DI, RING = R::RING, BRING = R::BRING, FETCH = R::FETCH, LOADS = R::LOADS;
     __shared__ __align__(16) typename R::Shared S;
     const int lane = threadIdx.x & 31;
     const int w = __shfl_sync(FULL_MASK, int(threadIdx.x) >> 5, 0); // warp-uniform for the compiler
@@ -252,10 +261,20 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 word2 = four_columns(b2, 4 * lane, Q.n, aligned2);
                 word2_next = four_columns(b2, 128 + 4 * lane, Q.n, aligned2);
             }
-            auto fetch = [&](int i) { // start the copy of the row entries of interval i
-                const int c = i * C + 2 * lane;
-                if (group && 2 * lane < C && c < n) cp_async_cg16(&S.stage[i & (STAGES - 1)][2 * lane], row + c);
-                cp_async_commit();
+            // Start the loads of the row entries of intervals i .. i + FETCH - 1.
+            auto fetch = [&](int i, int2 (&e)[LOADS]) {
+#pragma unroll
+                for (int x = 0; x < LOADS; ++x) {
+                    const int c = i * C + 32 * x + lane;
+                    e[x] = make_int2(0, group);
+                    if (group && c < n) e[x] = ld_relaxed_pair(row + c);
+                }
+            };
+            // This lane's entry of the x-th of those intervals.
+            auto entry = [&](const int2 (&e)[LOADS], int x) {
+                if constexpr (C == 32) return e[x];
+                else return make_int2(__shfl_sync(FULL_MASK, e[0].x, lane + C * x),
+                                      __shfl_sync(FULL_MASK, e[0].y, lane + C * x));
             };
             auto give_up = [&]() { // another wait gave up, or this one has reached its limit
                 const uint64_t now = globaltimer_ns();
@@ -267,17 +286,14 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 }
                 return __any_sync(FULL_MASK, late || ld_relaxed_gpu(L.counters + 1)) != 0;
             };
-            auto deliver = [&](int i) {
+            auto deliver = [&](int i, int2 e) { // e: the lane's row entry as fetch found it
                 const int c = i * C + lane;
                 const bool in = lane < C && c < n;
                 int v = in ? m + c : INT_MAX;
                 if constexpr (TWO) // ids plus one
                     v = (c < P.n ? P.m + c + 1 : 0x7FFF) | (c < Q.n ? Q.m + c + 1 : 0x7FFF) << 16;
                 if (group) {
-                    cp_async_wait<PF - 1>();
-                    __syncwarp();
-                    int2 e = make_int2(0, group);
-                    if (in) e = S.stage[i & (STAGES - 1)][lane];
+                    if (!in) e.y = group;
                     for (int polls = 0; !dead && __any_sync(FULL_MASK, e.y != group); ++polls) {
                         if (e.y != group) e = ld_relaxed_pair(row + c);
                         if ((polls & 31) == 31) dead = give_up();
@@ -327,21 +343,31 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                     }
                 }
             };
-#pragma unroll
-            for (int x = 0; x < PF; ++x) fetch(x);
-            deliver(0);
-            fetch(PF);
+            int2 now[LOADS], ahead[LOADS];
+            fetch(0, now);
+            deliver(0, entry(now, 0));
+            if constexpr (R::DEEP) fetch(FETCH, ahead);
+            else if constexpr (FETCH == 1) fetch(1, now);
             sync<W>();
-            for (int i = 0; i < ni; ++i) {
-                if (i) flush(i - 1);
-                if (i + 1 < nw) {
-                    deliver(i + 1);
-                    fetch(i + 1 + PF);
+            for (int i0 = 0; i0 < ni; i0 += FETCH) {
+#pragma unroll
+                for (int x = 0; x < FETCH; ++x) {
+                    const int i = i0 + x, next = (x + 1) % FETCH; // the entry to deliver
+                    if (i >= ni) break;
+                    if (i) flush(i - 1);
+                    if (i + 1 < nw) {
+                        if (R::DEEP && next == 0) {
+#pragma unroll
+                            for (int l = 0; l < LOADS; ++l) now[l] = ahead[l];
+                        }
+                        deliver(i + 1, entry(now, next));
+                        if (R::DEEP && next == 0) fetch(i + 1 + FETCH, ahead);
+                        if (!R::DEEP && next == FETCH - 1) fetch(i + 2, now);
+                    }
+                    sync<W>();
                 }
-                sync<W>();
             }
             flush(ni - 1);
-            cp_async_wait<0>();
         } else {
             // Intervals before this warp's first block, with its blocks, and
             // after its last one.

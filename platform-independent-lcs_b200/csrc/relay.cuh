@@ -38,10 +38,10 @@ inline int32_t relay_groups(int32_t m, const RelayShape &s)
     const int32_t rows = 32 * s.tm * s.warps;
     return (m + rows - 1) / rows;
 }
-// Entries of the hand-down row of a pair (0 with one group), even.
+// Entries of the hand-down row of a pair (0 with one group).
 inline int64_t relay_row_elems(int32_t m, int32_t n, const RelayShape &s)
 {
-    return relay_groups(m, s) > 1 ? (int64_t(n) + 1) / 2 * 2 : 0;
+    return relay_groups(m, s) > 1 ? int64_t(n) : 0;
 }
 slcs_status launch_relay(const RelayLaunch &L, const RelayShape &s, int sms, cudaStream_t stream);
 
