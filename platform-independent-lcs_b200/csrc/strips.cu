@@ -18,7 +18,6 @@
 // at once; strips multiply the chains of a short pair, so that they fill the
 // GPU.  Column strips are also the per-GPU unit of the multi-GPU split.
 #include <algorithm>
-#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -43,6 +42,53 @@ __global__ void perm_to_strands_kernel(const int32_t *__restrict__ r2c, int32_t 
         else if (c >= n && int64_t(c) < size)
             h[c - n] = int32_t(i);
     }
+}
+
+// The tiles of a comb, numbered band by band, and its schedule, written on the
+// device (a copy from the call's own memory would be read again, long after
+// that memory is gone, by every replay of a graph that the call was captured in).
+struct Tiles {
+    int32_t m, n, bands, strips;
+    int32_t stripe_rows, stripes; // rows of a stripe, stripes of a
+    int32_t per;                  // stripes of a task: 1, or a relay group's
+    int32_t base;                 // columns of every strip but the last
+    int64_t hand;                 // entries of a band's scratch or hand-down rows; 0: no tile needs one
+
+    __host__ __device__ int64_t row(int64_t r) const // first row of band r
+    {
+        const int64_t x = int64_t(stripes) * r / bands * stripe_rows;
+        return r < bands && x < m ? x : m;
+    }
+    __host__ __device__ int64_t column(int64_t s) const { return s < strips ? s * base : n; }
+    __host__ __device__ int64_t tasks(int64_t r) const // of one tile of band r
+    {
+        const int64_t count = int64_t(stripes) * (r + 1) / bands - int64_t(stripes) * r / bands;
+        return (count + per - 1) / per;
+    }
+    __host__ __device__ int64_t tasks_before(int64_t r) const // of all tiles of the bands above r
+    {
+        if (per == 1) return int64_t(stripes) * r / bands * strips;
+        int64_t t = 0;
+        for (int64_t x = 0; x < r; ++x) t += tasks(x);
+        return t * strips;
+    }
+    __host__ __device__ PairDev tile(int64_t r, int64_t s) const
+    {
+        const int64_t a0 = row(r), b0 = column(s), h = row(r + 1) - a0;
+        return PairDev{a0, b0, strips * a0 + r * n + s * h + b0, int32_t(h), int32_t(column(s + 1) - b0)};
+    }
+};
+
+// One block per tile.
+__global__ void __launch_bounds__(128) tiles_kernel(const Tiles G, PairDev *pairs, int2 *tasks, int64_t *hand_off)
+{
+    const int t = blockIdx.x, r = t / G.strips, s = t % G.strips;
+    const int64_t count = G.tasks(r), first = G.tasks_before(r) + s * count;
+    if (threadIdx.x == 0) {
+        pairs[t] = G.tile(r, s);
+        hand_off[t] = r * G.hand + (G.hand > 0 ? G.column(s) : 0); // strips start at multiples of 16
+    }
+    for (int64_t k = threadIdx.x; k < count; k += blockDim.x) tasks[first + k] = make_int2(t, int(k));
 }
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -268,35 +314,16 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     const int S = strip_count(cfg, n);
     const std::vector<int32_t> hgt = band_heights(m, R, tm);
     const std::vector<int32_t> w = strip_widths(n, S);
-    // Tile (r, s) = (band r of a, strip s of b), numbered r * S + s.
+    // Tile (r, s) = (band r of a, strip s of b), numbered r * S + s; the tasks
+    // of the comb are the stripes (relay: groups of stripes) of every tile,
+    // tile after tile, so that a task's producer is the one before it.
     const int T = R * S;
-    std::vector<slcs_pair_desc> pd(static_cast<size_t>(T));
-    int64_t o0 = 0;
-    {
-        int64_t a0 = 0;
-        for (int r = 0; r < R; ++r) {
-            int64_t b0 = 0;
-            for (int s = 0; s < S; ++s) {
-                pd[size_t(r * S + s)] = slcs_pair_desc{a0, b0, o0, hgt[size_t(r)], w[size_t(s)]};
-                b0 += w[size_t(s)];
-                o0 += int64_t(hgt[size_t(r)]) + w[size_t(s)];
-            }
-            a0 += hgt[size_t(r)];
-        }
-    }
-    const int64_t total = o0; // S*m + R*n strands
-    // Schedule of the comb: the stripes (relay: groups of stripes) of every
-    // tile, tile after tile, so that a stripe's producer is the task before it.
-    std::vector<int2> tasks;
-    std::vector<int64_t> scr_off(size_t(T), 0);
-    int64_t scr_elems = 0; // int32 of the wavefront's scratch, int2 of the relay's rows
-    for (int t = 0; t < T; ++t) {
-        const slcs_pair_desc &d = pd[size_t(t)];
-        const int32_t count = relay ? relay_groups(d.m, *relay) : stripes_of(d.m, tm);
-        for (int32_t k = 0; k < count; ++k) tasks.push_back(make_int2(t, k));
-        scr_off[size_t(t)] = scr_elems;
-        scr_elems += relay ? relay_row_elems(d.m, d.n, *relay) : scratch_elems(d.m, d.n, tm);
-    }
+    Tiles G{m, n, R, S, 32 * tm, stripes_of(m, tm), relay ? relay->warps : 1, w[0], 0};
+    const int64_t total = int64_t(S) * m + int64_t(R) * n; // strands
+    const int64_t ntasks = G.tasks_before(R);
+    if (ntasks > T) // int32 of the wavefront's scratch, int2 of the relay's rows; whole 32-byte sectors
+        G.hand = G.column(S - 1) + (int64_t(w[size_t(S - 1)]) + 7) / 8 * 8;
+    const int64_t scr_elems = R * G.hand;
     const int cutoff = (cfg && cfg->braid_cutoff > 0) ? cfg->braid_cutoff : 0;
     // The merge tree: strips of every band glue with overlap = band height
     // (column glue), all bands side by side; then the bands glue with overlap
@@ -306,8 +333,8 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     {
         std::vector<std::vector<Perm>> rows(static_cast<size_t>(R));
         for (int t = 0; t < T; ++t) {
-            const slcs_pair_desc &d = pd[size_t(t)];
-            rows[size_t(t / S)].push_back({d.out_offset, int64_t(d.m) + d.n});
+            const PairDev d = G.tile(t / S, t % S);
+            rows[size_t(t / S)].push_back({d.out_off, int64_t(d.m) + d.n});
         }
         while (rows[0].size() > 1) {
             std::vector<Level::Job> jobs;
@@ -327,12 +354,12 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     // strands / permutations (two buffers of S*m+R*n), braid workspaces.
     const size_t o_pairs = 0;
     const size_t o_tasks = align256(o_pairs + sizeof(PairDev) * size_t(T));
-    const size_t o_soff = align256(o_tasks + sizeof(int2) * tasks.size());
+    const size_t o_soff = align256(o_tasks + sizeof(int2) * size_t(ntasks));
     const size_t o_work = align256(o_soff + sizeof(int64_t) * size_t(T));
     // The counters and, after them, what must be zero with them: the
     // wavefront's progress or the relay's rows.
     const size_t scr_bytes = size_t(scr_elems) * (relay ? sizeof(int2) : sizeof(int32_t));
-    const size_t work_bytes = align256(relay ? 16 + scr_bytes : sizeof(int32_t) * (4 + tasks.size()));
+    const size_t work_bytes = align256(relay ? 16 + scr_bytes : sizeof(int32_t) * (4 + size_t(ntasks)));
     const size_t o_scr = o_work + work_bytes;
     const size_t o_x = align256(o_scr + (relay ? 0 : scr_bytes + 16));
     const size_t o_y = align256(o_x + sizeof(int32_t) * size_t(total));
@@ -345,12 +372,9 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
     auto cu = [&](cudaError_t e, const char *what) {
         if (s == SLCS_OK && e != cudaSuccess) s = cuda_fail(e, what);
     };
-    // A pageable copy has left the vector when it returns.
-    std::vector<char> head(o_work);
-    std::memcpy(head.data() + o_pairs, pd.data(), sizeof(PairDev) * size_t(T));
-    std::memcpy(head.data() + o_tasks, tasks.data(), sizeof(int2) * tasks.size());
-    std::memcpy(head.data() + o_soff, scr_off.data(), sizeof(int64_t) * size_t(T));
-    cu(cudaMemcpyAsync(ws, head.data(), o_work, cudaMemcpyHostToDevice, st), "descriptors, tasks, scratch offsets");
+    tiles_kernel<<<T, 128, 0, st>>>(G, reinterpret_cast<PairDev *>(ws + o_pairs), reinterpret_cast<int2 *>(ws + o_tasks),
+                                    reinterpret_cast<int64_t *>(ws + o_soff));
+    cu(cudaGetLastError(), "tiles");
     cu(cudaMemsetAsync(ws + o_work, 0, work_bytes, st), "counters");
     int32_t *X = reinterpret_cast<int32_t *>(ws + o_x);
     int32_t *Y = reinterpret_cast<int32_t *>(ws + o_y);
@@ -358,7 +382,7 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         RelayLaunch L{};
         L.pairs = reinterpret_cast<const PairDev *>(ws + o_pairs);
         L.items = reinterpret_cast<const int2 *>(ws + o_tasks);
-        L.nitems = int32_t(tasks.size());
+        L.nitems = int32_t(ntasks);
         L.a_blob = a;
         L.b_blob = b;
         L.out = X;
@@ -372,7 +396,7 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         CombLaunch L{};
         L.pairs = reinterpret_cast<const PairDev *>(ws + o_pairs);
         L.tasks = reinterpret_cast<const int2 *>(ws + o_tasks);
-        L.ntasks = int32_t(tasks.size());
+        L.ntasks = int32_t(ntasks);
         L.a_blob = a;
         L.b_blob = b;
         L.out = X;
@@ -382,13 +406,9 @@ slcs_status comb_strips(const uint8_t *a, int32_t m, const uint8_t *b, int32_t n
         L.progress = L.counters + 4;
         L.status = device_status_word();
         L.wait_ns = wait_limit_ns(cfg);
-        int64_t chain = 0, width = INT64_MAX;
-        for (const slcs_pair_desc &d : pd) {
-            chain = std::max<int64_t>(chain, stripes_of(d.m, tm));
-            width = std::min<int64_t>(width, d.n);
-        }
-        L.tw = pick_tw(tm, chain, width, b);
-        L.wide = std::any_of(pd.begin(), pd.end(), [&](const slcs_pair_desc &d) { return wide_ids(d.m, d.n, cfg); });
+        const int32_t tallest = *std::max_element(hgt.begin(), hgt.end());
+        L.tw = pick_tw(tm, stripes_of(tallest, tm), *std::min_element(w.begin(), w.end()), b);
+        L.wide = wide_ids(tallest, *std::max_element(w.begin(), w.end()), cfg);
         s = launch_comb(L, tm, warps, st, nullptr);
     }
     // Strands of every tile -> its permutation (row -> col) in Y.
