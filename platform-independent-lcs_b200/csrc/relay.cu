@@ -154,7 +154,7 @@ struct Relay {
     // where intervals are shorter than an L2 round trip and a lane's word is
     // only one of them (DEEP), that many intervals earlier.  A load waits for
     // the one before it: with one per interval, two intervals ahead, 4096 x
-    // 4096 took 176 us and 1003 x 250007 482, so 152 and 434 (the latter 472
+    // 4096 took 176 us and 1003 x 250007 482, so 150 and 434 (the latter 472
     // without DEEP).
     static constexpr bool DEEP = C == 32 && TM * TW < 32;
     static constexpr int FETCH = DEEP ? 2 : 32 / C;
@@ -276,15 +276,22 @@ __global__ void __launch_bounds__((W + 1) * 32) relay_kernel(const RelayLaunch L
                 else return make_int2(__shfl_sync(FULL_MASK, e[0].x, lane + C * x),
                                       __shfl_sync(FULL_MASK, e[0].y, lane + C * x));
             };
-            auto give_up = [&]() { // another wait gave up, or this one has reached its limit
-                const uint64_t now = globaltimer_ns();
-                if (t0 == 0) t0 = now;
-                const bool late = now - t0 > L.wait_ns;
-                if (late && lane == 0) {
-                    st_relaxed_gpu(L.counters + 1, 1);
-                    raise_status(L.status, DEV_ERR_TIMEOUT);
+            // Another wait gave up, or this one has reached its limit.  Lane 0
+            // decides for the warp: a lane that stopped alone would hand down
+            // what it has not got, with no word to the host.
+            auto give_up = [&]() {
+                bool over = false;
+                if (lane == 0) {
+                    const uint64_t now = globaltimer_ns();
+                    if (t0 == 0) t0 = now;
+                    over = ld_relaxed_gpu(L.counters + 1) != 0;
+                    if (!over && now - t0 > L.wait_ns) {
+                        over = true;
+                        st_relaxed_gpu(L.counters + 1, 1);
+                        raise_status(L.status, DEV_ERR_TIMEOUT);
+                    }
                 }
-                return __any_sync(FULL_MASK, late || ld_relaxed_gpu(L.counters + 1)) != 0;
+                return __shfl_sync(FULL_MASK, int(over), 0) != 0;
             };
             auto deliver = [&](int i, int2 e) { // e: the lane's row entry as fetch found it
                 const int c = i * C + lane;
