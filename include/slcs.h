@@ -68,8 +68,9 @@ typedef struct {
     int32_t blocks_per_sm; /* batch plans: resident blocks per SM (default: 2 for plans with packed
                               pairs, else as many as fit)                                 */
     int32_t strand_bits;   /* batch plans: 16 = combine two pairs per register where ids fit 15 bits,
-                              32 = 32-bit strands only, 0 = engine default; wavefront combs: 32 =
-                              the cell rule for ids of any size                            */
+                              32 = 32-bit strands only, 0 = engine default; single pairs and
+                              wavefront plans: 64 = the cell rule for ids of any size, which
+                              pairs of more than 2^30 ids take by themselves               */
     int32_t bands;         /* row bands of a for SLCS_ALGO_STRIPS (glued by row-glue products) */
     int32_t pool_pct;      /* batch plans: percent of each stream class's work kept in a pool that
                               segments claim pair by pair once their own lists are done

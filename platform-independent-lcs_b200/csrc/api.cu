@@ -1332,6 +1332,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     {
         CombLaunch dummy{};
         dummy.ntasks = 1;
+        dummy.wide = P->wide;
         slcs_status ps = P->stm > 0 ? launch_batch(BatchLaunch{dummy}, P->tns, PREPARE_ONLY, &full_grid)
                                     : launch_comb(dummy, P->tm, P->warps, PREPARE_ONLY, nullptr);
         if (ps == SLCS_OK && P->couple_tm > 0) ps = launch_couples(CouplesLaunch{}, P->couple_tm, 0, false, 1, PREPARE_ONLY);

@@ -620,7 +620,7 @@ struct Balanced {
     int smem = 0;
 };
 
-template <int TM, int TW>
+template <int TM, int TW, bool WIDE>
 slcs_status balanced_setup(Balanced &B)
 {
     int dev = 0, per_sm = 0, optin = 0;
@@ -628,13 +628,13 @@ slcs_status balanced_setup(Balanced &B)
     SLCS_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     SLCS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa{};
-    SLCS_CUDA(cudaFuncGetAttributes(&fa, comb_wavefront_kernel<TM, WF_SM_WARPS, TW>));
+    SLCS_CUDA(cudaFuncGetAttributes(&fa, comb_wavefront_kernel<TM, WF_SM_WARPS, TW, WIDE>));
     const int want = per_sm / 2 + 1024 - int(fa.sharedSizeBytes);
     if (want <= 0 || want + int(fa.sharedSizeBytes) > optin) return SLCS_OK;
-    SLCS_CUDA(cudaFuncSetAttribute(comb_wavefront_kernel<TM, WF_SM_WARPS, TW>,
+    SLCS_CUDA(cudaFuncSetAttribute(comb_wavefront_kernel<TM, WF_SM_WARPS, TW, WIDE>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, want));
     int occ = 0;
-    SLCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, comb_wavefront_kernel<TM, WF_SM_WARPS, TW>,
+    SLCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, comb_wavefront_kernel<TM, WF_SM_WARPS, TW, WIDE>,
                                                             WF_SM_WARPS * 32, size_t(want)));
     B.smem = want;
     B.ok = occ == 1;
@@ -642,7 +642,7 @@ slcs_status balanced_setup(Balanced &B)
 }
 
 // Launches the balanced form when it applies; *done tells whether it did.
-template <int TM, int TW>
+template <int TM, int TW, bool WIDE>
 slcs_status launch_balanced(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out, bool *done)
 {
     // Function attributes belong to a device: one set-up per device.
@@ -657,7 +657,7 @@ slcs_status launch_balanced(const CombLaunch &L, long sms, cudaStream_t stream, 
     {
         std::lock_guard<std::mutex> g(mu);
         if (!ready[dev]) {
-            const slcs_status s = balanced_setup<TM, TW>(B);
+            const slcs_status s = balanced_setup<TM, TW, WIDE>(B);
             if (s != SLCS_OK) return s;
             ready[dev] = true;
         }
@@ -668,7 +668,7 @@ slcs_status launch_balanced(const CombLaunch &L, long sms, cudaStream_t stream, 
     *done = true;
     if (stream == PREPARE_ONLY) return SLCS_OK;
     const long grid = std::min<long>(sms, L.ntasks);
-    comb_wavefront_kernel<TM, WF_SM_WARPS, TW><<<int(grid), int(per_sm) * 32, size_t(B.smem), stream>>>(L);
+    comb_wavefront_kernel<TM, WF_SM_WARPS, TW, WIDE><<<int(grid), int(per_sm) * 32, size_t(B.smem), stream>>>(L);
     if (grid_out) *grid_out = int(grid);
     SLCS_CUDA(cudaGetLastError());
     return SLCS_OK;
@@ -700,22 +700,22 @@ slcs_status launch_persistent(const CombLaunch &L, long sms, cudaStream_t stream
     return SLCS_OK;
 }
 
-template <int TM, int WARPS, int TW>
+template <int TM, int WARPS, int TW, bool WIDE>
 slcs_status launch_variant_tw(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out)
 {
     bool done = false;
-    const slcs_status bs = launch_balanced<TM, TW>(L, sms, stream, grid_out, &done);
+    const slcs_status bs = launch_balanced<TM, TW, WIDE>(L, sms, stream, grid_out, &done);
     if (bs != SLCS_OK || done) return bs;
-    return launch_persistent<TM, WARPS, TW, false>(L, sms, stream, grid_out);
+    return launch_persistent<TM, WARPS, TW, WIDE>(L, sms, stream, grid_out);
 }
 
-template <int TM, int WARPS>
+template <int TM, int WARPS, bool WIDE>
 slcs_status launch_variant(const CombLaunch &L, long sms, cudaStream_t stream, int *grid_out)
 {
     if constexpr (TM == 14 || TM == 16) {
-        if (L.tw == 8) return launch_variant_tw<TM, WARPS, 8>(L, sms, stream, grid_out);
+        if (L.tw == 8) return launch_variant_tw<TM, WARPS, 8, WIDE>(L, sms, stream, grid_out);
     }
-    return launch_variant_tw<TM, WARPS, 4>(L, sms, stream, grid_out);
+    return launch_variant_tw<TM, WARPS, 4, WIDE>(L, sms, stream, grid_out);
 }
 
 template <int TNS, int WARPS>
@@ -738,28 +738,33 @@ slcs_status launch_batch_variant(const BatchLaunch &B, cudaStream_t stream, int 
 
 } // namespace
 
-// Dispatch on rows per lane and warps per block.
+// Dispatch on rows per lane, warps per block and the cell rule.
+template <int TM>
+static slcs_status launch_rows(const CombLaunch &L, int warps, long sms, cudaStream_t stream, int *grid_out)
+{
+    if (L.wide) {
+        if (warps == 2) return launch_variant<TM, 2, true>(L, sms, stream, grid_out);
+        if (warps == 8) return launch_variant<TM, 8, true>(L, sms, stream, grid_out);
+        return launch_variant<TM, 4, true>(L, sms, stream, grid_out);
+    }
+    if (warps == 2) return launch_variant<TM, 2, false>(L, sms, stream, grid_out);
+    if (warps == 8) return launch_variant<TM, 8, false>(L, sms, stream, grid_out);
+    return launch_variant<TM, 4, false>(L, sms, stream, grid_out);
+}
+
 static slcs_status launch_comb_sms(const CombLaunch &L, int tile_m, int warps, long sms, cudaStream_t stream,
                                    int *grid_out)
 {
     if (L.ntasks <= 0) return SLCS_OK;
-#define SLCS_TM_CASE(TM)                                                                   \
-    case TM:                                                                               \
-        if (L.wide) return launch_persistent<TM, 4, 4, true>(L, sms, stream, grid_out);    \
-        if (warps == 2) return launch_variant<TM, 2>(L, sms, stream, grid_out);            \
-        if (warps == 8) return launch_variant<TM, 8>(L, sms, stream, grid_out);            \
-        return launch_variant<TM, 4>(L, sms, stream, grid_out);
     switch (tile_m) {
-        SLCS_TM_CASE(2)
-        SLCS_TM_CASE(4)
-        SLCS_TM_CASE(8)
-        SLCS_TM_CASE(12)
-        SLCS_TM_CASE(14)
-        SLCS_TM_CASE(16)
-    default:
-        return fail(SLCS_ERR_UNSUPPORTED, "tile_m must be one of 2, 4, 8, 12, 14, 16");
+    case 2: return launch_rows<2>(L, warps, sms, stream, grid_out);
+    case 4: return launch_rows<4>(L, warps, sms, stream, grid_out);
+    case 8: return launch_rows<8>(L, warps, sms, stream, grid_out);
+    case 12: return launch_rows<12>(L, warps, sms, stream, grid_out);
+    case 14: return launch_rows<14>(L, warps, sms, stream, grid_out);
+    case 16: return launch_rows<16>(L, warps, sms, stream, grid_out);
+    default: return fail(SLCS_ERR_UNSUPPORTED, "tile_m must be one of 2, 4, 8, 12, 14, 16");
     }
-#undef SLCS_TM_CASE
 }
 
 slcs_status launch_comb_on(const CombLaunch &L, int tile_m, int warps, int sms, cudaStream_t stream)

@@ -33,7 +33,7 @@ struct CombLaunch {
 constexpr int64_t FAST_IDS = 0x3F800000;
 inline bool wide_ids(int64_t m, int64_t n, const slcs_config *cfg)
 {
-    return m + n > FAST_IDS || (cfg && cfg->strand_bits == 32);
+    return m + n > FAST_IDS || (cfg && cfg->strand_bits == 64);
 }
 
 // Columns per step for a wavefront launch whose longest stripe chain has
