@@ -28,11 +28,13 @@ thread_local std::string g_last_error;
 struct DeviceState {
     uint32_t *host_status = nullptr;
     uint32_t *dev_status = nullptr;
+    cudaMemPool_t plan_pool = nullptr; // of the batch plans' blocks; null: they come from cudaMalloc
     int sms = 0;
     bool init = false;
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[64];
+constexpr uint64_t PLAN_POOL_KEPT = uint64_t(64) << 20;
 
 DeviceState &dev_state()
 {
@@ -53,6 +55,19 @@ DeviceState &dev_state()
         if (cudaDeviceGetDefaultMemPool(&pool, d) == cudaSuccess) {
             uint64_t keep = UINT64_MAX;
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        // Batch plans have a pool of their own, which keeps PLAN_POOL_KEPT and
+        // gives the rest back when a plan is destroyed: their blocks can be
+        // gigabytes and may never be wanted again.
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = d;
+        if (cudaMemPoolCreate(&s.plan_pool, &props) == cudaSuccess) {
+            uint64_t keep = PLAN_POOL_KEPT;
+            cudaMemPoolSetAttribute(s.plan_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        } else {
+            s.plan_pool = nullptr;
         }
         cudaGetLastError();
         void *p = nullptr;
@@ -566,6 +581,7 @@ struct slcs_batch_plan {
     uint64_t wait_ns = DEFAULT_WAIT_NS;
     bool use_graph = false;
     char *d_block = nullptr; // every device array of the plan lies in it
+    bool pooled = false;     // it is the plans' pool's
     PairDev *d_pairs = nullptr;
     int32_t *d_seg_off = nullptr;
     int32_t *d_seg_list = nullptr;
@@ -1637,10 +1653,13 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     place(&P->d_scratch, P->stm > 0 ? 0 : size_t(S.scratch_elems));
     place(&P->d_work, P->work_bytes / sizeof(int32_t));
     place(&P->d_relay_ws, P->relay_ws_bytes);
-    // From the memory pool that the workspaces of other calls come from (a
-    // cudaMalloc beyond a megabyte maps memory, about 300 us a plan); the copy
-    // below orders it before any stream's work.
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&P->d_block), std::max<size_t>(bytes, 256), nullptr);
+    // From the plans' pool (a cudaMalloc beyond a megabyte maps memory, about
+    // 300 us a plan).  The block and what is copied to it are there when the
+    // stream has synchronised: runs may use streams that do not wait for it.
+    P->pooled = dev_state().plan_pool != nullptr;
+    cudaError_t e = P->pooled ? cudaMallocFromPoolAsync(reinterpret_cast<void **>(&P->d_block), std::max<size_t>(bytes, 256),
+                                                        dev_state().plan_pool, nullptr)
+                              : cudaMalloc(reinterpret_cast<void **>(&P->d_block), std::max<size_t>(bytes, 256));
     auto rebase = [&](auto *&ptr) {
         ptr = e == cudaSuccess ? reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(
                                      P->d_block + reinterpret_cast<uintptr_t>(ptr))
@@ -1664,6 +1683,7 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     rebase(P->d_work);
     rebase(P->d_relay_ws);
     if (e == cudaSuccess && !up.empty()) e = cudaMemcpy(P->d_block, up.data(), up.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (P->nrelay > 0 && !P->relay_all && P->relay_sms > 0 && P->nstream > 0) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming);
@@ -1971,7 +1991,12 @@ slcs_status slcs_batch_plan_destroy(slcs_batch_plan *P)
         cudaGetDevice(&cur);
         if (cur != P->device) cudaSetDevice(P->device);
         cudaDeviceSynchronize(); // as cudaFree waits: the plan may still be running
-        cudaFreeAsync(P->d_block, nullptr);
+        if (P->pooled) {
+            cudaFreeAsync(P->d_block, nullptr);
+            cudaStreamSynchronize(nullptr); // gives back what is past PLAN_POOL_KEPT
+        } else {
+            cudaFree(P->d_block);
+        }
         if (cur != P->device) cudaSetDevice(cur);
     }
     cudaFree(P->h_stage);
