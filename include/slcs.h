@@ -247,9 +247,9 @@ typedef struct {
      * not stream, or (relay_all) of every pair, in which case the fields above
      * say what a configuration naming a variant would get.                     */
     int32_t relay_groups;
-    int32_t relay_all;
-    int32_t relay_duos; /* entries of two pairs a register holds (0: the relay kernel's registers hold one) */
-} slcs_plan_info;
+    uint32_t relay_all : 1;
+    uint32_t relay_duos : 31; /* entries of two pairs a register holds (0: the relay kernel's registers hold one) */
+} slcs_plan_info; /* 48 bytes, as long as it has been: a caller's may be no longer */
 SLCS_API slcs_status slcs_batch_plan_info(const slcs_batch_plan *plan, slcs_plan_info *info);
 
 /* ---- permutation matrix ------------------------------------------------ */

@@ -52,11 +52,11 @@ class PlanInfo(ctypes.Structure):
     _fields_ = [("stream_tile_m", ctypes.c_int32), ("seg", ctypes.c_int32), ("wavefront_tile_m", ctypes.c_int32),
                 ("warps", ctypes.c_int32), ("stream_pairs", ctypes.c_int32), ("wavefront_tasks", ctypes.c_int32),
                 ("stream_classes", ctypes.c_int32), ("tile_n", ctypes.c_int32), ("grid", ctypes.c_int32),
-                ("packed_pairs", ctypes.c_int32), ("relay_groups", ctypes.c_int32), ("relay_all", ctypes.c_int32),
-                ("relay_duos", ctypes.c_int32)]
+                ("packed_pairs", ctypes.c_int32), ("relay_groups", ctypes.c_int32), ("relay_all", ctypes.c_uint32, 1),
+                ("relay_duos", ctypes.c_uint32, 31)]
 
     def as_dict(self):
-        return {k: int(getattr(self, k)) for k, _ in self._fields_ if k != "reserved"}
+        return {k: int(getattr(self, k)) for k, *_ in self._fields_ if k != "reserved"}
 
 
 class PairInfo(ctypes.Structure):
