@@ -1123,6 +1123,7 @@ static void plan_add_chunks(slcs_batch_plan *P, const slcs_pair_desc *pairs, int
         if (plan_create_impl(&k.plan, pairs + p0, p1 - p0, cfg, true) != SLCS_OK) {
             for (auto &x : ch) slcs_batch_plan_destroy(x.plan);
             if (k.plan) slcs_batch_plan_destroy(k.plan);
+            cudaGetLastError(); // not the next launch's
             return;
         }
         ch.push_back(k);
@@ -1731,6 +1732,16 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     }
     if (e != cudaSuccess) {
         slcs_batch_plan_destroy(P);
+        if (e == cudaErrorMemoryAllocation && !wavefront_only && !chunk) {
+            // No room for staged couples or hand-down rows: wavefront plans need
+            // the least.  (A chunk is only there to be faster.)
+            cudaGetLastError();
+            slcs_config least{};
+            least.algo = SLCS_ALGO_WAVEFRONT;
+            least.use_graph = cfg ? cfg->use_graph : 0;
+            least.wait_ms = cfg ? cfg->wait_ms : 0;
+            return plan_create_impl(plan_out, pairs, npairs, &least, chunk);
+        }
         return cuda_fail(e, "batch plan upload");
     }
     *plan_out = P;
