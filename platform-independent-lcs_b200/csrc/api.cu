@@ -1723,7 +1723,8 @@ static slcs_status plan_create_impl(slcs_batch_plan **plan_out, const slcs_pair_
     rebase(P->d_scratch);
     rebase(P->d_work);
     rebase(P->d_relay_ws);
-    if (e == cudaSuccess && !up.empty()) e = cudaMemcpy(P->d_block, up.data(), up.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !up.empty())
+        e = cudaMemcpyAsync(P->d_block, up.data(), up.size(), cudaMemcpyHostToDevice, nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (P->nrelay > 0 && !P->relay_all && P->relay_sms > 0 && P->nstream > 0) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking);
