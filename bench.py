@@ -417,7 +417,7 @@ def main():
         "roofline": {"bound": "int32", "achieved": kern_gcups, "peak": roof_gcups, "unit": "GCUPS",
                      "frac": kern_gcups / roof_gcups, "traffic": read_traffic("reads_20000"),
                      "peak_source": "measured here: INT32 min/max issue rate / 5 ops per cell",
-                     "int32_tops": int_ops / 1e12, "cell_rule_ceiling_gcups": cell_rate / 1e9},
+                     "int32_tops": int_ops / 1e12, "compare_select_rule_gcups": cell_rate / 1e9},
         "clocks": sampler.summary(),
         "bitexact_vs_reference": bitexact,
     }

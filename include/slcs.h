@@ -65,8 +65,9 @@ typedef struct {
     int32_t use_graph;     /* batch plans: replay the launch as a captured CUDA graph */
     int32_t seg;           /* batch stream mode: lanes per pipeline segment (8/16/32) */
     int32_t wait_ms;       /* limit of one device-side wait (default 10000 ms)        */
-    int32_t blocks_per_sm; /* batch plans: resident blocks per SM (default: 2 for plans with packed
-                              pairs, else as many as fit)                                 */
+    int32_t blocks_per_sm; /* batch plans: resident blocks per SM of the 32-bit stream kernel (default:
+                              as many as fit); of pairs combed two per register, warps per SM
+                              sub-partition (1 to 3, more count as 3, the default)         */
     int32_t strand_bits;   /* batch plans: 16 = combine two pairs per register where ids fit 15 bits,
                               32 = 32-bit strands only, 0 = engine default; single pairs and
                               wavefront plans: 64 = the cell rule for ids of any size, which
@@ -74,8 +75,8 @@ typedef struct {
     int32_t bands;         /* row bands of a for SLCS_ALGO_STRIPS (glued by row-glue products) */
     int32_t pool_pct;      /* batch plans: percent of each stream class's work kept in a pool that
                               segments claim pair by pair once their own lists are done
-                              (0 = default: 50 for plans with packed pairs, else 15;
-                              -1 = none: every pair in a fixed list)        */
+                              (0 = default: 15; -1 = none: every pair in a fixed list); pairs
+                              combed two per register have no pool                         */
     int32_t reserved[3];
 } slcs_config;
 
@@ -272,7 +273,8 @@ SLCS_API slcs_status slcs_permutation_to_strands(const int32_t *row_to_col, int3
  * whole-string one against its prefix DP (src/lcs_reference.hpp:71-132).
  * v_strands (n), begin, end and llcs_out (nq) are device arrays; a query
  * outside 0 <= begin <= end <= n gets -1 and slcs_device_status() reports
- * SLCS_ERR_INVALID. */
+ * SLCS_ERR_INVALID.  For n of 16384 and more the call may take a workspace of
+ * about 4 n bytes from the device's memory pool; it runs without one, too. */
 SLCS_API slcs_status slcs_substring_llcs(const int32_t *v_strands, int32_t m, int32_t n, const int32_t *begin,
                                          const int32_t *end, int32_t nq, int32_t *llcs_out, void *stream);
 
@@ -333,9 +335,11 @@ SLCS_API slcs_status slcs_costmodel_grad(const float *params, int32_t k, const f
 
 /* ---- diagnostics (no counterpart in the reference) --------------------- */
 
-/* Measured integer ceilings of the current device, the denominators of the
- * combing roofline: the INT32 min/max issue rate (ops/s) and the cell rate
- * of the combing rule on register-resident strands (cells/s). */
+/* Measured integer rates of the current device: the INT32 min/max issue rate
+ * (ops/s), the denominator of the combing roofline at 5 operations a cell, and
+ * the cell rate of the rule as two compares and two selects on
+ * register-resident strands (cells/s; the kernels' rules take fewer
+ * instructions, so it is no ceiling for them). */
 SLCS_API slcs_status slcs_probe_int_rates(int32_t iters, double *int32_ops_per_s, double *cells_per_s,
                                           void *stream);
 

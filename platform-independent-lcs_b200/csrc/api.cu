@@ -127,8 +127,9 @@ int pick_tile_m(const slcs_config *cfg, int32_t m_typical, int64_t total_cells)
     return pick_tile_m_for(cfg, m_typical, tall ? sm_count() : 1);
 }
 
-// Column strips for one pair when nothing is configured, fitted to B200
-// timings of uniform {0..3} pairs.  One wavefront keeps few warps busy below
+// Column strips for one pair when nothing is configured and no relay shape
+// takes it (on 148 SMs below 2^19 rows only pairs of more than 2^30 ids), fitted
+// to B200 timings of uniform {0..3} pairs.  One wavefront keeps few warps busy below
 // about 2^19 rows (stripe t starts 32 column blocks after stripe t-1), while
 // every strip adds a braid product with overlap m.  About n / sqrt(4096 m)
 // strips (a power of two, rounded up from 2^(k+0.45); 1..64 strips of at
@@ -147,8 +148,8 @@ int auto_strips(int32_t m, int32_t n)
     return S;
 }
 
-// Row bands for one tall pair (at least 2^19 rows) when nothing is
-// configured.  The stripes of a band form a chain that fills and drains in
+// Row bands for one tall pair (at least 2^19 rows) when nothing is configured
+// and no relay shape takes it (on 148 SMs beyond 1,060,864 rows).  The stripes of a band form a chain that fills and drains in
 // about 44 steps of 4 columns per stripe, so a pair combed in R bands spends
 // about (n + 176 * stripes / R) / n times its cell time; every band adds
 // row-glue products, about log2(R) * m + (R - 1) * n permutation entries in
@@ -223,7 +224,11 @@ double merge_us(double k, double count)
 // The relay kernel's plan for one pair: shape, column strips and row bands
 // with the least predicted time among those whose groups fit one to an SM
 // (two blocks on one SM slow the whole chain: 342 groups of (4, 2, 3) on 148
-// SMs combed 131072 x 131072 in 13.2 ms, 128 of (8, 4, 4) in 6.4 ms).
+// SMs combed 131072 x 131072 in 13.2 ms, 128 of (8, 4, 4) in 6.4 ms; 152 groups
+// of (14, 4, 16) combed the 2^20 pair in 353 ms, 148 in 190).  Bands one after
+// another would need no more SMs but are not planned: a pair past the tallest
+// shape, 1,060,864 rows on 148 SMs, takes the wavefront kernel (1,060,865 x
+// 30,000: 17.4 ms).
 // relay.tm == 0: no shape fits.  Predicted: a chain's steps (columns, then
 // the lags of its warps and blocks) at the shape's step time, and the merge
 // levels.

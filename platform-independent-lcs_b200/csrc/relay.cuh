@@ -5,8 +5,8 @@
 
 namespace slcs {
 
-// One launch: items are groups of RELAY_WARPS row stripes (32 * rows per lane
-// rows each) of a pair.  Groups of a pair are consecutive items in ascending
+// One launch: items are groups of RelayShape::warps row stripes (32 * rows per
+// lane rows each) of a pair.  Groups of a pair are consecutive items in ascending
 // order, so the producer of a group was claimed first by a running block.
 struct RelayLaunch {
     const PairDev *pairs;   // device; null = the one pair of `single`

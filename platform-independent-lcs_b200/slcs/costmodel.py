@@ -29,7 +29,9 @@ DB_PATH = os.path.join(HERE, "data", "timings.npz")
 # pair of a shape with slcs_comb_pair under a tiling and a steady-ant cutoff
 # (src/braid_multiplication.hpp:204-270 is the recursion whose base case the
 # cutoff moves), and apply to shapes of at most PAIR_BATCH_MAX pairs.
-# Variant 0 is what the library does for a batch when nothing is configured.
+# Variant 0 is what the library does for a batch when nothing is configured;
+# stream_auto_bpsm4 is the same launch where all pairs are combed two per
+# register (4 warps a sub-partition count as 3, the default there).
 PAIR_BATCH_MAX = 8
 VARIANTS: List[dict] = [
     {"name": "stream_auto", "kind": "batch", "cfg": {}},

@@ -317,7 +317,8 @@ def strips_and_braid(ad, bd, o, gold_hash, dev):
         gbs = algo_bytes / (ms * 1e-3) / 1e9
         braid[str(cutoff)] = {"ms": ms, "algorithmic_bytes": algo_bytes, "achieved_gbs": gbs, "frac": gbs / peak}
     tiles = pair_plan_info(m, n)
-    return {"long_pair_tiles": {"workload": f"pair_1M as {tiles['bands']} row bands x {tiles['strips']} column "
+    bands, strips = (tiles[("relay_" if tiles["relay_tile_m"] else "") + k] for k in ("bands", "strips"))
+    return {"long_pair_tiles": {"workload": f"pair_1M as {bands} row bands x {strips} column "
                                              "strips + braid merge trees", "cutoff_sweep": sweep},
             "braid_top_merge": {"workload": "staggered_multiply<false>(P(a,b[:n/2]), P(a,b[n/2:]), k=2^20)",
                                 "bound": "hbm", "peak_gbs": peak, "peak_source": peak_src, "by_cutoff": braid}}
